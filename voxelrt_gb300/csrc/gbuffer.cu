@@ -30,14 +30,13 @@ struct GbufferParams {
 // order the oracle states (getMaterialColor and its square, round-half-even to 8 bits,
 // packGNormal; proj * (pos / 16, 1) then z / w).
 template <bool kGlsl>
-__device__ __forceinline__ void gbuffer_texel(const RayState& s, bool hit, const uint32_t* pal, const float* m,
-                                              uint32_t& texel, float& depth) {
+__device__ __forceinline__ void gbuffer_texel(const RayState& s, bool hit, uint32_t c, const float* m, uint32_t& texel,
+                                              float& depth) {
     if (!hit) {
         texel = 0x00FFFFFFu;
         depth = -1.0f;
         return;
     }
-    const uint32_t c = pal[s.material];
     const float r = __fmul_rn(__uint2float_rn((c >> 11) & 31u), 1.0f / 31);
     const float g = __fmul_rn(__uint2float_rn((c >> 5) & 63u), 1.0f / 63);
     const float b = __fmul_rn(__uint2float_rn(c & 31u), 1.0f / 31);
@@ -54,18 +53,16 @@ __device__ __forceinline__ void gbuffer_texel(const RayState& s, bool hit, const
     depth = __fdiv_rn(z, w);
 }
 
-// 8x8 pixels per block; the palette and the matrix go to shared memory first.
+// 8x8 pixels per block.  The palette is read where it lies, in the parameters' constant bank: a
+// load takes a turn per distinct material of a warp's hits, a few in most scenes.  (Staging
+// it in shared memory cost every block 256 constant reads at 32 addresses a warp, and a
+// barrier: the address divergence unit was busy half the time.  1280x720 GLSL G-buffer of a
+// 512-voxel terrain: 51.5 us staged, 41.9 us direct.)
 template <bool kGlsl, bool kAniso>
-__global__ void __launch_bounds__(64) gbuffer_kernel(DevWorld w, ViewDev v, GbufferParams gp,
+__global__ void __launch_bounds__(64) gbuffer_kernel(DevWorld w, ViewDev v, const __grid_constant__ GbufferParams gp,
                                                     uint32_t* __restrict__ tex, float* __restrict__ depth,
                                                     uint4* __restrict__ out) {
     if constexpr (kAniso) fill_forward_lut();
-    __shared__ uint32_t s_pal[256];
-    __shared__ float s_proj[16];
-    const uint32_t t = threadIdx.y * 8 + threadIdx.x;
-    for (uint32_t i = t; i < 256; i += 64) s_pal[i] = gp.palette[i];
-    if (t < 16) s_proj[t] = gp.proj[t];
-    __syncthreads();
     const uint32_t px = blockIdx.x * 8 + threadIdx.x, py = blockIdx.y * 8 + threadIdx.y;
     if (px >= v.width || py >= v.height) return;
     const uint32_t pixel = py * v.width + px;
@@ -81,7 +78,7 @@ __global__ void __launch_bounds__(64) gbuffer_kernel(DevWorld w, ViewDev v, Gbuf
     const bool hit = st == kStepHit && i < v.max_iters;
     uint32_t texel;
     float d;
-    gbuffer_texel<kGlsl>(s, hit, s_pal, s_proj, texel, d);
+    gbuffer_texel<kGlsl>(s, hit, gp.palette[s.material], gp.proj, texel, d);
     tex[pixel] = texel;
     depth[pixel] = d;
     if (out) out[pixel] = pack_state<kGlsl>(s, hit, i, pixel);

@@ -31,69 +31,92 @@ __device__ __forceinline__ uint32_t compact_even_bits(uint32_t k) {
     return k;
 }
 
-template <bool kCount, bool kGlsl>
-__device__ __forceinline__ bool run_ray(RayState& s, bool safe, const DevWorld& w, int32_t wox, int32_t woy,
-                                        int32_t woz, uint32_t max_iters, uint32_t& steps, TraceCounters& cnt,
-                                        bool coarse_ray = false, bool aniso = false) {
-    uint32_t i = 0;
-    uint32_t st = dda_steps_mode<kCount, kGlsl>(s, w, wox, woy, woz, cnt, safe, coarse_ray, coarse_ray, aniso, 0, i,
-                                                max_iters);
-    if (max_iters == 0) st = kStepOut;
-    steps = i;
-    return st == kStepHit && i < max_iters;
+// What the rays of one view share, from its camera origin: whether that is inside and near
+// (origin_inside_near) with the distances to the clip box's sides.
+struct ViewStart {
+    ClipBox clip;
+    BoxSides box;
+    uint32_t inside;
+};
+
+VRT_HD inline ViewStart view_start(const DevWorld& w, const ViewDev& v) {
+    ViewStart s{};
+    s.clip = clip_box(w, v.wo);
+    s.box = box_sides(s.clip, v.ox, v.oy, v.oz);
+    s.inside = origin_inside_near(s.clip, v.ox, v.oy, v.oz) ? 1u : 0u;
+    return s;
 }
 
-// One thread per pixel, whole path (VoxelRender.comp:27-93 structure).
-template <bool kGlsl, bool kAniso = false>
-__global__ void __launch_bounds__(64) view_path_kernel(DevWorld w, ViewDev v, uint4* __restrict__ out) {
-    if constexpr (kAniso) fill_forward_lut();
-    const uint32_t px = blockIdx.x * 8 + threadIdx.x;
-    const uint32_t py = blockIdx.y * 8 + threadIdx.y;
-    if (px >= v.width || py >= v.height) return;
-    const uint32_t pixel = py * v.width + px;
-    const uint64_t plane = (uint64_t)v.width * v.height;
-    const int32_t wox = v.wo[0], woy = v.wo[1], woz = v.wo[2];
-    TraceCounters cnt{0, 0};
-    float ox = v.ox, oy = v.oy, oz = v.oz, dx, dy, dz;
-    camera_ray(v.d0, v.du, v.dv, px, py, dx, dy, dz);
-    RayState s;
-    bool safe = ray_start<kGlsl>(s, w, ox, oy, oz, dx, dy, dz, wox, woy, woz);
-    uint32_t steps;
-    bool hit = run_ray<false, kGlsl>(s, safe, w, wox, woy, woz, v.max_iters, steps, cnt, false, kAniso);
+// One pixel's whole path: the primary ray, then its sun ray or bounces, or with kFull the GPU
+// renderer's path (VoxelRender.comp:27-93); returns the rays traced.  One loop over the rays,
+// so that the step loop is compiled once.
+template <bool kGlsl, bool kAniso, bool kBounces>
+__device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld& w, const ViewStart& vs, uint32_t px,
+                                                uint32_t py, uint4* __restrict__ out) {
+    const uint32_t pixel = py * v.width + px, last = v.last_kind();
     uint4* o = out + v.out_base + pixel;
-    o[0] = pack_state<kGlsl>(s, hit, steps, pixel);
-    const uint32_t last = v.last_kind();
-    const bool full = (v.path & kPathFull) != 0;
-    float pox = 0.0f, poy = 0.0f, poz = 0.0f, pnx = 0.0f, pny = 0.0f, pnz = 0.0f;  // full path: last hit frame
-    for (uint32_t k = 1; k <= last; k++) {
-        if (!hit) {
-            o[k * plane] = no_ray_hit();
-            continue;
+    float dx, dy, dz;
+    camera_ray(v.d0, v.du, v.dv, px, py, dx, dy, dz);
+    const int32_t wox = v.wo[0], woy = v.wo[1], woz = v.wo[2];
+    const bool full = kBounces && (v.path & kPathFull) != 0;
+    RayState s;
+    uint32_t i = 0;
+    if (vs.inside) {
+        ray_start_inside<kGlsl>(s, vs.box, v.ox, v.oy, v.oz, dx, dy, dz, wox, woy, woz);
+    } else {
+        ray_start<kGlsl>(s, vs.clip, v.ox, v.oy, v.oz, dx, dy, dz, wox, woy, woz);
+    }
+    TraceCounters cnt{0, 0};
+    float hx = 0.0f, hy = 0.0f, hz = 0.0f, nx = 0.0f, ny = 0.0f, nz = 0.0f;  // the last hit frame
+    for (uint32_t k = 0;;) {
+        // GLSL mode: shadow and bounce rays are rayCastCoarse's (VoxelRender.comp:56,74)
+        const bool coarse = kGlsl && k != 0;
+        const uint32_t iters = coarse ? min(v.max_iters, kCoarseMaxIters) : v.max_iters;
+        const uint32_t st = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, i, iters);
+        const bool hit = st == kStepHit;
+        *o = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, i, pixel);
+        if (k == last) return k + 1;
+        // the path goes on after a hit, and the whole path after a sun ray, hit or miss
+        const bool go = hit || (full && full_is_sun(k));
+        const size_t plane = (size_t)v.width * v.height;
+        if (!go) {
+            const uint32_t n = k + 1;
+            for (; k < last; k++) *(o += plane) = no_ray_hit();
+            return n;
         }
-        if (full) {
+        k++;
+        o += plane;
+        if (kBounces) {
             // a sun ray starts from the hit just traced; a bounce from the hit before its
-            // sun ray (saved), or from the bounce just traced when no sun ray follows it
-            if (full_is_sun(k) || !full_is_sun(k - 1)) hit_frame<kGlsl>(s, pox, poy, poz, pnx, pny, pnz);
-            ox = pox;
-            oy = poy;
-            oz = poz;
-            if (full_is_sun(k)) {
+            // sun ray (kept), or from the bounce just traced when no sun ray follows it
+            if (!full || full_is_sun(k) || !full_is_sun(k - 1)) hit_frame<kGlsl>(s, hx, hy, hz, nx, ny, nz);
+            if (full ? full_is_sun(k) : v.shadow() != 0) {
                 dx = v.sun[0];
                 dy = v.sun[1];
                 dz = v.sun[2];
             } else {
-                bounce_dir(pixel, full_bounce(k), pnx, pny, pnz, dx, dy, dz);
+                bounce_dir(pixel, full ? full_bounce(k) : k, nx, ny, nz, dx, dy, dz);
             }
         } else {
-            next_path_ray<kGlsl>(s, v.shadow() != 0, v.sun, pixel, k, ox, oy, oz, dx, dy, dz);
+            hit_frame<kGlsl>(s, hx, hy, hz, nx, ny, nz);
+            dx = v.sun[0];
+            dy = v.sun[1];
+            dz = v.sun[2];
         }
-        safe = ray_start<kGlsl>(s, w, ox, oy, oz, dx, dy, dz, wox, woy, woz, false, kGlsl);
-        // GLSL mode: shadow and bounce rays are rayCastCoarse's (VoxelRender.comp:56,74)
-        hit = run_ray<false, kGlsl>(s, safe, w, wox, woy, woz, kGlsl ? min(v.max_iters, kCoarseMaxIters) : v.max_iters,
-                                    steps, cnt, kGlsl, kAniso);
-        o[k * plane] = pack_state<kGlsl>(s, hit, steps, pixel);
-        if (full && full_is_sun(k)) hit = true;  // the path goes on after a sun ray, hit or miss
+        ray_start<kGlsl>(s, vs.clip, hx, hy, hz, dx, dy, dz, wox, woy, woz, kGlsl);
+        i = 0;
     }
+}
+
+// One thread per pixel, whole path (VoxelRender.comp:27-93 structure).
+template <bool kGlsl, bool kAniso = false>
+__global__ void __launch_bounds__(64) view_path_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
+                                                       const __grid_constant__ ViewStart vs, uint4* __restrict__ out) {
+    if constexpr (kAniso) fill_forward_lut();
+    const uint32_t px = blockIdx.x * 8 + threadIdx.x;
+    const uint32_t py = blockIdx.y * 8 + threadIdx.y;
+    if (px >= v.width || py >= v.height) return;
+    trace_pixel<kGlsl, kAniso, true>(v, w, vs, px, py, out);
 }
 
 // View-table loads: read-only through the non-coherent path, or at L2 (coherent with
@@ -120,6 +143,16 @@ __device__ __forceinline__ V vget4(const V* a) {
     return *a;
 }
 
+// A world-table entry (the table does not change while a launch runs).
+__device__ __forceinline__ DevWorld load_world(const DevWorld* p) {
+    DevWorld w;
+    const uint4* a = reinterpret_cast<const uint4*>(p);
+    uint4* b = reinterpret_cast<uint4*>(&w);
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(DevWorld) / 16); i++) b[i] = __ldg(a + i);
+    return w;
+}
+
 constexpr uint32_t kClaimEmpty = 0xFFFFFFFFu, kClaimStop = 0xFFFFFFFEu;
 
 constexpr uint32_t kNoChunk = 0xFFFFFFFFu;
@@ -134,7 +167,7 @@ struct ResidentWarp {
     uint32_t idle_ns, sleep_ns;      // sleep while idle
     uint32_t acc_view, acc_n;        // finished pixels of view acc_view not yet subtracted
     uint32_t cached_view;            // view held in the warp's shared copy of the table entry
-    uint32_t q_inside;               // origin_inside_safe() for that view's camera
+    uint32_t q_inside;               // origin_inside_near() for that view's camera
 };
 constexpr uint32_t kNoView = 0xFFFFFFFFu;
 
@@ -232,17 +265,14 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
     const uint32_t lt = (1u << lane) - 1u;
     // warp-uniform queue state: rays [q_next, q_end) of view q_view
     uint32_t q_view = 0, q_next = 0, q_end = 0;
-    bool q_empty = false, q_inside = false;  // q_inside: origin_inside_safe() for q_view's camera
+    bool q_empty = false, q_inside = false;  // q_inside: origin_inside_near() for q_view's camera
     // lane state
     bool active = false;
     // path: kind of the current ray (0 primary, then shadow or bounce number) in bits
     // 0-7, last kind of the pixel's path in bits 8-15, shadow flag in bit 16, ray
-    // ended with its record pending in bit 17 (kEnded), that ray hit in bit 18 (kHit),
-    // the ray is safe for ray_step<kCount, true> in bit 19 (kSafe)
-    constexpr uint32_t kEnded = 1u << 17, kHit = 1u << 18, kSafe = 1u << 19;
-    uint32_t pixel = 0, path = 0, iter = 0, max_iters = 0, plane = 0, vidx = 0;
-    DevWorld w{};
-    int32_t wox = 0, woy = 0, woz = 0;
+    // ended with its record pending in bit 17 (kEnded), that ray hit in bit 18 (kHit)
+    constexpr uint32_t kEnded = 1u << 17, kHit = 1u << 18;
+    uint32_t pixel = 0, path = 0, iter = 0, vidx = 0;
     RayState s;
     uint32_t rays = 0, hits = 0;
     TraceCounters cnt{0, 0};
@@ -266,14 +296,17 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
         // them instead of once per lane that happens to end on a given step.
         if (path & kEnded) {
             const bool hit = (path & kHit) != 0;
-            path &= ~(kEnded | kHit | kSafe);
+            path &= ~(kEnded | kHit);
             const ViewDev* v = p.views + vidx;
             const bool vs = kResident && vidx == rw.cached_view;
             if (vs) v = &sview;
             uint4* rec = p.out + vget<kResident>(&v->out_base, vs) + pixel;
             uint32_t kind = path & 0xFF;
             const uint32_t last_kind = (path >> 8) & 0xFF;
-            rec[(size_t)kind * plane] = pack_state<kGlsl>(s, hit, iter, pixel);
+            const int4 wv = vs ? *reinterpret_cast<const int4*>(v->wo) : ldv<kResident>(reinterpret_cast<const int4*>(v->wo));
+            const size_t plane = (size_t)vget<kResident>(&v->width, vs) * vget<kResident>(&v->height, vs);
+            const DevWorld w = load_world(p.worlds + wv.w);
+            rec[kind * plane] = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, iter, pixel);
             rays++;
             if (kCount && hit) hits++;
             // the GPU renderer's whole path goes on after a sun ray, hit or miss
@@ -317,12 +350,11 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
                 } else {
                     next_path_ray<kGlsl>(s, ((path >> 16) & 1u) != 0, sun, pixel, kind, ox, oy, oz, dx, dy, dz);
                 }
-                path &= ~kSafe;
-                if (ray_start<kGlsl>(s, w, ox, oy, oz, dx, dy, dz, wox, woy, woz, false, kGlsl)) path |= kSafe;
+                const int32_t wo3[3] = {wv.x, wv.y, wv.z};
+                ray_start<kGlsl>(s, clip_box(w, wo3), ox, oy, oz, dx, dy, dz, wv.x, wv.y, wv.z, kGlsl);
                 iter = 0;
-                if (kGlsl) max_iters = min(max_iters, kCoarseMaxIters);  // rayCastCoarse's cap
             } else {
-                for (uint32_t kk = kind + 1; kk <= last_kind; kk++) rec[(size_t)kk * plane] = no_ray_hit();
+                for (uint32_t kk = kind + 1; kk <= last_kind; kk++) rec[kk * plane] = no_ray_hit();
                 active = false;
                 finished = true;
             }
@@ -430,10 +462,10 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
                     // the view's camera origin, shared by its rays: inside the clip box?
                     // (a resident view's world index is checked before it is used)
                     const int4 qwv = vget4<kResident>(reinterpret_cast<const int4*>(qv->wo));  // origin xyz, world
+                    const int32_t qwo[3] = {qwv.x, qwv.y, qwv.z};
                     const bool inside = (!kResident || (uint32_t)qwv.w < p.n_worlds) &&
-                                        origin_inside_safe(p.worlds[qwv.w], vget<kResident>(&qv->ox, true),
-                                                           vget<kResident>(&qv->oy, true), vget<kResident>(&qv->oz, true),
-                                                           qwv.x, qwv.y, qwv.z);
+                                        origin_inside_near(clip_box(p.worlds[qwv.w], qwo), vget<kResident>(&qv->ox, true),
+                                                           vget<kResident>(&qv->oy, true), vget<kResident>(&qv->oz, true));
                     if (kResident) {  // kept with the warp's other shared state (registers are short)
                         if (lane == 0) rw.q_inside = inside ? 1u : 0u;
                         __syncwarp();
@@ -480,14 +512,9 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
                     if (valid) {
                         vidx = q_view;
                         pixel = py * width + px;
-                        plane = width * height;
                         iter = 0;
-                        max_iters = mp.x;
                         path = mp.y;
-                        w = p.worlds[wv.w];
-                        wox = wv.x;
-                        woy = wv.y;
-                        woz = wv.z;
+                        const DevWorld w = load_world(p.worlds + wv.w);
                         // d0, du, dv with the camera origin in the fourth lanes
                         const float4 g0 = vget4<kResident>(reinterpret_cast<const float4*>(v->d0));
                         const float4 g1 = vget4<kResident>(reinterpret_cast<const float4*>(v->du));
@@ -495,9 +522,13 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
                         const float d0[3] = {g0.x, g0.y, g0.z}, du[3] = {g1.x, g1.y, g1.z}, dv[3] = {g2.x, g2.y, g2.z};
                         float dx, dy, dz;
                         camera_ray(d0, du, dv, px, py, dx, dy, dz);
-                        if (ray_start<kGlsl>(s, w, g0.w, g1.w, g2.w, dx, dy, dz, wox, woy, woz,
-                                             kResident ? rw.q_inside != 0 : q_inside))
-                            path |= kSafe;
+                        const int32_t wo3[3] = {wv.x, wv.y, wv.z};
+                        const ClipBox clip = clip_box(w, wo3);
+                        if (kResident ? rw.q_inside != 0 : q_inside)
+                            ray_start_inside<kGlsl>(s, box_sides(clip, g0.w, g1.w, g2.w), g0.w, g1.w, g2.w, dx, dy, dz, wv.x,
+                                                    wv.y, wv.z);
+                        else
+                            ray_start<kGlsl>(s, clip, g0.w, g1.w, g2.w, dx, dy, dz, wv.x, wv.y, wv.z);
                         active = true;
                     }
                 }
@@ -519,25 +550,44 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
             rw.idle_ns = 0;
             rw.sleep_ns = 1000;
         }
-        // one DDA round: up to p.inner steps, fewer when the iteration cap comes first
-        // (an active lane always has iter < max_iters); the fast step when every
-        // tracing lane of the warp is safe
-        const bool all_safe = __all_sync(0xffffffffu, !active || (path & kSafe) != 0);
         // GLSL mode: does any lane trace a shadow or bounce ray (rayCastCoarse's)?
         const bool any_coarse = kGlsl && __any_sync(0xffffffffu, active && (path & 0xFFu) != 0);
+        // The lane's world origin, cap and world, read again for each round: held in registers
+        // across the retirement and refill above they cost the step loop spills.
+        int4 wv{};
+        DevWorld w{};
+        uint32_t max_iters = 0;
         if (active) {
-            const uint32_t kmax = min(p.inner, max_iters - iter);
-            uint32_t k = 0, st = kStepContinue;
-            // GLSL mode: the rayCastCoarse variant while some lane traces a shadow or
-            // bounce ray, the anisotropic one for views that ask for it
-            st = dda_steps_mode<kCount, kGlsl>(s, w, wox, woy, woz, cnt, all_safe, any_coarse, (path & 0xFFu) != 0,
-                                               kAniso, iter, k, kmax);
-            iter += k;  // the iteration a ray left on, or max_iters when the cap ran out
-            if (st != kStepContinue)
-                path |= kEnded | (st == kStepHit ? kHit : 0u);
-            else if (iter >= max_iters)
-                path |= kEnded;
+            const ViewDev* v = p.views + vidx;
+            if (kResident && vidx == rw.cached_view) {
+                wv = *reinterpret_cast<const int4*>(sview.wo);
+                max_iters = sview.max_iters;
+            } else {
+                wv = ldv<kResident>(reinterpret_cast<const int4*>(v->wo));
+                max_iters = ldv<kResident>(&v->max_iters);
+            }
+            if (kGlsl && (path & 0xFFu)) max_iters = min(max_iters, kCoarseMaxIters);  // rayCastCoarse's cap
+            w = load_world(p.worlds + wv.w);
         }
+        // Steps until half the tracing lanes have ended, in slices of p.inner: the lanes left
+        // keep the warp busy, and enough have ended to share a retirement.  Two 720p views of
+        // 4 bounces: 468 us, one slice a round 472 us, a quarter left 485 us.
+        const uint32_t stop = (uint32_t)__popc(__ballot_sync(0xffffffffu, active)) / 2u;
+        do {
+            if (active && !(path & kEnded)) {
+                const uint32_t kmax = min(p.inner, max_iters - iter);  // an active lane has iter < max_iters
+                uint32_t k = 0;
+                // GLSL mode: the rayCastCoarse variant while some lane traces a shadow or
+                // bounce ray, the anisotropic one for views that ask for it
+                const uint32_t st = dda_steps_mode<kCount, kGlsl>(s, w, wv.x, wv.y, wv.z, cnt, any_coarse,
+                                                                  (path & 0xFFu) != 0, kAniso, iter, k, kmax);
+                iter += k;  // the iteration a ray left on, or max_iters when the cap ran out
+                if (st != kStepContinue)
+                    path |= kEnded | (st == kStepHit ? kHit : 0u);
+                else if (iter >= max_iters)
+                    path |= kEnded;
+            }
+        } while ((uint32_t)__popc(__ballot_sync(0xffffffffu, active && !(path & kEnded))) > stop);
     }
     // warp totals, one atomic per warp
     for (int off = 16; off > 0; off >>= 1) {
@@ -603,12 +653,14 @@ vrt_status launch_view_path(vrt_world* w, const ViewDev& v, bool glsl, vrt_hit* 
     vrt_status st = l2.enter(w, stream);
     if (st != VRT_OK) return st;
     uint4* out = reinterpret_cast<uint4*>(hits);
+    const DevWorld dw = w->dev();
+    const ViewStart vs = view_start(dw, v);
     if (glsl && v.aniso)
-        view_path_kernel<true, true><<<grid, block, 0, stream>>>(w->dev(), v, out);
+        view_path_kernel<true, true><<<grid, block, 0, stream>>>(dw, v, vs, out);
     else if (glsl)
-        view_path_kernel<true><<<grid, block, 0, stream>>>(w->dev(), v, out);
+        view_path_kernel<true><<<grid, block, 0, stream>>>(dw, v, vs, out);
     else
-        view_path_kernel<false><<<grid, block, 0, stream>>>(w->dev(), v, out);
+        view_path_kernel<false><<<grid, block, 0, stream>>>(dw, v, vs, out);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }
@@ -734,9 +786,6 @@ vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, cons
 
 namespace {
 
-// Resident blocks per SM of the instantiation that a launch of this kind runs: the GLSL
-// and anisotropic variants differ from the default one in registers and shared memory
-// (the anisotropic LUT is 8 KB per block).
 // The instantiation a launch runs: counting, traversal mode, resident, whole-path views.
 using PersistentFn = void (*)(BatchParams);
 template <bool kCount, bool kResident, bool kFull>
@@ -753,6 +802,8 @@ PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, boo
     return full ? persistent_fn_mode<false, false, true>(glsl, aniso) : persistent_fn_mode<false, false, false>(glsl, aniso);
 }
 
+// Resident blocks per SM of that kernel: the variants differ in registers and shared memory
+// (the anisotropic LUT is 8 KB per block).
 cudaError_t persistent_occupancy(int& occ, int threads, bool count, bool glsl, bool aniso, bool resident, bool full) {
     const size_t smem = full ? (size_t)threads * 6 * sizeof(float) : 0;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, persistent_fn(count, glsl, aniso, resident, full),

@@ -57,9 +57,11 @@ __device__ __forceinline__ void gbuffer_texel(const RayState& s, bool hit, uint3
 // load takes a turn per distinct material of a warp's hits, a few in most scenes.  (Staging
 // it in shared memory cost every block 256 constant reads at 32 addresses a warp, and a
 // barrier: the address divergence unit was busy half the time.  1280x720 GLSL G-buffer of a
-// 512-voxel terrain: 51.5 us staged, 41.9 us direct.)
+// 512-voxel terrain: 51.5 us staged, 41.9 us direct; 35.9 us with the step of trace_core.cuh.)
 template <bool kGlsl, bool kAniso>
-__global__ void __launch_bounds__(64) gbuffer_kernel(DevWorld w, ViewDev v, const __grid_constant__ GbufferParams gp,
+__global__ void __launch_bounds__(64) gbuffer_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
+                                                    const __grid_constant__ ClipBox clip, bool inside,
+                                                    const __grid_constant__ BoxSides box, const __grid_constant__ GbufferParams gp,
                                                     uint32_t* __restrict__ tex, float* __restrict__ depth,
                                                     uint4* __restrict__ out) {
     if constexpr (kAniso) fill_forward_lut();
@@ -69,19 +71,23 @@ __global__ void __launch_bounds__(64) gbuffer_kernel(DevWorld w, ViewDev v, cons
     float dx, dy, dz;
     camera_ray(v.d0, v.du, v.dv, px, py, dx, dy, dz);
     RayState s;
-    const bool safe = ray_start<kGlsl>(s, w, v.ox, v.oy, v.oz, dx, dy, dz, v.wo[0], v.wo[1], v.wo[2]);
+    if (inside)
+        ray_start_inside<kGlsl>(s, box, v.ox, v.oy, v.oz, dx, dy, dz, v.wo[0], v.wo[1], v.wo[2]);
+    else
+        ray_start<kGlsl>(s, clip, v.ox, v.oy, v.oz, dx, dy, dz, v.wo[0], v.wo[1], v.wo[2]);
     TraceCounters cnt{0, 0};
     uint32_t i = 0;
-    uint32_t st = dda_steps_mode<false, kGlsl>(s, w, v.wo[0], v.wo[1], v.wo[2], cnt, safe, false, false, kAniso, 0, i,
+    uint32_t st = dda_steps_mode<false, kGlsl>(s, w, v.wo[0], v.wo[1], v.wo[2], cnt, false, false, kAniso, 0, i,
                                                 v.max_iters);
     if (v.max_iters == 0) st = kStepOut;
     const bool hit = st == kStepHit && i < v.max_iters;
     uint32_t texel;
     float d;
-    gbuffer_texel<kGlsl>(s, hit, gp.palette[s.material], gp.proj, texel, d);
+    const uint32_t material = hit_material(s, w.payload, hit);
+    gbuffer_texel<kGlsl>(s, hit, gp.palette[material], gp.proj, texel, d);
     tex[pixel] = texel;
     depth[pixel] = d;
-    if (out) out[pixel] = pack_state<kGlsl>(s, hit, i, pixel);
+    if (out) out[pixel] = pack_state<kGlsl>(s, material, hit, i, pixel);
 }
 
 vrt_status launch_gbuffer(vrt_world* w, const vrt_view* view, const uint32_t* palette, const float* proj,
@@ -92,12 +98,16 @@ vrt_status launch_gbuffer(vrt_world* w, const vrt_view* view, const uint32_t* pa
     const ViewDev v = make_view_dev(*view);
     dim3 block(8, 8), grid((v.width + 7) / 8, (v.height + 7) / 8);
     uint4* out = reinterpret_cast<uint4*>(hits);
+    const DevWorld dw = w->dev();
+    const ClipBox clip = clip_box(dw, v.wo);
+    const bool inside = origin_inside_near(clip, v.ox, v.oy, v.oz);
+    const BoxSides box = box_sides(clip, v.ox, v.oy, v.oz);
     if (view_glsl(*view) && view_aniso(*view))
-        gbuffer_kernel<true, true><<<grid, block, 0, stream>>>(w->dev(), v, gp, tex, depth, out);
+        gbuffer_kernel<true, true><<<grid, block, 0, stream>>>(dw, v, clip, inside, box, gp, tex, depth, out);
     else if (view_glsl(*view))
-        gbuffer_kernel<true, false><<<grid, block, 0, stream>>>(w->dev(), v, gp, tex, depth, out);
+        gbuffer_kernel<true, false><<<grid, block, 0, stream>>>(dw, v, clip, inside, box, gp, tex, depth, out);
     else
-        gbuffer_kernel<false, false><<<grid, block, 0, stream>>>(w->dev(), v, gp, tex, depth, out);
+        gbuffer_kernel<false, false><<<grid, block, 0, stream>>>(dw, v, clip, inside, box, gp, tex, depth, out);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }

@@ -21,33 +21,45 @@ uint32_t eff_iters(uint32_t max_iters, bool glsl = false) {
     return max_iters > 65535u ? 65535u : max_iters;
 }
 
-__global__ void __launch_bounds__(64) render_view_kernel(DevWorld w, vrt_camera cam, uint32_t max_iters,
+// inside: the camera origin is (origin_inside_near); box: its distances to the clip box's sides
+__global__ void __launch_bounds__(64) render_view_kernel(const __grid_constant__ DevWorld w,
+                                                        const __grid_constant__ vrt_camera cam,
+                                                        const __grid_constant__ ClipBox clip, bool inside,
+                                                        const __grid_constant__ BoxSides box, uint32_t max_iters,
                                                         uint4* __restrict__ out) {
     const uint32_t px = blockIdx.x * 8 + threadIdx.x;
     const uint32_t py = blockIdx.y * 8 + threadIdx.y;
     if (px >= cam.width || py >= cam.height) return;
     float dx, dy, dz;
     camera_ray(cam, px, py, dx, dy, dz);
-    TraceResult r;
+    const int32_t wox = cam.world_origin[0], woy = cam.world_origin[1], woz = cam.world_origin[2];
+    RayState s;
+    if (inside)
+        ray_start_inside<false>(s, box, cam.origin[0], cam.origin[1], cam.origin[2], dx, dy, dz, wox, woy, woz);
+    else
+        ray_start<false>(s, clip, cam.origin[0], cam.origin[1], cam.origin[2], dx, dy, dz, wox, woy, woz);
     TraceCounters cnt;
-    trace_ray<false>(w, cam.origin[0], cam.origin[1], cam.origin[2], dx, dy, dz, cam.world_origin[0],
-                     cam.world_origin[1], cam.world_origin[2], max_iters, r, cnt);
+    uint32_t i = 0;
+    const bool hit = dda_steps_mode<false, false>(s, w, wox, woy, woz, cnt, false, false, false, 0, i, max_iters) == kStepHit;
     const uint32_t pix = py * cam.width + px;
-    out[pix] = pack_hit(r, dx, dy, dz, pix);
+    out[pix] = pack_state<false>(s, hit_material(s, w.payload, hit), hit, i, pix);
 }
 
 template <bool kGlsl, bool kAniso = false>
-__global__ void __launch_bounds__(256) cast_kernel(DevWorld w, const float4* __restrict__ rays, uint32_t n,
+__global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ClipBox clip,
+                                                  const float4* __restrict__ rays, uint32_t n,
                                                   int32_t wox, int32_t woy, int32_t woz, uint32_t max_iters,
                                                   uint4* __restrict__ out, bool coarse) {
     if constexpr (kAniso) fill_forward_lut();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
-    TraceResult r;
+    RayState s;
+    ray_start<kGlsl>(s, clip, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, coarse);
     TraceCounters cnt;
-    trace_ray<false, kGlsl>(w, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, max_iters, r, cnt, coarse, kAniso);
-    out[i] = pack_hit<kGlsl>(r, a.w, b.x, b.y, __float_as_uint(b.z));
+    uint32_t k = 0;
+    const bool hit = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, k, max_iters) == kStepHit;
+    out[i] = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, k, __float_as_uint(b.z));
 }
 
 // Explicit rays whose lengths vary widely (random origins and directions: some hit at
@@ -60,7 +72,8 @@ __global__ void __launch_bounds__(256) cast_kernel(DevWorld w, const float4* __r
 // cast_kernel: a lane's steps continue from where its ray left off, and a ray's record
 // is packed from the state at its exit.
 template <bool kGlsl, bool kAniso = false>
-__global__ void __maxnreg__(48) cast_persistent_kernel(DevWorld w, const float4* __restrict__ rays, uint32_t n,
+__global__ void __maxnreg__(48) cast_persistent_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ClipBox clip,
+                                                             const float4* __restrict__ rays, uint32_t n,
                                                              int32_t wox, int32_t woy, int32_t woz, uint32_t max_iters,
                                                              uint32_t inner, uint32_t refill, uint4* __restrict__ out,
                                                              bool coarse) {
@@ -69,13 +82,13 @@ __global__ void __maxnreg__(48) cast_persistent_kernel(DevWorld w, const float4*
     const uint32_t stride = (gridDim.x * blockDim.x) & ~31u;  // rays between a warp's chunks
     uint32_t next = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;  // first ray of the warp's next chunk
     uint32_t q_next = 0, q_end = 0;
-    bool active = false, ended = false, hit = false, safe = false;
+    bool active = false, ended = false, hit = false;
     uint32_t ri = 0, iter = 0, tag = 0;
     RayState s;
     TraceCounters cnt{0, 0};
     for (;;) {
         if (ended) {
-            out[ri] = pack_state<kGlsl>(s, hit, iter, tag);
+            out[ri] = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, iter, tag);
             ended = false;
             active = false;
         }
@@ -97,7 +110,7 @@ __global__ void __maxnreg__(48) cast_persistent_kernel(DevWorld w, const float4*
                     ri = q_next + rank;
                     const float4 a = __ldg(rays + 2 * (size_t)ri), b = __ldg(rays + 2 * (size_t)ri + 1);
                     tag = __float_as_uint(b.z);
-                    safe = ray_start<kGlsl>(s, w, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, false, coarse);
+                    ray_start<kGlsl>(s, clip, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, coarse);
                     iter = 0;
                     active = true;
                 }
@@ -106,13 +119,12 @@ __global__ void __maxnreg__(48) cast_persistent_kernel(DevWorld w, const float4*
             }
         }
         if (__ballot_sync(0xffffffffu, active) == 0) break;
-        const bool all_safe = __all_sync(0xffffffffu, !active || safe);
         if (active) {
             const uint32_t kmax = min(inner, max_iters - iter);
             uint32_t k = 0;
             // GLSL variants (rayCastCoarse, anisotropic LODs) are uniform over the launch
-            const uint32_t st = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, all_safe, coarse, coarse, kAniso,
-                                                             iter, k, kmax);
+            const uint32_t st = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, iter, k,
+                                                             kmax);
             iter += k;
             if (st != kStepContinue || iter >= max_iters) {
                 ended = true;
@@ -138,16 +150,21 @@ vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters
     L2Window l2;
     vrt_status st = l2.enter(w, stream);
     if (st != VRT_OK) return st;
-    render_view_kernel<<<grid, block, 0, stream>>>(w->dev(), *cam, eff_iters(max_iters),
+    const DevWorld dw = w->dev();
+    const float* o = cam->origin;
+    const ClipBox clip = clip_box(dw, cam->world_origin);
+    render_view_kernel<<<grid, block, 0, stream>>>(dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]),
+                                                   box_sides(clip, o[0], o[1], o[2]), eff_iters(max_iters),
                                                    reinterpret_cast<uint4*>(hits));
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }
 
 // Launch shape of cast_persistent_kernel (also capped at 48 registers, for more warps to hide
-// L2 latency): measured on GB300 with the 2^26 random rays
-// of the incoherent workload.
-constexpr uint32_t kCastThreads = 128, kCastInner = 12, kCastRefill = 28;
+// L2 latency: 40 and 56 measured 301 and 292 us against 286).  On 4.2 M random rays in a
+// 512-voxel world, slices of 8 steps take 268 us, of 12 steps (the best of the step before)
+// 285 us and of 16 steps 291 us.
+constexpr uint32_t kCastThreads = 128, kCastInner = 8, kCastRefill = 28;
 // Below this many rays the thread-per-ray kernel is used (too few rays to fill the
 // persistent grid's lanes twice).
 constexpr uint32_t kCastPersistentMin = 1u << 18;
@@ -161,12 +178,14 @@ vrt_status launch_cast(vrt_world* w, const vrt_ray* rays, uint32_t n, const vrt_
     uint4* o4 = reinterpret_cast<uint4*>(hits);
     uint32_t iters = eff_iters(p->max_iters, glsl);
     if (coarse) iters = std::min<uint32_t>(iters, VRT_GLSL_COARSE_MAX_ITERS);
+    const DevWorld dw = w->dev();
+    const ClipBox clip = clip_box(dw, p->world_origin);
     L2Window l2;
     vrt_status st = l2.enter(w, stream);
     if (st != VRT_OK) return st;
     if (n < kCastPersistentMin) {
         auto kernel = glsl ? (aniso ? cast_kernel<true, true> : cast_kernel<true>) : cast_kernel<false>;
-        kernel<<<(n + 255) / 256, 256, 0, stream>>>(w->dev(), r4, n, p->world_origin[0], p->world_origin[1],
+        kernel<<<(n + 255) / 256, 256, 0, stream>>>(dw, clip, r4, n, p->world_origin[0], p->world_origin[1],
                                                     p->world_origin[2], iters, o4, coarse);
     } else {
         auto kernel = glsl ? (aniso ? cast_persistent_kernel<true, true> : cast_persistent_kernel<true>)
@@ -176,7 +195,7 @@ vrt_status launch_cast(vrt_world* w, const vrt_ray* rays, uint32_t n, const vrt_
         VRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         VRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kCastThreads, 0));
         const uint32_t blocks = (uint32_t)(sms * std::max(occ, 1));
-        kernel<<<blocks, kCastThreads, 0, stream>>>(w->dev(), r4, n, p->world_origin[0], p->world_origin[1],
+        kernel<<<blocks, kCastThreads, 0, stream>>>(dw, clip, r4, n, p->world_origin[0], p->world_origin[1],
                                                     p->world_origin[2], iters, kCastInner, kCastRefill, o4, coarse);
     }
     VRT_CUDA(cudaGetLastError());

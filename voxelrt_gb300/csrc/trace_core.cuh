@@ -38,6 +38,55 @@ __device__ __forceinline__ uint32_t imad(uint32_t a, uint32_t b, uint32_t c) {
     return a * b + c;
 #endif
 }
+// a + b rounded down.
+__device__ __forceinline__ float add_rd(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fadd_rd(a, b);
+#else
+    // f - b is exact in double here (f and b are close, or f is an infinity or NaN)
+    float f = (float)((double)a + (double)b);
+    if ((double)f - (double)b > (double)a) {
+        uint32_t u = __float_as_uint(f);
+        u = f > 0.0f ? u - 1u : (f < 0.0f ? u + 1u : 0x80000001u);
+        f = __uint_as_float(u);
+    }
+    return f;
+#endif
+}
+
+// a * 2^-3 + b rounded down, for a * 2^-3 exact.
+__device__ __forceinline__ float eighth_add_rd(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fmaf_rd(a, 0.125f, b);
+#else
+    return add_rd(a * 0.125f, b);
+#endif
+}
+
+// Voxel coordinates as floats with an integer part in the low bits.  kVoxelBias is the
+// bit pattern of M = 1.5 * 2^23, where one ulp is 1: for an integer |n| < 2^22 the float
+// M + n has the bits kVoxelBias + n.  With a near world origin the float K = M + worldOrigin
+// is exact, and add_rd(pos, K) is M + worldOrigin + floor(pos): one add on the FMA pipe takes
+// the place of a conversion (on a quarter-rate unit, the longest latency in the step's chain)
+// and of the add of worldOrigin.  A position out of the grid, an infinity or NaN among them,
+// gives bits below kVoxelBias or at least the grid's size above it (unsigned).  Back in the ray frame, the float minus K is exactly
+// voxel - worldOrigin.
+constexpr uint32_t kVoxelBias = 0x4B400000u;
+// The brick coordinate of a voxel in the grid the same way: from the biased voxel r the
+// float 2^23 + (v >> 3), bits kBrickBias + (v >> 3).
+constexpr uint32_t kBrickBias = 0x4B000000u;
+__device__ __forceinline__ uint32_t biased_brick(float r) {
+    return __float_as_uint(eighth_add_rd(r, 8388608.0f - 12582912.0f / 8.0f));
+}
+// Table address that takes a biased brick index bx + bz*bsx + by*bsxz: the biases add up to
+// kBrickBias * (1 + bsx + bsxz) mod 2^32, a multiple of 2^24, and a table has at most 2^23
+// entries, so the 32-bit index never wraps past its bias.
+__device__ __forceinline__ const uint32_t* biased_table(const DevWorld& w) {
+    return w.bricks - (size_t)(kBrickBias * (1u + w.bsx + w.bsxz));
+}
+// K of an axis
+__device__ __forceinline__ float voxel_frame(int32_t wo) { return __uint_as_float(kVoxelBias + (uint32_t)wo); }
+
 // v - worldOrigin (wrapping), the ray-frame coordinate of a voxel
 __device__ __forceinline__ float rel_voxel(int32_t v, int32_t wo) {
     return __int2float_rn((int32_t)imad((uint32_t)wo, 0xFFFFFFFFu, (uint32_t)v));
@@ -47,7 +96,7 @@ struct TraceResult {
     float cx, cy, cz;  // final position (HitResult.Pos)
     float sx, sy, sz;  // final side distances
     float tb;          // GLSL mode: biased tmin of the last step (hit.dist)
-    int32_t vx, vy, vz;
+    uint32_t voxel;    // of a hit, as the record packs it
     uint32_t steps;
     uint32_t material;
     bool hit;
@@ -98,41 +147,72 @@ struct RayState {
     float tsx, tsy, tsz;  // tStart
     float cx, cy, cz;     // currPos
     float sx, sy, sz;     // sideDist
-    float tb;             // GLSL mode: biased tmin of the last step
-    int32_t vx, vy, vz;   // voxel of the last step (hit voxel on a hit)
+    float tb;             // biased tmin of the last step, the distance of the current position (0 at the start)
+    float t_lo, t_hi;     // positions at distances in [t_lo, t_hi) are in the grid (ray_init)
     int32_t gx, gy, gz;   // -1 where dir < 0, else 0 (cell alignment side)
-    uint32_t material;
+    // A hit ends the use of tStart: the step that hits leaves the voxel (as the record packs
+    // it) and the brick's slot there, so a lane waiting for its retirement holds no more.
+    __device__ __forceinline__ void set_hit(uint32_t x, uint32_t y, uint32_t z, uint32_t slot) {
+        tsx = __uint_as_float(imad(z, 1u << 21, imad(y, 1u << 11, x)));
+        tsy = __uint_as_float(slot);
+    }
+    __device__ __forceinline__ uint32_t hit_voxel() const { return __float_as_uint(tsx); }
+    __device__ __forceinline__ size_t hit_byte() const {  // of the payload
+        const uint32_t v = __float_as_uint(tsx);
+        return (size_t)__float_as_uint(tsy) * 512 + ((v & 7u) | ((v >> 21) & 7u) << 3 | ((v >> 11) & 7u) << 6);
+    }
 };
 
-// Bounds that keep a ray free of NaN and infinities inside the DDA loop: with
-// |origin| < 2^30 and |1/dir| < 2^95, |tStart| and |(voxel - worldOrigin) * invDir|
-// stay below 2^126 (voxel - worldOrigin < 2^31), so side distances and t are finite,
-// and the position o + t*dir is finite or an infinity (never NaN) that leaves the grid.
-constexpr float kSafeOrigin = 0x1p30f, kSafeInvDir = 0x1p95f;
+// A ray takes the fast step (ray_step<.., true>) while its distance lies in [t_lo, t_hi), where
+// it cannot leave the grid nor meet a NaN, and the general step elsewhere.  The range is empty
+// unless the ray is near and steep enough for these bounds:
+// - |worldOrigin| <= 2^16 and |origin| <= 2^17, so positions in the grid are rounded by less
+//   than 2^-6 and voxels have their biased form;
+// - |1/dir| < 2^95: |tStart| and |(voxel - worldOrigin) * invDir| stay below 2^126, so side
+//   distances and t are finite.
+// The range's ends are where the ray enters (0 when the origin is strictly inside) and leaves
+// the clip box, whose sides lie a voxel inside the grid's: at a distance between them the
+// position o + t*d is within the box on every axis up to the rounding of the ends, of t*d and
+// of the sum, together less than 2^-3.
+constexpr int32_t kNearWorldOrigin = 1 << 16;
+constexpr float kNearOrigin = 0x1p17f, kSafeInvDir = 0x1p95f;
 
-// The clip box [1 - worldOrigin, size - 1 - worldOrigin] (VoxelTraversal.glsl:166) holds
-// the origin strictly inside, and the origin is within the safe bound: ray_init then
-// needs neither the slab test nor the origin's bound check.  Camera rays of a view
-// share their origin, so the persistent kernel evaluates this once per queue chunk.
-__device__ __forceinline__ bool origin_inside_safe(const DevWorld& w, float ox, float oy, float oz, int32_t wox,
-                                                   int32_t woy, int32_t woz) {
-    const float lx = __int2float_rn(1 - wox), ly = __int2float_rn(1 - woy), lz = __int2float_rn(1 - woz);
-    const float hx = __fsub_rn(__fsub_rn(__uint2float_rn(w.size_x), __int2float_rn(wox)), 1.0f);
-    const float hy = __fsub_rn(__fsub_rn(__uint2float_rn(w.size_y), __int2float_rn(woy)), 1.0f);
-    const float hz = __fsub_rn(__fsub_rn(__uint2float_rn(w.size_z), __int2float_rn(woz)), 1.0f);
-    return lx < ox && ox < hx && ly < oy && oy < hy && lz < oz && oz < hz && fabsf(ox) < kSafeOrigin &&
-           fabsf(oy) < kSafeOrigin && fabsf(oz) < kSafeOrigin;
+// The clip box [1 - worldOrigin, size - 1 - worldOrigin] (VoxelTraversal.glsl:166) of a world
+// origin, and whether that is near: the same for every ray of a view or cast.
+struct ClipBox {
+    float lo[3], hi[3];
+    uint32_t near;
+};
+VRT_HD inline ClipBox clip_box(const DevWorld& w, const int32_t wo[3]) {
+    const uint32_t size[3] = {w.size_x, w.size_y, w.size_z};
+    ClipBox b;
+    b.near = 1;
+    for (int c = 0; c < 3; c++) {
+        b.lo[c] = (float)(1 - wo[c]);
+        b.hi[c] = ((float)size[c] - (float)wo[c]) - 1.0f;
+        if ((uint32_t)wo[c] + (uint32_t)kNearWorldOrigin > 2u * (uint32_t)kNearWorldOrigin) b.near = 0;
+    }
+    return b;
+}
+// The box holds the origin strictly inside, and the world origin is near: a ray's start then
+// needs neither the slab test nor the bounds of the origin.  Camera rays of a view share
+// their origin, so this is evaluated once per view, or per claimed chunk.
+VRT_HD inline bool origin_inside_near(const ClipBox& b, float ox, float oy, float oz) {
+    return b.near && b.lo[0] < ox && ox < b.hi[0] && b.lo[1] < oy && oy < b.hi[1] && b.lo[2] < oz && oz < b.hi[2];
+}
+// The distances from an origin to the box's sides, per axis the low and the high one.
+struct BoxSides {
+    float lo[3], hi[3];
+};
+VRT_HD inline BoxSides box_sides(const ClipBox& b, float ox, float oy, float oz) {
+    return BoxSides{{b.lo[0] - ox, b.lo[1] - oy, b.lo[2] - oz}, {b.hi[0] - ox, b.hi[1] - oy, b.hi[2] - oz}};
 }
 
-// invDir, tStart and the clipped start position (VoxelTraversal.glsl:133-145,163-167).
-// Returns whether the ray is safe in the sense above (ray_step<kCount, true> applies).
-// inside_safe: origin_inside_safe() is known to hold for this origin.
-__device__ __forceinline__ bool ray_init(RayState& s, const DevWorld& w, float ox, float oy, float oz, float dx,
-                                         float dy, float dz, int32_t wox, int32_t woy, int32_t woz,
-                                         bool inside_safe = false) {
-    s.ox = ox;
-    s.oy = oy;
-    s.oz = oz;
+// What every start sets: origin, direction, invDir, tStart, the alignment sides.
+__device__ __forceinline__ void ray_set(RayState& s, float ox, float oy, float oz, float dx, float dy, float dz) {
+    s.ox = s.cx = ox;
+    s.oy = s.cy = oy;
+    s.oz = s.cz = oz;
     s.dx = dx;
     s.dy = dy;
     s.dz = dz;
@@ -143,68 +223,108 @@ __device__ __forceinline__ bool ray_init(RayState& s, const DevWorld& w, float o
     s.tsx = __fmul_rn(__fsub_rn(dx < 0.0f ? 0.0f : 1.0f, ox), s.ix);
     s.tsy = __fmul_rn(__fsub_rn(dy < 0.0f ? 0.0f : 1.0f, oy), s.iy);
     s.tsz = __fmul_rn(__fsub_rn(dz < 0.0f ? 0.0f : 1.0f, oz), s.iz);
-    // An origin strictly inside the clip box never clips: per axis l - o < 0 < h - o,
-    // so min(t1, t2) is negative (or -inf, or NaN when dir is NaN, which minps/maxps
-    // drop) and tmin <= 0 on every path.  Camera rays of a view share the origin, so
-    // the slab test below runs only for views from outside the world.
-    bool clip = false;
-    float tmin = 0.0f;
-    bool origin_ok = true;
-    if (!inside_safe && !origin_inside_safe(w, ox, oy, oz, wox, woy, woz)) {
-        // clip box [1 - worldOrigin, size - 1 - worldOrigin] (VoxelTraversal.glsl:166)
-        const float lx = __int2float_rn(1 - wox), ly = __int2float_rn(1 - woy), lz = __int2float_rn(1 - woz);
-        const float hx = __fsub_rn(__fsub_rn(__uint2float_rn(w.size_x), __int2float_rn(wox)), 1.0f);
-        const float hy = __fsub_rn(__fsub_rn(__uint2float_rn(w.size_y), __int2float_rn(woy)), 1.0f);
-        const float hz = __fsub_rn(__fsub_rn(__uint2float_rn(w.size_z), __int2float_rn(woz)), 1.0f);
-        const float t1x = __fmul_rn(__fsub_rn(lx, ox), s.ix);
-        const float t1y = __fmul_rn(__fsub_rn(ly, oy), s.iy);
-        const float t1z = __fmul_rn(__fsub_rn(lz, oz), s.iz);
-        const float t2x = __fmul_rn(__fsub_rn(hx, ox), s.ix);
-        const float t2y = __fmul_rn(__fsub_rn(hy, oy), s.iy);
-        const float t2z = __fmul_rn(__fsub_rn(hz, oz), s.iz);
-        tmin = max_x86(min_x86(t1x, t2x), max_x86(min_x86(t1y, t2y), min_x86(t1z, t2z)));
-        const float tmax = min_x86(max_x86(t1x, t2x), min_x86(max_x86(t1y, t2y), max_x86(t1z, t2z)));
-        clip = tmin > 0.0f && tmin < tmax;
-        origin_ok = fabsf(ox) < kSafeOrigin && fabsf(oy) < kSafeOrigin && fabsf(oz) < kSafeOrigin;
-    }
-    s.cx = clip ? __fadd_rn(ox, __fmul_rn(dx, tmin)) : ox;
-    s.cy = clip ? __fadd_rn(oy, __fmul_rn(dy, tmin)) : oy;
-    s.cz = clip ? __fadd_rn(oz, __fmul_rn(dz, tmin)) : oz;
-    s.sx = s.sy = s.sz = 0.0f;
-    s.vx = s.vy = s.vz = INT32_MIN;
     s.gx = dx < 0.0f ? -1 : 0;
     s.gy = dy < 0.0f ? -1 : 0;
     s.gz = dz < 0.0f ? -1 : 0;
-    s.material = 0;
-    return origin_ok && fabsf(s.ix) < kSafeInvDir && fabsf(s.iy) < kSafeInvDir && fabsf(s.iz) < kSafeInvDir;
+    s.sx = s.sy = s.sz = s.tb = s.t_lo = 0.0f;
+}
+__device__ __forceinline__ bool ray_finite(const RayState& s) {
+    return fabsf(s.ix) < kSafeInvDir && fabsf(s.iy) < kSafeInvDir && fabsf(s.iz) < kSafeInvDir;
 }
 
-// GLSL mode (VoxelTraversal.glsl rayCast): the start voxel worldOrigin + floor(start),
-// from which iteration 0 takes its side distances (:164-167).
-template <bool kGlsl>
+// Start of a ray whose origin is inside and near.  Such an origin never clips: per axis
+// l - o < 0 < h - o, so min(t1, t2) of the slab test is negative (or -inf, or NaN when dir is
+// NaN, which minps/maxps drop) and tmin <= 0 on every path.
+__device__ __forceinline__ void ray_init_inside(RayState& s, const BoxSides& b, float ox, float oy, float oz, float dx,
+                                                float dy, float dz) {
+    ray_set(s, ox, oy, oz, dx, dy, dz);
+    const float t = fminf(fminf(__fmul_rn(dx < 0.0f ? b.lo[0] : b.hi[0], s.ix), __fmul_rn(dy < 0.0f ? b.lo[1] : b.hi[1], s.iy)),
+                          __fmul_rn(dz < 0.0f ? b.lo[2] : b.hi[2], s.iz));
+    s.t_hi = ray_finite(s) ? t : 0.0f;
+}
+
+// Start of any ray: the clipped start position (VoxelTraversal.glsl:133-145,163-167) and the
+// range of the fast step.
+__device__ __forceinline__ void ray_init(RayState& s, const ClipBox& b, float ox, float oy, float oz, float dx,
+                                         float dy, float dz) {
+    const BoxSides d = box_sides(b, ox, oy, oz);
+    if (origin_inside_near(b, ox, oy, oz)) {
+        ray_init_inside(s, d, ox, oy, oz, dx, dy, dz);
+        return;
+    }
+    ray_set(s, ox, oy, oz, dx, dy, dz);
+    const float t1x = __fmul_rn(d.lo[0], s.ix), t1y = __fmul_rn(d.lo[1], s.iy), t1z = __fmul_rn(d.lo[2], s.iz);
+    const float t2x = __fmul_rn(d.hi[0], s.ix), t2y = __fmul_rn(d.hi[1], s.iy), t2z = __fmul_rn(d.hi[2], s.iz);
+    const float tmin = max_x86(min_x86(t1x, t2x), max_x86(min_x86(t1y, t2y), min_x86(t1z, t2z)));
+    const float tmax = min_x86(max_x86(t1x, t2x), min_x86(max_x86(t1y, t2y), max_x86(t1z, t2z)));
+    s.t_hi = 0.0f;
+    if (tmin > 0.0f && tmin < tmax) {
+        s.cx = __fadd_rn(ox, __fmul_rn(dx, tmin));
+        s.cy = __fadd_rn(oy, __fmul_rn(dy, tmin));
+        s.cz = __fadd_rn(oz, __fmul_rn(dz, tmin));
+        if (b.near && ray_finite(s) && fabsf(ox) < kNearOrigin && fabsf(oy) < kNearOrigin && fabsf(oz) < kNearOrigin) {
+            s.tb = s.t_lo = tmin;
+            s.t_hi = tmax;
+        }
+    }
+}
+
+// GLSL mode: the step's distance and position from its side distances.  tmin + 5 ulp as
+// an integer add on the bits; a NaN tmin stays NaN (its bit pattern differs between
+// platforms: the GPU's 0x7FFFFFFF would wrap to a denormal).  A rayCastCoarse ray takes
+// tmin + 0.001 (VoxelTraversal.glsl:213).  Kept as the hit distance, so min keeps the minps
+// rule.
+template <bool kSafe>
+__device__ __forceinline__ void glsl_advance(RayState& s, bool coarse_ray) {
+    const float m = min_x86(min_x86(s.sx, s.sy), s.sz);
+    const float t = coarse_ray ? __fadd_rn(m, 0.001f) : (!kSafe && m != m) ? m : __uint_as_float(__float_as_uint(m) + 5u);
+    s.tb = t;
+    s.cx = __fadd_rn(s.ox, __fmul_rn(t, s.dx));
+    s.cy = __fadd_rn(s.oy, __fmul_rn(t, s.dy));
+    s.cz = __fadd_rn(s.oz, __fmul_rn(t, s.dz));
+}
+
+// GLSL mode (VoxelTraversal.glsl rayCast): the start voxel worldOrigin + floor(start), and
+// the side distances and position that iteration 0 takes from it (:164-174), so that a step
+// of either mode begins with its position and ends with the next one.
 // coarse_origin (GLSL mode, a rayCastCoarse ray): the clipped start replaces the origin,
 // so tStart, positions and the hit distance count from it (VoxelTraversal.glsl:207-210);
 // rayCast keeps the origin and starts from the clipped voxel only (:162-167).  Without
 // a clip the start is the origin and nothing changes.
-__device__ __forceinline__ bool ray_start(RayState& s, const DevWorld& w, float ox, float oy, float oz, float dx,
-                                          float dy, float dz, int32_t wox, int32_t woy, int32_t woz,
-                                          bool inside_safe = false, bool coarse_origin = false) {
-    const bool safe = ray_init(s, w, ox, oy, oz, dx, dy, dz, wox, woy, woz, inside_safe);
-    if (kGlsl && coarse_origin) {
+template <bool kGlsl>
+__device__ __forceinline__ void glsl_start(RayState& s, int32_t wox, int32_t woy, int32_t woz, bool coarse_origin) {
+    if (!kGlsl) return;
+    if (coarse_origin) {
         s.ox = s.cx;
         s.oy = s.cy;
         s.oz = s.cz;
-        s.tsx = __fmul_rn(__fsub_rn(dx < 0.0f ? 0.0f : 1.0f, s.ox), s.ix);
-        s.tsy = __fmul_rn(__fsub_rn(dy < 0.0f ? 0.0f : 1.0f, s.oy), s.iy);
-        s.tsz = __fmul_rn(__fsub_rn(dz < 0.0f ? 0.0f : 1.0f, s.oz), s.iz);
+        s.tsx = __fmul_rn(__fsub_rn(s.dx < 0.0f ? 0.0f : 1.0f, s.ox), s.ix);
+        s.tsy = __fmul_rn(__fsub_rn(s.dy < 0.0f ? 0.0f : 1.0f, s.oy), s.iy);
+        s.tsz = __fmul_rn(__fsub_rn(s.dz < 0.0f ? 0.0f : 1.0f, s.oz), s.iz);
+        // distances count from the clipped start, and so do the range's ends
+        s.t_hi = s.t_hi > 0.0f ? __fsub_rn(s.t_hi, s.t_lo) : 0.0f;
+        s.t_lo = 0.0f;
     }
-    if (kGlsl) {
-        s.vx = wadd(wox, floor2i(s.cx));
-        s.vy = wadd(woy, floor2i(s.cy));
-        s.vz = wadd(woz, floor2i(s.cz));
-        s.tb = 0.0f;
-    }
-    return safe;
+    // (voxel - worldOrigin in wrapping arithmetic, where the start voxel saturated)
+    s.sx = __fadd_rn(s.tsx, __fmul_rn(rel_voxel(wadd(wox, floor2i(s.cx)), wox), s.ix));
+    s.sy = __fadd_rn(s.tsy, __fmul_rn(rel_voxel(wadd(woy, floor2i(s.cy)), woy), s.iy));
+    s.sz = __fadd_rn(s.tsz, __fmul_rn(rel_voxel(wadd(woz, floor2i(s.cz)), woz), s.iz));
+    glsl_advance<false>(s, coarse_origin);
+}
+
+// A ray's start, and that of a ray whose origin is inside and near (origin_inside_near).
+template <bool kGlsl>
+__device__ __forceinline__ void ray_start(RayState& s, const ClipBox& b, float ox, float oy, float oz, float dx,
+                                          float dy, float dz, int32_t wox, int32_t woy, int32_t woz,
+                                          bool coarse_origin = false) {
+    ray_init(s, b, ox, oy, oz, dx, dy, dz);
+    glsl_start<kGlsl>(s, wox, woy, woz, coarse_origin);
+}
+template <bool kGlsl>
+__device__ __forceinline__ void ray_start_inside(RayState& s, const BoxSides& b, float ox, float oy, float oz, float dx,
+                                                 float dy, float dz, int32_t wox, int32_t woy, int32_t woz) {
+    ray_init_inside(s, b, ox, oy, oz, dx, dy, dz);
+    glsl_start<kGlsl>(s, wox, woy, woz, false);
 }
 
 enum : uint32_t { kStepContinue = 0, kStepHit = 1, kStepOut = 2 };
@@ -246,58 +366,82 @@ __device__ __forceinline__ uint32_t coarse_bits(bool coarse_ray, uint32_t i) {
     return coarse_ray ? (kCoarseRay | (i >= kCoarseFrom ? kCoarseNow : 0u)) : 0u;
 }
 
-// One iteration of RayCast (CpuRenderer.cpp:186-201) with GetStepPos (:135-171).
-// kSafe: the ray passed the bounds of ray_init, so no NaN can occur; the NaN test
-// is skipped and min uses fminf, which equals the minps rule on non-NaN operands up
-// to the sign of a zero result, which the +0.001 bias removes.
-// kGlsl: one iteration of rayCast (VoxelTraversal.glsl:170-199) instead: side
-// distances of the current voxel, tmin + 5 ulp (kept as the hit distance, so min
-// keeps the minps rule), position, bounds, then getStepPos (:100-131) whose empty
-// sectors take the 4th-level mask from the brick table.  kCoarse (with kGlsl): the
-// step may belong to a rayCastCoarse ray, as `coarse` (coarse_bits) says: tmin + 0.001
-// (:213) instead, and from iteration 31 an empty voxel whose 4^3 cell holds a solid
-// voxel stops the ray at the cell's first solid voxel in mask order (getStepPos with
-// coarse, :125-128, and findAnyOccupiedPos, :41-53).  Without kCoarse `coarse` is 0.
-// kAniso (with kGlsl): anisotropic LODs (u_UseAnisotropicLods, :116-121): the mask of
-// the current level (cell, sector or sector group, read raw instead of through the
-// precomputed codes) is restricted to the cells ahead of the ray before its LOD is taken.
-template <bool kCount, bool kSafe = false, bool kGlsl = false, bool kCoarse = false, bool kAniso = false>
-__device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int32_t wox, int32_t woy, int32_t woz,
-                                             TraceCounters& cnt, uint32_t coarse = 0) {
+// The end of a step: from the voxel (of a safe ray in its biased form) and the alignment
+// mask of its cell to the cell's side distances, tmin and the next position.
+template <bool kSafe, bool kGlsl, bool kCoarse>
+__device__ __forceinline__ void step_on(RayState& s, uint32_t vx, uint32_t vy, uint32_t vz, uint32_t m, int32_t wox,
+                                        int32_t woy, int32_t woz, uint32_t coarse) {
+    // dir < 0 ? pos & ~m : pos | m, as (pos | m) ^ (g & m) with g = -1 for dir < 0
+    vx = (vx | m) ^ ((uint32_t)s.gx & m);
+    vy = (vy | m) ^ ((uint32_t)s.gy & m);
+    vz = (vz | m) ^ ((uint32_t)s.gz & m);
+    const float fx = kSafe ? __fsub_rn(__uint_as_float(vx), voxel_frame(wox)) : rel_voxel((int32_t)vx, wox);
+    const float fy = kSafe ? __fsub_rn(__uint_as_float(vy), voxel_frame(woy)) : rel_voxel((int32_t)vy, woy);
+    const float fz = kSafe ? __fsub_rn(__uint_as_float(vz), voxel_frame(woz)) : rel_voxel((int32_t)vz, woz);
+    s.sx = __fadd_rn(s.tsx, __fmul_rn(fx, s.ix));
+    s.sy = __fadd_rn(s.tsy, __fmul_rn(fy, s.iy));
+    s.sz = __fadd_rn(s.tsz, __fmul_rn(fz, s.iz));
     if (kGlsl) {
-        s.sx = __fadd_rn(s.tsx, __fmul_rn(rel_voxel(s.vx, wox), s.ix));
-        s.sy = __fadd_rn(s.tsy, __fmul_rn(rel_voxel(s.vy, woy), s.iy));
-        s.sz = __fadd_rn(s.tsz, __fmul_rn(rel_voxel(s.vz, woz), s.iz));
-        // +5 ulp as an integer add on the bits; a NaN tmin stays NaN (its bit pattern
-        // differs between platforms: the GPU's 0x7FFFFFFF would wrap to a denormal)
-        const float m = min_x86(min_x86(s.sx, s.sy), s.sz);
-        const float t = (kCoarse && (coarse & kCoarseRay)) ? __fadd_rn(m, 0.001f)
-                        : (!kSafe && m != m) ? m
-                                             : __uint_as_float(__float_as_uint(m) + 5u);
+        glsl_advance<kSafe>(s, kCoarse && (coarse & kCoarseRay) != 0);
+    } else {
+        const float t = kSafe ? __fadd_rn(fminf(fminf(s.sx, s.sy), s.sz), 0.001f)
+                              : __fadd_rn(min_x86(min_x86(s.sx, s.sy), s.sz), 0.001f);
         s.tb = t;
         s.cx = __fadd_rn(s.ox, __fmul_rn(t, s.dx));
         s.cy = __fadd_rn(s.oy, __fmul_rn(t, s.dy));
         s.cz = __fadd_rn(s.oz, __fmul_rn(t, s.dz));
     }
-    // floor2i: a NaN coordinate converts to INT32_MIN on x86 and leaves the grid;
-    // cvt.rmi saturates infinities and out-of-range values, which leave the grid
-    // too (|world origin| <= 2^30 is enforced at the API), so only NaN needs a test
-    // and one NaN among the three shows in their sum.
-    if (!kSafe) {
+}
+
+// One iteration of RayCast (CpuRenderer.cpp:186-201) with GetStepPos (:135-171): the voxel
+// of the current position, its bounds and table entries, then the side distances of the cell
+// reached, tmin and the next position.
+// kSafe: the distance lies in the ray's range of ray_init, so the position is in the grid, no
+// NaN can occur and voxels are kept in the biased form of kVoxelBias; min uses fminf, which
+// equals the minps rule on non-NaN operands up to the sign of a zero result, which the +0.001
+// bias removes.
+// kGlsl: rayCast (VoxelTraversal.glsl:170-199), whose iteration takes its position first
+// (ray_start has iteration 0's): bounds, then getStepPos (:100-131), whose empty sectors take
+// the 4th-level mask from the brick table.  kCoarse (with kGlsl): the step may belong to a
+// rayCastCoarse ray, as `coarse` (coarse_bits) says: from iteration 31 an empty voxel whose
+// 4^3 cell holds a solid voxel stops the ray at the cell's first solid voxel in mask order
+// (getStepPos with coarse, :125-128, and findAnyOccupiedPos, :41-53).  Without kCoarse
+// `coarse` is 0.
+// kAniso (with kGlsl): anisotropic LODs (u_UseAnisotropicLods, :116-121): the mask of
+// the current level (cell, sector or sector group, read raw instead of through the
+// precomputed codes) is restricted to the cells ahead of the ray before its LOD is taken.
+template <bool kCount, bool kSafe = false, bool kGlsl = false, bool kCoarse = false, bool kAniso = false>
+__device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, const uint32_t* biased, int32_t wox,
+                                             int32_t woy, int32_t woz, TraceCounters& cnt, uint32_t coarse = 0) {
+    uint32_t vx, vy, vz;  // the voxel; of a safe ray its biased form
+    uint32_t bx, by, bz;  // its brick, likewise
+    uint32_t e;
+    constexpr uint32_t kBias = kSafe ? kVoxelBias : 0u;
+    if (kSafe) {
+        const float rx = add_rd(s.cx, voxel_frame(wox)), ry = add_rd(s.cy, voxel_frame(woy)),
+                    rz = add_rd(s.cz, voxel_frame(woz));
+        vx = __float_as_uint(rx);
+        vy = __float_as_uint(ry);
+        vz = __float_as_uint(rz);
+        bx = biased_brick(rx);
+        by = biased_brick(ry);
+        bz = biased_brick(rz);
+        e = __ldg(biased + imad(by, w.bsxz, imad(bz, w.bsx, bx)));
+    } else {
+        // floor2i: a NaN coordinate converts to INT32_MIN on x86 and leaves the grid;
+        // cvt.rmi saturates infinities and out-of-range values, which leave the grid
+        // too (|world origin| <= 2^30 is enforced at the API), so only NaN needs a test
+        // and one NaN among the three shows in their sum.
         const float nan_probe = __fadd_rn(__fadd_rn(s.cx, s.cy), s.cz);
-        if (nan_probe != nan_probe) {
-            s.vx = s.vy = s.vz = INT32_MIN;
-            return kStepOut;
-        }
-    }
-    int32_t vx = (int32_t)imad((uint32_t)__float2int_rd(s.cx), 1u, (uint32_t)wox);
-    int32_t vy = (int32_t)imad((uint32_t)__float2int_rd(s.cy), 1u, (uint32_t)woy);
-    int32_t vz = (int32_t)imad((uint32_t)__float2int_rd(s.cz), 1u, (uint32_t)woz);
-    if (!((uint32_t)vx < w.size_x && (uint32_t)vy < w.size_y && (uint32_t)vz < w.size_z)) {
-        s.vx = vx;
-        s.vy = vy;
-        s.vz = vz;
-        return kStepOut;
+        if (nan_probe != nan_probe) return kStepOut;
+        vx = (uint32_t)wadd(__float2int_rd(s.cx), wox);
+        vy = (uint32_t)wadd(__float2int_rd(s.cy), woy);
+        vz = (uint32_t)wadd(__float2int_rd(s.cz), woz);
+        if (!(vx < w.size_x && vy < w.size_y && vz < w.size_z)) return kStepOut;
+        bx = vx >> 3;
+        by = vy >> 3;
+        bz = vz >> 3;
+        e = __ldg(w.bricks + bx + bz * w.bsx + by * w.bsxz);
     }
     if (kCount) cnt.step_calls++;
     // The brick table holds the slot of an allocated brick, or for an empty one the
@@ -305,20 +449,15 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int
     // (3 + skip_levels).  An allocated brick's voxel code is kCodeSolid (the hit) or
     // the alignment mask of the skip level of the voxel's 4^3 cell; both replace the
     // two mask fetches of the reference with their precomputed outcome.
-    const uint32_t bx = (uint32_t)vx >> 3, by = (uint32_t)vy >> 3, bz = (uint32_t)vz >> 3;
-    const uint32_t e = __ldg(w.bricks + bx + bz * w.bsx + by * w.bsxz);
-    int32_t m;
+    uint32_t m;
     if (kGlsl && kAniso) {
         if (e < kBrickEmpty) {
             if (kCount) cnt.occ_fetches++;
-            const uint32_t lx = (uint32_t)vx & 7u, ly = (uint32_t)vy & 7u, lz = (uint32_t)vz & 7u;
+            const uint32_t lx = vx & 7u, ly = vy & 7u, lz = vz & 7u;
             const uint64_t cm = __ldg(w.cells + (size_t)e * 8 + ((lx >> 2) | (lz >> 2) << 1 | (ly >> 2) << 2));
             const uint32_t idx = (lx & 3u) | (lz & 3u) << 2 | (ly & 3u) << 4;
             if ((cm >> idx) & 1u) {
-                s.material = __ldg(w.payload + (size_t)e * 512 + (lx | lz << 3 | ly << 6));
-                s.vx = vx;
-                s.vy = vy;
-                s.vz = vz;
+                s.set_hit(vx - kBias, vy - kBias, vz - kBias, e);
                 return kStepHit;
             }
             const uint32_t li = idx + 64u * ((uint32_t)(s.gx + 1) | (uint32_t)(s.gy + 1) << 1 | (uint32_t)(s.gz + 1) << 2);
@@ -326,98 +465,75 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int
             if (kCoarse && (coarse & kCoarseNow) && am != 0) {
                 // findAnyOccupiedPos on the masked cell mask: its lowest set bit
                 const uint32_t j = (uint32_t)__ffsll((long long)am) - 1u;
-                s.vx = (vx & ~3) | (int32_t)(j & 3u);
-                s.vy = (vy & ~3) | (int32_t)(j >> 4);
-                s.vz = (vz & ~3) | (int32_t)((j >> 2) & 3u);
-                s.material = __ldg(w.payload + (size_t)e * 512 +
-                                   (((uint32_t)s.vx & 7u) | ((uint32_t)s.vz & 7u) << 3 | ((uint32_t)s.vy & 7u) << 6));
+                s.set_hit(((vx - kBias) & ~3u) | (j & 3u), ((vy - kBias) & ~3u) | (j >> 4),
+                          ((vz - kBias) & ~3u) | ((j >> 2) & 3u), e);
                 return kStepHit;
             }
-            m = am == 0 ? 3 : ((cm & s_forward_lut[1][li]) == 0 ? 1 : 0);
+            m = am == 0 ? 3u : ((cm & s_forward_lut[1][li]) == 0 ? 1u : 0u);
         } else {
             // an empty brick: the sector mask (scale 8) or, in an empty sector, the
             // sector-group mask (scale 32) restricted to the ray's octant, whose skip level
             // the table entry carries per octant
             const uint32_t oct2 = ((uint32_t)(s.gx + 1) | (uint32_t)(s.gy + 1) << 1 | (uint32_t)(s.gz + 1) << 2) * 2u;
             const uint32_t skip = ((e >> (kAnisoShift + oct2)) & 3u) + ((e >> 4) & 2u);
-            m = (int32_t)((8u << skip) - 1u);
+            m = (8u << skip) - 1u;
         }
     } else if (e < kBrickEmpty) {
         if (kCount) cnt.occ_fetches++;
-        // voxel in brick v = x | z<<3 | y<<6 from v - 8*(v >> 3) per axis; its code byte
-        const uint32_t lx = imad(bx, 0xFFFFFFF8u, (uint32_t)vx), ly = imad(by, 0xFFFFFFF8u, (uint32_t)vy),
-                       lz = imad(bz, 0xFFFFFFF8u, (uint32_t)vz);
+        // voxel in brick v = x | z<<3 | y<<6 from v - 8*(v >> 3) per axis; its code byte.
+        // The biases of a safe ray's sum (a multiple of 2^22, so v < 512 does not carry)
+        // go into the base address.
+        constexpr uint32_t kViBias = kSafe ? 73u * (kVoxelBias - 8u * kBrickBias) : 0u;
+        const uint32_t lx = imad(bx, 0xFFFFFFF8u, vx), ly = imad(by, 0xFFFFFFF8u, vy), lz = imad(bz, 0xFFFFFFF8u, vz);
         const uint32_t vi = imad(ly, 64u, imad(lz, 8u, lx));
-        const uint32_t code = __ldg(w.codes + (size_t)e * 512 + vi);
+        const uint32_t code = __ldg(w.codes - (size_t)kViBias + (size_t)e * 512 + vi);
         if (code == kCodeSolid) {
-            s.material = __ldg(w.payload + (size_t)e * 512 + vi);
-            s.vx = vx;
-            s.vy = vy;
-            s.vz = vz;
+            s.set_hit(vx - kBias, vy - kBias, vz - kBias, e);
             return kStepHit;
         }
         if (kGlsl && kCoarse && (coarse & kCoarseNow) && code != 3u) {
             // the cell's mask is not empty (lod < 4): its first solid voxel, bit
             // x + z*4 + y*16 of the cell mask, is the hit (mask-order scan of the payload)
-            const uint8_t* cell = w.payload + (size_t)e * 512 + ((lx & 4u) | (lz & 4u) << 3 | (ly & 4u) << 6);
+            const size_t cell = (size_t)e * 512 + ((vx & 4u) | (vz & 4u) << 3 | (vy & 4u) << 6);
             for (uint32_t j = 0; j < 64; j++) {
-                const uint32_t mat = __ldg(cell + ((j & 3u) | ((j >> 2) & 3u) << 3 | (j >> 4) << 6));
-                if (mat) {
-                    s.material = mat;
-                    s.vx = (vx & ~3) | (int32_t)(j & 3u);
-                    s.vy = (vy & ~3) | (int32_t)(j >> 4);
-                    s.vz = (vz & ~3) | (int32_t)((j >> 2) & 3u);
+                const size_t c = cell + ((j & 3u) | ((j >> 2) & 3u) << 3 | (j >> 4) << 6);
+                if (__ldg(w.payload + c)) {
+                    s.set_hit(((vx - kBias) & ~3u) | (j & 3u), ((vy - kBias) & ~3u) | (j >> 4),
+                              ((vz - kBias) & ~3u) | ((j >> 2) & 3u), e);
                     return kStepHit;
                 }
             }
         }
-        m = (int32_t)code;
+        m = code;
     } else {
-        m = kGlsl ? (int32_t)((e >> 8) & 127u) : (int32_t)(e & 31u);
+        m = kGlsl ? (e >> 8) & 127u : e & 31u;
     }
-    // dir < 0 ? pos & ~m : pos | m, as (pos | m) ^ (g & m) with g = -1 for dir < 0
-    vx = (vx | m) ^ (s.gx & m);
-    vy = (vy | m) ^ (s.gy & m);
-    vz = (vz | m) ^ (s.gz & m);
-    if (kGlsl) {  // the next GLSL iteration starts from this voxel
-        s.vx = vx;
-        s.vy = vy;
-        s.vz = vz;
-        return kStepContinue;
-    }
-    // (the CPU loop needs the voxel only in the record of a hit or of a ray that left the
-    // grid, whose paths above set it)
-    s.sx = __fadd_rn(s.tsx, __fmul_rn(rel_voxel(vx, wox), s.ix));
-    s.sy = __fadd_rn(s.tsy, __fmul_rn(rel_voxel(vy, woy), s.iy));
-    s.sz = __fadd_rn(s.tsz, __fmul_rn(rel_voxel(vz, woz), s.iz));
-    const float t = kSafe ? __fadd_rn(fminf(fminf(s.sx, s.sy), s.sz), 0.001f)
-                          : __fadd_rn(min_x86(min_x86(s.sx, s.sy), s.sz), 0.001f);
-    s.cx = __fadd_rn(s.ox, __fmul_rn(t, s.dx));
-    s.cy = __fadd_rn(s.oy, __fmul_rn(t, s.dy));
-    s.cz = __fadd_rn(s.oz, __fmul_rn(t, s.dz));
+    step_on<kSafe, kGlsl, kCoarse>(s, vx, vy, vz, m, wox, woy, woz, coarse);
     return kStepContinue;
 }
 
 // Steps k = k .. kmax-1 of a ray whose first step here is its iteration i0 + k, until
-// one ends it (the returned status) or kmax is reached (kStepContinue).  safe: the
-// fast step (ray_init's bounds hold); coarse_ray: a rayCastCoarse ray (kCoarse only).
+// one ends it (the returned status) or kmax is reached (kStepContinue): fast steps while the
+// distance lies in the ray's range, then general ones (a ray that misses takes one or two at
+// the grid's edge).  The loops follow each other; a choice between them cost the fast one ten
+// register moves a step (59 instead of 48 instructions).  coarse_ray: a rayCastCoarse ray
+// (kCoarse only).
 template <bool kCount, bool kGlsl, bool kCoarse, bool kAniso>
 __device__ __forceinline__ uint32_t dda_steps(RayState& s, const DevWorld& w, int32_t wox, int32_t woy, int32_t woz,
-                                              TraceCounters& cnt, bool safe, bool coarse_ray, uint32_t i0,
-                                              uint32_t& k, uint32_t kmax) {
+                                              TraceCounters& cnt, bool coarse_ray, uint32_t i0, uint32_t& k,
+                                              uint32_t kmax) {
     uint32_t st = kStepContinue;
-    if (safe) {
-        for (; k < kmax; k++) {
-            st = ray_step<kCount, true, kGlsl, kCoarse, kAniso>(s, w, wox, woy, woz, cnt,
-                                                                kCoarse ? coarse_bits(coarse_ray, i0 + k) : 0u);
-            if (st != kStepContinue) break;
-        }
-    } else {
-        for (; k < kmax; k++) {
-            st = ray_step<kCount, false, kGlsl, kCoarse, kAniso>(s, w, wox, woy, woz, cnt,
-                                                                 kCoarse ? coarse_bits(coarse_ray, i0 + k) : 0u);
-            if (st != kStepContinue) break;
-        }
+    const uint32_t* biased = biased_table(w);
+    while (k < kmax && s.tb >= s.t_lo && s.tb < s.t_hi) {
+        st = ray_step<kCount, true, kGlsl, kCoarse, kAniso>(s, w, biased, wox, woy, woz, cnt,
+                                                            kCoarse ? coarse_bits(coarse_ray, i0 + k) : 0u);
+        if (st != kStepContinue) return st;
+        k++;
+    }
+    for (; k < kmax; k++) {
+        st = ray_step<kCount, false, kGlsl, kCoarse, kAniso>(s, w, nullptr, wox, woy, woz, cnt,
+                                                             kCoarse ? coarse_bits(coarse_ray, i0 + k) : 0u);
+        if (st != kStepContinue) break;
     }
     return st;
 }
@@ -426,18 +542,23 @@ __device__ __forceinline__ uint32_t dda_steps(RayState& s, const DevWorld& w, in
 // group may be a rayCastCoarse ray; coarse_ray says whether this one is) and aniso.
 template <bool kCount, bool kGlsl>
 __device__ __forceinline__ uint32_t dda_steps_mode(RayState& s, const DevWorld& w, int32_t wox, int32_t woy,
-                                                   int32_t woz, TraceCounters& cnt, bool safe, bool coarse,
+                                                   int32_t woz, TraceCounters& cnt, bool coarse,
                                                    bool coarse_ray, bool aniso, uint32_t i0, uint32_t& k,
                                                    uint32_t kmax) {
     if constexpr (!kGlsl) {
-        return dda_steps<kCount, false, false, false>(s, w, wox, woy, woz, cnt, safe, false, i0, k, kmax);
+        return dda_steps<kCount, false, false, false>(s, w, wox, woy, woz, cnt, false, i0, k, kmax);
     } else {
         if (aniso)
-            return coarse ? dda_steps<kCount, true, true, true>(s, w, wox, woy, woz, cnt, safe, coarse_ray, i0, k, kmax)
-                          : dda_steps<kCount, true, false, true>(s, w, wox, woy, woz, cnt, safe, false, i0, k, kmax);
-        return coarse ? dda_steps<kCount, true, true, false>(s, w, wox, woy, woz, cnt, safe, coarse_ray, i0, k, kmax)
-                      : dda_steps<kCount, true, false, false>(s, w, wox, woy, woz, cnt, safe, false, i0, k, kmax);
+            return coarse ? dda_steps<kCount, true, true, true>(s, w, wox, woy, woz, cnt, coarse_ray, i0, k, kmax)
+                          : dda_steps<kCount, true, false, true>(s, w, wox, woy, woz, cnt, false, i0, k, kmax);
+        return coarse ? dda_steps<kCount, true, true, false>(s, w, wox, woy, woz, cnt, coarse_ray, i0, k, kmax)
+                      : dda_steps<kCount, true, false, false>(s, w, wox, woy, woz, cnt, false, i0, k, kmax);
     }
+}
+
+// Voxel id of a hit (0 on a miss), read once its ray has ended.
+__device__ __forceinline__ uint32_t hit_material(const RayState& s, const uint8_t* payload, bool hit) {
+    return hit ? __ldg(payload + s.hit_byte()) : 0u;
 }
 
 // Whole RayCast (or rayCast / rayCastCoarse, kGlsl) for one ray.
@@ -447,9 +568,10 @@ __device__ __forceinline__ void trace_ray(const DevWorld& w, float ox, float oy,
                                           TraceResult& r, TraceCounters& cnt, bool coarse_ray = false,
                                           bool aniso = false) {
     RayState s;
-    const bool safe = ray_start<kGlsl>(s, w, ox, oy, oz, dx, dy, dz, wox, woy, woz, false, coarse_ray);
+    const int32_t wo[3] = {wox, woy, woz};
+    ray_start<kGlsl>(s, clip_box(w, wo), ox, oy, oz, dx, dy, dz, wox, woy, woz, coarse_ray);
     uint32_t i = 0;
-    uint32_t st = dda_steps_mode<kCount, kGlsl>(s, w, wox, woy, woz, cnt, safe, coarse_ray, coarse_ray, aniso, 0, i,
+    uint32_t st = dda_steps_mode<kCount, kGlsl>(s, w, wox, woy, woz, cnt, coarse_ray, coarse_ray, aniso, 0, i,
                                                 max_iters);
     if (max_iters == 0) st = kStepOut;
     r.cx = s.cx;
@@ -459,12 +581,10 @@ __device__ __forceinline__ void trace_ray(const DevWorld& w, float ox, float oy,
     r.sy = s.sy;
     r.sz = s.sz;
     r.tb = s.tb;
-    r.vx = s.vx;
-    r.vy = s.vy;
-    r.vz = s.vz;
+    r.voxel = s.hit_voxel();
     r.steps = i;  // == max_iters when the cap ran out
-    r.material = s.material;
     r.hit = st == kStepHit && i < max_iters;
+    r.material = hit_material(s, w.payload, r.hit);
 }
 
 // The 16-byte vrt_hit record as one vector store.  kGlsl: t is the biased tmin and
@@ -491,8 +611,7 @@ __device__ __forceinline__ uint4 pack_hit(const TraceResult& r, float dx, float 
         else
             face = dz < 0.0f ? 5u : 4u;
     }
-    const uint32_t voxel = (uint32_t)r.vx | (uint32_t)r.vy << 11 | (uint32_t)r.vz << 21;
-    return make_uint4(voxel, face | r.material << 8 | r.steps << 16, __float_as_uint(t), tag);
+    return make_uint4(r.voxel, face | r.material << 8 | r.steps << 16, __float_as_uint(t), tag);
 }
 
 __device__ __forceinline__ uint4 no_ray_hit() {
@@ -578,17 +697,16 @@ __device__ __forceinline__ void bounce_dir(uint32_t pixel, uint32_t bounce, floa
 
 // Hit record from a finished RayState (steps = iteration index at exit).
 template <bool kGlsl = false>
-__device__ __forceinline__ uint4 pack_state(const RayState& s, bool hit, uint32_t steps, uint32_t tag) {
+__device__ __forceinline__ uint4 pack_state(const RayState& s, uint32_t material, bool hit, uint32_t steps,
+                                           uint32_t tag) {
     TraceResult r;
     r.sx = s.sx;
     r.sy = s.sy;
     r.sz = s.sz;
     r.tb = s.tb;
-    r.vx = s.vx;
-    r.vy = s.vy;
-    r.vz = s.vz;
+    r.voxel = s.hit_voxel();
     r.steps = steps;
-    r.material = s.material;
+    r.material = material;
     r.hit = hit;
     return pack_hit<kGlsl>(r, s.dx, s.dy, s.dz, tag);
 }

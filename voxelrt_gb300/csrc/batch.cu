@@ -32,11 +32,17 @@ __device__ __forceinline__ uint32_t compact_even_bits(uint32_t k) {
 }
 
 // What the rays of one view share, from its camera origin: whether that is inside and near
-// (origin_inside_near) with the distances to the clip box's sides.
+// (origin_inside_near) with the distances to the clip box's sides, and (tile_kernel, CPU
+// traversal) what iteration 0 finds there: the origin's voxel in biased form and the alignment
+// mask of its cell, or that it is solid.
+constexpr uint32_t kStartUnknown = 0xFFFFFFFFu, kStartSolid = 0xFFFFFFFEu;
 struct ViewStart {
     ClipBox clip;
     BoxSides box;
     uint32_t inside;
+    uint32_t mask;      // kStartUnknown, kStartSolid or the alignment mask
+    uint32_t voxel[3];
+    uint32_t material;  // of a solid origin
 };
 
 VRT_HD inline ViewStart view_start(const DevWorld& w, const ViewDev& v) {
@@ -44,6 +50,7 @@ VRT_HD inline ViewStart view_start(const DevWorld& w, const ViewDev& v) {
     s.clip = clip_box(w, v.wo);
     s.box = box_sides(s.clip, v.ox, v.oy, v.oz);
     s.inside = origin_inside_near(s.clip, v.ox, v.oy, v.oz) ? 1u : 0u;
+    s.mask = kStartUnknown;
     return s;
 }
 
@@ -57,12 +64,22 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
     uint4* o = out + v.out_base + pixel;
     float dx, dy, dz;
     camera_ray(v.d0, v.du, v.dv, px, py, dx, dy, dz);
+    if (!kGlsl && !kBounces && vs.mask == kStartSolid && last == 0) {
+        // the camera stands in a solid voxel: every ray hits it on iteration 0 at t = 0, face X
+        const uint32_t x = vs.voxel[0] - kVoxelBias, y = vs.voxel[1] - kVoxelBias, z = vs.voxel[2] - kVoxelBias;
+        *o = make_uint4(x | y << 11 | z << 21, (dx < 0.0f ? 1u : 0u) | vs.material << 8, 0u, pixel);
+        return 1;
+    }
     const int32_t wox = v.wo[0], woy = v.wo[1], woz = v.wo[2];
     const bool full = kBounces && (v.path & kPathFull) != 0;
     RayState s;
     uint32_t i = 0;
     if (vs.inside) {
         ray_start_inside<kGlsl>(s, vs.box, v.ox, v.oy, v.oz, dx, dy, dz, wox, woy, woz);
+        if (!kGlsl && !kBounces && vs.mask < kStartSolid && s.t_hi > 0.0f) {
+            step_on<true, false, false>(s, vs.voxel[0], vs.voxel[1], vs.voxel[2], vs.mask, wox, woy, woz, 0);
+            i = 1;
+        }
     } else {
         ray_start<kGlsl>(s, vs.clip, v.ox, v.oy, v.oz, dx, dy, dz, wox, woy, woz);
     }
@@ -608,6 +625,116 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
     }
 }
 
+// Launches whose views have no bounces (primary rays, or primary and one sun ray): each warp
+// claims a chunk of tiles and traces it 32 rays at a time, a pixel's rays per lane
+// (trace_pixel) before it takes the next 32.  Bound by instruction issue.  Neighbouring camera
+// rays are of a length (92-96 % of lanes busy in an 8x4 group on terrain), so nothing is
+// gained by refilling lanes one by one, and without it the view, its world and what its rays
+// share (ViewStart) belong to the warp: in shared memory, read at a ray's start, the step
+// loop's part in registers.  Warp instructions for 32 primary rays, against the persistent
+// kernel: 240 and 48 a step, against 335 and 52, and 170 in all for a camera in a solid voxel.
+// 44 M rays over 154 views of 16 mixed worlds: 701 us against 1109 us;
+// six 1080p terrain views with sun rays: 754 us against 1035 us.  72 registers, 28 warps a
+// SM: 64 spill (713 and 767 us), 56 more so (759 and 803 us), 80 leave 24 warps (735 and 788 us).
+template <bool kGlsl, bool kAniso>
+__global__ void __maxnreg__(72) tile_kernel(BatchParams p) {
+    if constexpr (kAniso) fill_forward_lut();
+    // what the warp's view needs at a ray's start (warps_per_block <= 16)
+    struct Warp {
+        ViewDev v;
+        DevWorld w;
+        ViewStart start;
+    };
+    __shared__ Warp s_warps[16];
+    Warp& sw = s_warps[threadIdx.x >> 5];
+    const ViewDev& v = sw.v;
+    DevWorld w{};  // a copy in registers: the step loop reads its table addresses and strides
+    const uint32_t lane = threadIdx.x & 31;
+    // the lane's pixel in a tile's first 32; the next 32 lie `rows` rows below
+    uint32_t kx, ky;
+    if (p.morton) {
+        kx = compact_even_bits(lane);
+        ky = compact_even_bits(lane >> 1);
+    } else {
+        kx = lane & ((1u << p.tile_w_log2) - 1u);
+        ky = lane >> p.tile_w_log2;
+    }
+    const uint32_t rows = 32u >> p.tile_w_log2, tile_h = 1u << (p.tile_size_log2 - p.tile_w_log2);
+    const uint32_t chunk_tiles = p.chunk_rays >> p.tile_size_log2;
+    uint32_t view = 0, loaded = kNoView, rays = 0;
+    for (;;) {
+        uint32_t c = lane == 0 ? atomicAdd(p.queue, 1u) : 0u;
+        c = __shfl_sync(0xffffffffu, c, 0);
+        if (c >= p.total_chunks) break;
+        c += p.chunk_first;
+        // a warp's claims only grow, so the chunk lies in the last view or a later one
+        uint32_t hi = p.n_views;
+        if (view + 1 < hi && __ldg(p.chunk_base + view + 1) <= c)
+            view++;
+        else
+            hi = view + 1;
+        while (hi - view > 1) {
+            const uint32_t mid = (view + hi) >> 1;
+            if (__ldg(p.chunk_base + mid) <= c)
+                view = mid;
+            else
+                hi = mid;
+        }
+        if (view != loaded) {
+            loaded = view;
+            __syncwarp();
+            reinterpret_cast<uint32_t*>(&sw.v)[lane] = __ldg(reinterpret_cast<const uint32_t*>(p.views + view) + lane);
+            const uint32_t wi = __ldg(&p.views[view].world);
+            if (lane < sizeof(DevWorld) / 4)
+                reinterpret_cast<uint32_t*>(&sw.w)[lane] = __ldg(reinterpret_cast<const uint32_t*>(p.worlds + wi) + lane);
+            __syncwarp();
+            w = sw.w;
+            ViewStart vs = view_start(w, v);
+            if (!kGlsl && vs.inside) {
+                // iteration 0 of every ray of the view: the table entry and code at the origin
+                const uint32_t x = (uint32_t)(v.wo[0] + __float2int_rd(v.ox)), y = (uint32_t)(v.wo[1] + __float2int_rd(v.oy)),
+                               z = (uint32_t)(v.wo[2] + __float2int_rd(v.oz));
+                const uint32_t e = __ldg(w.bricks + (x >> 3) + (z >> 3) * w.bsx + (y >> 3) * w.bsxz);
+                if (e < kBrickEmpty) {
+                    const size_t at = (size_t)e * 512 + ((x & 7u) | (z & 7u) << 3 | (y & 7u) << 6);
+                    const uint32_t code = __ldg(w.codes + at);
+                    vs.mask = code == kCodeSolid ? kStartSolid : code;
+                    vs.material = __ldg(w.payload + at);
+                } else {
+                    vs.mask = e & 31u;
+                }
+                vs.voxel[0] = x + kVoxelBias;
+                vs.voxel[1] = y + kVoxelBias;
+                vs.voxel[2] = z + kVoxelBias;
+            }
+            if (lane == 0) sw.start = vs;
+            __syncwarp();
+        }
+        uint32_t t = (c - v.chunk_base) * chunk_tiles;
+        const uint32_t t_end = min(t + chunk_tiles, v.n_rays >> p.tile_size_log2);
+        uint32_t ty = v.tiles_x_magic ? __umulhi(t, v.tiles_x_magic) : t;
+        if (ty * v.tiles_x > t) ty--;
+        uint32_t tx = t - ty * v.tiles_x;
+        uint32_t y = ty * tile_h;
+        for (;;) {
+            const uint32_t px = (tx << p.tile_w_log2) + kx, py = y + ky;
+            if (px < v.width && py < v.height) rays += trace_pixel<kGlsl, kAniso, false>(v, w, sw.start, px, py, p.out);
+            __syncwarp();
+            y += rows;
+            if ((y & (tile_h - 1u)) == 0) {  // the tile is done
+                if (++t == t_end) break;
+                y -= tile_h;
+                if (++tx == v.tiles_x) {
+                    tx = 0;
+                    y += tile_h;
+                }
+            }
+        }
+    }
+    for (int off = 16; off > 0; off >>= 1) rays += __shfl_xor_sync(0xffffffffu, rays, off);
+    if (lane == 0) atomicAdd(p.counters, (unsigned long long)rays);
+}
+
 uint32_t log2u(uint32_t v) {
     uint32_t r = 0;
     while ((1u << r) < v) r++;
@@ -724,6 +851,17 @@ uint32_t auto_chunk_tiles(uint64_t tiles, uint64_t warps) {
     return (uint32_t)std::min<uint64_t>(16, std::max<uint64_t>(1, tiles / (warps * 8)));
 }
 
+// Tiles per claim of tile_kernel where the config leaves it open, at most: the launch ends with
+// the last claims, and 16 tiles (1,024 rays) of long rays run on for a third of a millisecond
+// after the queue is empty (44 M rays over 154 views: 1466 us with 16 tiles, 1041 with 4, 968
+// with 2, 950 with 1 in the kernel's first build; terrain views as well).  2 halve the claims.
+constexpr uint32_t kTileChunk = 2;
+bool tile_launch(const vrt_view* views, uint32_t n) {
+    for (uint32_t i = 0; i < n; i++)
+        if (views[i].n_bounces) return false;
+    return true;
+}
+
 void resolve_batch_defaults(vrt_batch_config& cfg, const vrt_view* views, uint32_t n, uint64_t warps) {
     bool bounces = false;
     uint64_t tiles = 0;
@@ -734,6 +872,12 @@ void resolve_batch_defaults(vrt_batch_config& cfg, const vrt_view* views, uint32
     }
     if (cfg.refill_threshold == 0) cfg.refill_threshold = bounces ? 28 : 16;
     if (cfg.chunk_tiles == 0) cfg.chunk_tiles = bounces ? 1 : auto_chunk_tiles(tiles, warps);
+}
+
+void resolve_launch_config(vrt_batch_config& cfg, const vrt_view* views, uint32_t n, uint64_t warps) {
+    const bool open = cfg.chunk_tiles == 0;
+    resolve_batch_defaults(cfg, views, n, warps);
+    if (open && tile_launch(views, n)) cfg.chunk_tiles = std::min(cfg.chunk_tiles, kTileChunk);
 }
 
 vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, const vrt_batch_config& cfg_in,
@@ -748,11 +892,12 @@ vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, cons
     }
     if ((st = check_same_mode(views, n)) != VRT_OK) return st;
     vrt_batch_config cfg = cfg_in;
-    resolve_batch_defaults(cfg, views, n, warps);
+    resolve_launch_config(cfg, views, n, warps);
     plan.glsl = n > 0 && view_glsl(views[0]);
     plan.aniso = n > 0 && view_aniso(views[0]);
     plan.full = false;
     for (uint32_t i = 0; i < n; i++) plan.full |= view_full_path(views[i]);
+    plan.tiles = tile_launch(views, n);
     plan.cfg = cfg;
     plan.tile_w_log2 = log2u(cfg.tile_w);
     plan.tile_size_log2 = log2u(cfg.tile_w * cfg.tile_h);
@@ -786,7 +931,8 @@ vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, cons
 
 namespace {
 
-// The instantiation a launch runs: counting, traversal mode, resident, whole-path views.
+// The kernel a launch runs: tiles (no view has bounces), or the persistent kernel's
+// instantiation: counting, traversal mode, resident, whole-path views.
 using PersistentFn = void (*)(BatchParams);
 template <bool kCount, bool kResident, bool kFull>
 PersistentFn persistent_fn_mode(bool glsl, bool aniso) {
@@ -794,7 +940,9 @@ PersistentFn persistent_fn_mode(bool glsl, bool aniso) {
     if (glsl) return persistent_kernel<kCount, true, kResident, false, kFull>;
     return persistent_kernel<kCount, false, kResident, false, kFull>;
 }
-PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, bool full) {
+PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, bool full, bool tiles) {
+    if (tiles && !count && !resident)
+        return glsl ? (aniso ? tile_kernel<true, true> : tile_kernel<true, false>) : tile_kernel<false, false>;
     if (resident) return full ? persistent_fn_mode<false, true, true>(glsl, aniso)
                               : persistent_fn_mode<false, true, false>(glsl, aniso);
     if (count) return full ? persistent_fn_mode<true, false, true>(glsl, aniso)
@@ -804,20 +952,21 @@ PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, boo
 
 // Resident blocks per SM of that kernel: the variants differ in registers and shared memory
 // (the anisotropic LUT is 8 KB per block).
-cudaError_t persistent_occupancy(int& occ, int threads, bool count, bool glsl, bool aniso, bool resident, bool full) {
+cudaError_t persistent_occupancy(int& occ, int threads, bool count, bool glsl, bool aniso, bool resident, bool full,
+                                 bool tiles) {
     const size_t smem = full ? (size_t)threads * 6 * sizeof(float) : 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, persistent_fn(count, glsl, aniso, resident, full),
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, persistent_fn(count, glsl, aniso, resident, full, tiles),
                                                          threads, smem);
 }
 
 }  // namespace
 
 vrt_status persistent_grid(int device, const vrt_batch_config& cfg, bool count, bool glsl, bool aniso, bool resident,
-                           bool full, int& blocks, int& threads) {
+                           bool full, bool tiles, int& blocks, int& threads) {
     int sms = 0, occ = 0;
     threads = (int)cfg.warps_per_block * 32;
     VRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    VRT_CUDA(persistent_occupancy(occ, threads, count, glsl, aniso, resident, full));
+    VRT_CUDA(persistent_occupancy(occ, threads, count, glsl, aniso, resident, full, tiles));
     occ = std::max(occ, 1);
     const int per_sm = (!count && cfg.blocks_per_sm) ? std::min<int>((int)cfg.blocks_per_sm, occ) : occ;
     blocks = sms * per_sm;
@@ -847,11 +996,12 @@ BatchParams make_params(const LaunchPlan& plan, const DevWorld* worlds, const Vi
     p.glsl = plan.glsl ? 1u : 0u;
     p.aniso = plan.aniso ? 1u : 0u;
     p.full = plan.full ? 1u : 0u;
+    p.tiles = plan.tiles ? 1u : 0u;
     return p;
 }
 
 vrt_status launch_resident(const BatchParams& p, int blocks, int threads, cudaStream_t stream) {
-    const PersistentFn fn = persistent_fn(false, p.glsl != 0, p.aniso != 0, true, p.full != 0);
+    const PersistentFn fn = persistent_fn(false, p.glsl != 0, p.aniso != 0, true, p.full != 0, false);
     fn<<<blocks, threads, pend_bytes(p, threads), stream>>>(p);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
@@ -860,7 +1010,7 @@ vrt_status launch_resident(const BatchParams& p, int blocks, int threads, cudaSt
 vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool count, cudaStream_t stream,
                              bool reset_counters) {
     VRT_CUDA(cudaMemsetAsync(p.queue, 0, reset_counters ? 64 : 4, stream));
-    const PersistentFn fn = persistent_fn(count, p.glsl != 0, p.aniso != 0, false, p.full != 0);
+    const PersistentFn fn = persistent_fn(count, p.glsl != 0, p.aniso != 0, false, p.full != 0, p.tiles != 0);
     fn<<<blocks, threads, pend_bytes(p, threads), stream>>>(p);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
@@ -999,7 +1149,7 @@ vrt_status vrt_batch_create(vrt_world* const* worlds, uint32_t n_worlds, const v
         bool full = false;
         for (uint32_t i = 0; i < n_views; i++) full |= view_full_path(views[i]);
         if ((st = persistent_grid(worlds[0]->device, cfg, false, view_glsl(views[0]), view_aniso(views[0]), false,
-                                  full, grid_blocks, grid_threads)) != VRT_OK)
+                                  full, tile_launch(views, n_views), grid_blocks, grid_threads)) != VRT_OK)
             return st;
     }
     auto* b = new vrt_batch;
@@ -1036,9 +1186,9 @@ vrt_status vrt_batch_create(vrt_world* const* worlds, uint32_t n_worlds, const v
     b->d_counters = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(b->d_queue) + 16);
     if ((st = refresh_worlds(b, 0)) != VRT_OK) return fail(st);
     const bool glsl = b->plan.glsl, aniso = b->plan.aniso, full = b->plan.full;
-    if ((st = persistent_grid(b->device, cfg, false, glsl, aniso, false, full, b->blocks, b->threads)) != VRT_OK)
+    if ((st = persistent_grid(b->device, cfg, false, glsl, aniso, false, full, b->plan.tiles, b->blocks, b->threads)) != VRT_OK)
         return fail(st);
-    if ((st = persistent_grid(b->device, cfg, true, glsl, aniso, false, full, b->blocks_count, b->threads_count)) !=
+    if ((st = persistent_grid(b->device, cfg, true, glsl, aniso, false, full, false, b->blocks_count, b->threads_count)) !=
         VRT_OK)
         return fail(st);
     *out = b;

@@ -62,6 +62,7 @@ struct BatchParams {
     uint32_t inner;
     uint32_t glsl;  // traversal mode of every view (VRT_VIEW_GLSL)
     uint32_t aniso;  // ... with anisotropic LODs (VRT_VIEW_GLSL_ANISO)
+    uint32_t tiles;  // no view has bounces: tile_kernel traces the launch
     uint32_t full;   // some view traces the GPU renderer's whole path (sun rays among bounces)
     // resident launches (request server): views are published while the kernel runs
     unsigned long long* mailbox;  // host-mapped: published chunks | published views << 32 | closed << 63
@@ -91,6 +92,7 @@ struct LaunchPlan {
     uint32_t chunks = 0;
     bool glsl = false;   // every view traces in the GLSL mode
     bool aniso = false;  // ... with anisotropic LODs
+    bool tiles = false;  // no view has bounces (tile_launch)
     bool full = false;   // some view traces the GPU renderer's whole path
 };
 
@@ -116,19 +118,23 @@ vrt_status normalize_batch_config(const vrt_batch_config* in, vrt_batch_config& 
 // eight chunks per warp of the launch, 1..16 tiles.  Fixed chunks too large for a small
 // launch leave most warps without work; the tuned table names its chunks explicitly.
 uint32_t auto_chunk_tiles(uint64_t tiles, uint64_t warps);
+// Whether a launch of these views runs tile_kernel: no view has bounces.
+bool tile_launch(const vrt_view* views, uint32_t n);
 // Fill the fields a config leaves to the library (0): views with diffuse bounces (long,
 // uneven, incoherent paths per pixel) refill below 28 lanes and claim one tile at a time;
 // camera and sun rays refill below 16 and claim auto_chunk_tiles.
 void resolve_batch_defaults(vrt_batch_config& cfg, const vrt_view* views, uint32_t n, uint64_t warps);
+// The same for a launch of these views: with tile_kernel a chunk left open is at most 2 tiles.
+void resolve_launch_config(vrt_batch_config& cfg, const vrt_view* views, uint32_t n, uint64_t warps);
 // Validate views against n_worlds and lay them out (tiles, queue chunks, record offsets).
 // Fields left to the library are resolved for a launch of `warps` warps
-// (resolve_batch_defaults), and plan.cfg holds the config used.
+// (resolve_launch_config), and plan.cfg holds the config used.
 vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, const vrt_batch_config& cfg,
                       LaunchPlan& plan, uint64_t warps = 0);
 // Grid of the persistent kernel: every SM, as many blocks of the launched instantiation
 // (counting, traversal mode, resident) as fit, or cfg.blocks_per_sm of them.
 vrt_status persistent_grid(int device, const vrt_batch_config& cfg, bool count, bool glsl, bool aniso, bool resident,
-                           bool full, int& blocks, int& threads);
+                           bool full, bool tiles, int& blocks, int& threads);
 BatchParams make_params(const LaunchPlan& plan, const DevWorld* worlds, const ViewDev* views,
                         const uint32_t* chunk_base, uint32_t* queue, vrt_hit* out);
 // Queue reset (the tile counter, and with reset_counters the launch counters: 64

@@ -117,9 +117,11 @@ extern "C" vrt_status vrt_render_views_static(vrt_world* const* worlds, uint32_t
     const bool aniso = view_aniso(views[0]);
     bool full = false;
     for (uint32_t i = 0; i < n_views; i++) full |= view_full_path(views[i]);
+    const bool tiles = tile_launch(views, n_views);
     int blocks = 0, threads = 0;
-    if ((st = persistent_grid(device, cfg, false, glsl, aniso, false, full, blocks, threads)) != VRT_OK) return st;
-    resolve_batch_defaults(cfg, views, n_views, (uint64_t)blocks * (threads / 32));
+    if ((st = persistent_grid(device, cfg, false, glsl, aniso, false, full, tiles, blocks, threads)) != VRT_OK)
+        return st;
+    resolve_launch_config(cfg, views, n_views, (uint64_t)blocks * (threads / 32));
     // lay the views out behind one tile queue (same layout as vrt_batch)
     const uint32_t tw_log2 = log2u_static(cfg.tile_w), ts_log2 = log2u_static(cfg.tile_w * cfg.tile_h);
     uint64_t chunks = 0, records = 0;
@@ -129,14 +131,14 @@ extern "C" vrt_status vrt_render_views_static(vrt_world* const* worlds, uint32_t
         d = make_view_dev(v);
         const uint32_t tx = (v.cam.width + cfg.tile_w - 1) / cfg.tile_w;
         const uint32_t ty = (v.cam.height + cfg.tile_h - 1) / cfg.tile_h;
-        const uint64_t tiles = (uint64_t)tx * ty;
+        const uint64_t n_tiles = (uint64_t)tx * ty;
         d.tiles_x = tx;
         d.tiles_x_magic = div_magic(tx);
-        d.n_rays = (uint32_t)(tiles << ts_log2);
+        d.n_rays = (uint32_t)(n_tiles << ts_log2);
         d.chunk_base = (uint32_t)chunks;
         d.out_base = records;
         g_state.chunk_base[i] = (uint32_t)chunks;
-        chunks += (tiles + cfg.chunk_tiles - 1) / cfg.chunk_tiles;
+        chunks += (n_tiles + cfg.chunk_tiles - 1) / cfg.chunk_tiles;
         records += view_record_count(v);
         if (chunks >= 0xffffffffull) {
             set_error("too many ray tiles for one call");
@@ -172,6 +174,7 @@ extern "C" vrt_status vrt_render_views_static(vrt_world* const* worlds, uint32_t
     p.glsl = glsl ? 1u : 0u;
     p.aniso = aniso ? 1u : 0u;
     p.full = full ? 1u : 0u;
+    p.tiles = tiles ? 1u : 0u;
     // launch_persistent zeroes the queue counter and the launch counters first
     return launch_persistent(p, blocks, threads, false, stream);
 }

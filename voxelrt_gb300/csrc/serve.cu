@@ -123,10 +123,11 @@ struct vrt_server {
     vrt_server_config cfg{};
     vrt_batch_config bcfg{};
     // persistent grid per traversal mode (view_mode: 0, GLSL, GLSL + anisotropic) of the
-    // instantiation the server launches in its scheduling mode: blocks, threads
-    int grid[3][2] = {};
-    const int* grid_of(uint32_t mode) const {
-        return grid[(mode & VRT_VIEW_GLSL_ANISO) ? 2 : (mode & VRT_VIEW_GLSL) ? 1 : 0];
+    // instantiation the server launches in its scheduling mode: blocks, threads; the second
+    // for launches of views without bounces (tile_launch)
+    int grid[2][3][2] = {};
+    const int* grid_of(uint32_t mode, bool tiles = false) const {
+        return grid[tiles ? 1 : 0][(mode & VRT_VIEW_GLSL_ANISO) ? 2 : (mode & VRT_VIEW_GLSL) ? 1 : 0];
     }
     DevWorld* d_worlds = nullptr;
     uint8_t* arena = nullptr;  // output records of admitted requests
@@ -206,7 +207,7 @@ vrt_status launch_slot(vrt_server* sv, Slot& s, std::vector<Request*>& rs) {
     std::vector<vrt_view> views(rs.size());
     for (size_t i = 0; i < rs.size(); i++) views[i] = rs[i]->view;
     LaunchPlan plan;
-    const int* g = sv->grid_of(view_mode(views[0]));
+    const int* g = sv->grid_of(view_mode(views[0]), tile_launch(views.data(), (uint32_t)views.size()));
     vrt_status st = plan_views(views.data(), (uint32_t)views.size(), (uint32_t)sv->worlds.size(), sv->bcfg, plan,
                                (uint64_t)g[0] * (g[1] / 32));
     if (st != VRT_OK) return st;
@@ -812,10 +813,12 @@ vrt_status vrt_server_create(vrt_world* const* worlds, uint32_t n_worlds, const 
         resident = native != 0;
     }
     sv->resident = resident;
-    for (int m = 0; m < 3; m++)
-        if ((st = persistent_grid(sv->device, sv->bcfg, false, m >= 1, m == 2, resident, false, sv->grid[m][0],
-                                  sv->grid[m][1])) != VRT_OK)
+    for (int m = 0; m < 6; m++) {
+        int* g = sv->grid[m / 3][m % 3];
+        if ((st = persistent_grid(sv->device, sv->bcfg, false, m % 3 >= 1, m % 3 == 2, resident, false, m >= 3, g[0],
+                                  g[1])) != VRT_OK)
             return fail(st);
+    }
     if (resident && (st = resident_init(sv)) != VRT_OK) return fail(st);
     sv->worker = resident ? std::thread(worker_resident, sv) : std::thread(worker_main, sv);
     *out = sv;

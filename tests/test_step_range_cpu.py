@@ -1,6 +1,6 @@
-"""The fast step's range (trace_core.cuh: ray_init's [t_lo, t_hi)) against the oracle, on the
-host build of the device step: rays whose origins, directions and world origins lie on
-either side of every bound that decides between the fast and the general step.  Records are
+"""The fast step's bounds (trace_core.cuh: RayState::fast) against the oracle, on the host
+build of the device step: rays whose origins, directions and world origins lie on either
+side of every bound that decides between the fast and the general step.  Records are
 bit formats, so they are equal word by word."""
 import numpy as np
 import pytest
@@ -33,7 +33,7 @@ def edge_rays(rng, size, wo, n):
 
 
 @pytest.mark.parametrize("mode", MODES, ids=lambda m: "+".join(m) or "cpu")
-@pytest.mark.parametrize("wo", [(0, 0, 0), (37, -5, 60), (65536, -65536, 65535), (65537, 0, 0), (0, -65537, 3),
+@pytest.mark.parametrize("wo", [(0, 0, 0), (37, -5, 60), (65536, -65536, 65535), (65537, 0, 0), (0, -65537, 3), (1 << 21, -(1 << 21), 7), ((1 << 21) + 1, 0, 0),
                                 (1 << 22, 0, -(1 << 24)), (1 << 30, -(1 << 30), 0)])
 def test_range_edges(exe, tmp_path, mode, wo):  # noqa: F811
     rng = np.random.default_rng(abs(sum(wo)) + len(mode))
@@ -52,7 +52,7 @@ def test_range_edges(exe, tmp_path, mode, wo):  # noqa: F811
 
 
 def test_iteration_caps(exe, tmp_path):  # noqa: F811
-    """Caps at, before and after the step that leaves the range."""
+    """Caps at, before and after the step that ends the ray."""
     rng = np.random.default_rng(5)
     vol = np.zeros((32, 32, 64), np.uint8)
     vol[::8, ::8, ::8] = 3

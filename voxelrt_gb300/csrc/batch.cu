@@ -32,13 +32,11 @@ __device__ __forceinline__ uint32_t compact_even_bits(uint32_t k) {
 }
 
 // What the rays of one view share, from its camera origin: whether that is inside and near
-// (origin_inside_near) with the distances to the clip box's sides, and (tile_kernel, CPU
-// traversal) what iteration 0 finds there: the origin's voxel in biased form and the alignment
+// (origin_inside_near), and (tile_kernel, CPU traversal) what iteration 0 finds there: the origin's voxel in biased form and the alignment
 // mask of its cell, or that it is solid.
 constexpr uint32_t kStartUnknown = 0xFFFFFFFFu, kStartSolid = 0xFFFFFFFEu;
 struct ViewStart {
     ClipBox clip;
-    BoxSides box;
     uint32_t inside;
     uint32_t mask;      // kStartUnknown, kStartSolid or the alignment mask
     uint32_t voxel[3];
@@ -48,7 +46,6 @@ struct ViewStart {
 VRT_HD inline ViewStart view_start(const DevWorld& w, const ViewDev& v) {
     ViewStart s{};
     s.clip = clip_box(w, v.wo);
-    s.box = box_sides(s.clip, v.ox, v.oy, v.oz);
     s.inside = origin_inside_near(s.clip, v.ox, v.oy, v.oz) ? 1u : 0u;
     s.mask = kStartUnknown;
     return s;
@@ -75,8 +72,8 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
     RayState s;
     uint32_t i = 0;
     if (vs.inside) {
-        ray_start_inside<kGlsl>(s, vs.box, v.ox, v.oy, v.oz, dx, dy, dz, wox, woy, woz);
-        if (!kGlsl && !kBounces && vs.mask < kStartSolid && s.t_hi > 0.0f) {
+        ray_start_inside<kGlsl>(s, v.ox, v.oy, v.oz, dx, dy, dz, wox, woy, woz);
+        if (!kGlsl && !kBounces && vs.mask < kStartSolid && s.fast) {
             step_on<true, false, false>(s, vs.voxel[0], vs.voxel[1], vs.voxel[2], vs.mask, wox, woy, woz, 0);
             i = 1;
         }
@@ -274,9 +271,11 @@ __device__ __forceinline__ void resident_pixels_done(const BatchParams& p, uint3
 }
 
 // kFull: the launch may hold views with the GPU renderer's whole path (a separate
-// instantiation, so the others keep their code and registers).
+// instantiation, so the others keep their code and registers).  64 registers (32 warps a SM)
+// are enough for the CPU traversal (two 720p views of 4 bounces: 443 us against 450 us with
+// 72), not for the GLSL modes (two worlds' whole paths: 735 us against 717 us).
 template <bool kCount, bool kGlsl, bool kResident = false, bool kAniso = false, bool kFull = false>
-__global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
+__global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
     if constexpr (kAniso) fill_forward_lut();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
@@ -531,7 +530,6 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
                         pixel = py * width + px;
                         iter = 0;
                         path = mp.y;
-                        const DevWorld w = load_world(p.worlds + wv.w);
                         // d0, du, dv with the camera origin in the fourth lanes
                         const float4 g0 = vget4<kResident>(reinterpret_cast<const float4*>(v->d0));
                         const float4 g1 = vget4<kResident>(reinterpret_cast<const float4*>(v->du));
@@ -540,12 +538,11 @@ __global__ void __maxnreg__(72) persistent_kernel(BatchParams p) {
                         float dx, dy, dz;
                         camera_ray(d0, du, dv, px, py, dx, dy, dz);
                         const int32_t wo3[3] = {wv.x, wv.y, wv.z};
-                        const ClipBox clip = clip_box(w, wo3);
                         if (kResident ? rw.q_inside != 0 : q_inside)
-                            ray_start_inside<kGlsl>(s, box_sides(clip, g0.w, g1.w, g2.w), g0.w, g1.w, g2.w, dx, dy, dz, wv.x,
-                                                    wv.y, wv.z);
+                            ray_start_inside<kGlsl>(s, g0.w, g1.w, g2.w, dx, dy, dz, wv.x, wv.y, wv.z);
                         else
-                            ray_start<kGlsl>(s, clip, g0.w, g1.w, g2.w, dx, dy, dz, wv.x, wv.y, wv.z);
+                            ray_start<kGlsl>(s, clip_box(load_world(p.worlds + wv.w), wo3), g0.w, g1.w, g2.w, dx, dy, dz,
+                                             wv.x, wv.y, wv.z);
                         active = true;
                     }
                 }

@@ -61,7 +61,7 @@ __device__ __forceinline__ void gbuffer_texel(const RayState& s, bool hit, uint3
 template <bool kGlsl, bool kAniso>
 __global__ void __launch_bounds__(64) gbuffer_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
                                                     const __grid_constant__ ClipBox clip, bool inside,
-                                                    const __grid_constant__ BoxSides box, const __grid_constant__ GbufferParams gp,
+                                                    const __grid_constant__ GbufferParams gp,
                                                     uint32_t* __restrict__ tex, float* __restrict__ depth,
                                                     uint4* __restrict__ out) {
     if constexpr (kAniso) fill_forward_lut();
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(64) gbuffer_kernel(const __grid_constant__ Dev
     camera_ray(v.d0, v.du, v.dv, px, py, dx, dy, dz);
     RayState s;
     if (inside)
-        ray_start_inside<kGlsl>(s, box, v.ox, v.oy, v.oz, dx, dy, dz, v.wo[0], v.wo[1], v.wo[2]);
+        ray_start_inside<kGlsl>(s, v.ox, v.oy, v.oz, dx, dy, dz, v.wo[0], v.wo[1], v.wo[2]);
     else
         ray_start<kGlsl>(s, clip, v.ox, v.oy, v.oz, dx, dy, dz, v.wo[0], v.wo[1], v.wo[2]);
     TraceCounters cnt{0, 0};
@@ -101,13 +101,12 @@ vrt_status launch_gbuffer(vrt_world* w, const vrt_view* view, const uint32_t* pa
     const DevWorld dw = w->dev();
     const ClipBox clip = clip_box(dw, v.wo);
     const bool inside = origin_inside_near(clip, v.ox, v.oy, v.oz);
-    const BoxSides box = box_sides(clip, v.ox, v.oy, v.oz);
     if (view_glsl(*view) && view_aniso(*view))
-        gbuffer_kernel<true, true><<<grid, block, 0, stream>>>(dw, v, clip, inside, box, gp, tex, depth, out);
+        gbuffer_kernel<true, true><<<grid, block, 0, stream>>>(dw, v, clip, inside, gp, tex, depth, out);
     else if (view_glsl(*view))
-        gbuffer_kernel<true, false><<<grid, block, 0, stream>>>(dw, v, clip, inside, box, gp, tex, depth, out);
+        gbuffer_kernel<true, false><<<grid, block, 0, stream>>>(dw, v, clip, inside, gp, tex, depth, out);
     else
-        gbuffer_kernel<false, false><<<grid, block, 0, stream>>>(dw, v, clip, inside, box, gp, tex, depth, out);
+        gbuffer_kernel<false, false><<<grid, block, 0, stream>>>(dw, v, clip, inside, gp, tex, depth, out);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }

@@ -21,11 +21,11 @@ uint32_t eff_iters(uint32_t max_iters, bool glsl = false) {
     return max_iters > 65535u ? 65535u : max_iters;
 }
 
-// inside: the camera origin is (origin_inside_near); box: its distances to the clip box's sides
+// inside: the camera origin is (origin_inside_near)
 __global__ void __launch_bounds__(64) render_view_kernel(const __grid_constant__ DevWorld w,
                                                         const __grid_constant__ vrt_camera cam,
                                                         const __grid_constant__ ClipBox clip, bool inside,
-                                                        const __grid_constant__ BoxSides box, uint32_t max_iters,
+                                                        uint32_t max_iters,
                                                         uint4* __restrict__ out) {
     const uint32_t px = blockIdx.x * 8 + threadIdx.x;
     const uint32_t py = blockIdx.y * 8 + threadIdx.y;
@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(64) render_view_kernel(const __grid_constant__
     const int32_t wox = cam.world_origin[0], woy = cam.world_origin[1], woz = cam.world_origin[2];
     RayState s;
     if (inside)
-        ray_start_inside<false>(s, box, cam.origin[0], cam.origin[1], cam.origin[2], dx, dy, dz, wox, woy, woz);
+        ray_start_inside<false>(s, cam.origin[0], cam.origin[1], cam.origin[2], dx, dy, dz, wox, woy, woz);
     else
         ray_start<false>(s, clip, cam.origin[0], cam.origin[1], cam.origin[2], dx, dy, dz, wox, woy, woz);
     TraceCounters cnt;
@@ -154,8 +154,7 @@ vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters
     const float* o = cam->origin;
     const ClipBox clip = clip_box(dw, cam->world_origin);
     render_view_kernel<<<grid, block, 0, stream>>>(dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]),
-                                                   box_sides(clip, o[0], o[1], o[2]), eff_iters(max_iters),
-                                                   reinterpret_cast<uint4*>(hits));
+                                                   eff_iters(max_iters), reinterpret_cast<uint4*>(hits));
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }

@@ -25,19 +25,6 @@ __device__ __forceinline__ int32_t floor2i(float x) {
 __device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)((uint32_t)a + (uint32_t)b); }
 __device__ __forceinline__ int32_t wsub(int32_t a, int32_t b) { return (int32_t)((uint32_t)a - (uint32_t)b); }
 
-// a * b + c (mod 2^32) on the integer multiply-add unit.  The step loop is bound by
-// the ALU pipe (bit ops, compares, shifts) while the FMA pipe, which also executes
-// integer multiply-add, has room; inline PTX keeps the compiler from folding these
-// back into masks and adds (x - 8*(x >> 3) would become x & 7).
-__device__ __forceinline__ uint32_t imad(uint32_t a, uint32_t b, uint32_t c) {
-#ifdef __CUDA_ARCH__
-    uint32_t r;
-    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-    return r;
-#else
-    return a * b + c;
-#endif
-}
 // a + b rounded down.
 __device__ __forceinline__ float add_rd(float a, float b) {
 #ifdef __CUDA_ARCH__
@@ -54,15 +41,6 @@ __device__ __forceinline__ float add_rd(float a, float b) {
 #endif
 }
 
-// a * 2^-3 + b rounded down, for a * 2^-3 exact.
-__device__ __forceinline__ float eighth_add_rd(float a, float b) {
-#ifdef __CUDA_ARCH__
-    return __fmaf_rd(a, 0.125f, b);
-#else
-    return add_rd(a * 0.125f, b);
-#endif
-}
-
 // Voxel coordinates as floats with an integer part in the low bits.  kVoxelBias is the
 // bit pattern of M = 1.5 * 2^23, where one ulp is 1: for an integer |n| < 2^22 the float
 // M + n has the bits kVoxelBias + n.  With a near world origin the float K = M + worldOrigin
@@ -72,24 +50,12 @@ __device__ __forceinline__ float eighth_add_rd(float a, float b) {
 // gives bits below kVoxelBias or at least the grid's size above it (unsigned).  Back in the ray frame, the float minus K is exactly
 // voxel - worldOrigin.
 constexpr uint32_t kVoxelBias = 0x4B400000u;
-// The brick coordinate of a voxel in the grid the same way: from the biased voxel r the
-// float 2^23 + (v >> 3), bits kBrickBias + (v >> 3).
-constexpr uint32_t kBrickBias = 0x4B000000u;
-__device__ __forceinline__ uint32_t biased_brick(float r) {
-    return __float_as_uint(eighth_add_rd(r, 8388608.0f - 12582912.0f / 8.0f));
-}
-// Table address that takes a biased brick index bx + bz*bsx + by*bsxz: the biases add up to
-// kBrickBias * (1 + bsx + bsxz) mod 2^32, a multiple of 2^24, and a table has at most 2^23
-// entries, so the 32-bit index never wraps past its bias.
-__device__ __forceinline__ const uint32_t* biased_table(const DevWorld& w) {
-    return w.bricks - (size_t)(kBrickBias * (1u + w.bsx + w.bsxz));
-}
 // K of an axis
 __device__ __forceinline__ float voxel_frame(int32_t wo) { return __uint_as_float(kVoxelBias + (uint32_t)wo); }
 
 // v - worldOrigin (wrapping), the ray-frame coordinate of a voxel
 __device__ __forceinline__ float rel_voxel(int32_t v, int32_t wo) {
-    return __int2float_rn((int32_t)imad((uint32_t)wo, 0xFFFFFFFFu, (uint32_t)v));
+    return __int2float_rn(wsub(v, wo));
 }
 
 struct TraceResult {
@@ -147,13 +113,13 @@ struct RayState {
     float tsx, tsy, tsz;  // tStart
     float cx, cy, cz;     // currPos
     float sx, sy, sz;     // sideDist
-    float tb;             // biased tmin of the last step, the distance of the current position (0 at the start)
-    float t_lo, t_hi;     // positions at distances in [t_lo, t_hi) are in the grid (ray_init)
+    float tb;             // GLSL mode: biased tmin of the last step
+    bool fast;            // the ray takes the fast step (ray_init)
     int32_t gx, gy, gz;   // -1 where dir < 0, else 0 (cell alignment side)
     // A hit ends the use of tStart: the step that hits leaves the voxel (as the record packs
     // it) and the brick's slot there, so a lane waiting for its retirement holds no more.
     __device__ __forceinline__ void set_hit(uint32_t x, uint32_t y, uint32_t z, uint32_t slot) {
-        tsx = __uint_as_float(imad(z, 1u << 21, imad(y, 1u << 11, x)));
+        tsx = __uint_as_float(x | y << 11 | z << 21);
         tsy = __uint_as_float(slot);
     }
     __device__ __forceinline__ uint32_t hit_voxel() const { return __float_as_uint(tsx); }
@@ -163,19 +129,14 @@ struct RayState {
     }
 };
 
-// A ray takes the fast step (ray_step<.., true>) while its distance lies in [t_lo, t_hi), where
-// it cannot leave the grid nor meet a NaN, and the general step elsewhere.  The range is empty
-// unless the ray is near and steep enough for these bounds:
-// - |worldOrigin| <= 2^16 and |origin| <= 2^17, so positions in the grid are rounded by less
-//   than 2^-6 and voxels have their biased form;
-// - |1/dir| < 2^95: |tStart| and |(voxel - worldOrigin) * invDir| stay below 2^126, so side
-//   distances and t are finite.
-// The range's ends are where the ray enters (0 when the origin is strictly inside) and leaves
-// the clip box, whose sides lie a voxel inside the grid's: at a distance between them the
-// position o + t*d is within the box on every axis up to the rounding of the ends, of t*d and
-// of the sum, together less than 2^-3.
-constexpr int32_t kNearWorldOrigin = 1 << 16;
-constexpr float kNearOrigin = 0x1p17f, kSafeInvDir = 0x1p95f;
+// A ray takes the fast step (ray_step<.., true>) when no NaN or infinity can occur in its side
+// distances and voxels of the grid have their biased form:
+// - |worldOrigin| <= 2^21 (a near one), so K is exact;
+// - |origin| < 2^30 and |1/dir| < 2^95: |tStart| and |(voxel - worldOrigin) * invDir| stay below
+//   2^126, so side distances and t are finite, and the position o + t*d is finite or an
+//   infinity (never NaN) that leaves the grid.
+constexpr int32_t kNearWorldOrigin = 1 << 21;
+constexpr float kFastOrigin = 0x1p30f, kFastInvDir = 0x1p95f;
 
 // The clip box [1 - worldOrigin, size - 1 - worldOrigin] (VoxelTraversal.glsl:166) of a world
 // origin, and whether that is near: the same for every ray of a view or cast.
@@ -200,14 +161,6 @@ VRT_HD inline ClipBox clip_box(const DevWorld& w, const int32_t wo[3]) {
 VRT_HD inline bool origin_inside_near(const ClipBox& b, float ox, float oy, float oz) {
     return b.near && b.lo[0] < ox && ox < b.hi[0] && b.lo[1] < oy && oy < b.hi[1] && b.lo[2] < oz && oz < b.hi[2];
 }
-// The distances from an origin to the box's sides, per axis the low and the high one.
-struct BoxSides {
-    float lo[3], hi[3];
-};
-VRT_HD inline BoxSides box_sides(const ClipBox& b, float ox, float oy, float oz) {
-    return BoxSides{{b.lo[0] - ox, b.lo[1] - oy, b.lo[2] - oz}, {b.hi[0] - ox, b.hi[1] - oy, b.hi[2] - oz}};
-}
-
 // What every start sets: origin, direction, invDir, tStart, the alignment sides.
 __device__ __forceinline__ void ray_set(RayState& s, float ox, float oy, float oz, float dx, float dy, float dz) {
     s.ox = s.cx = ox;
@@ -226,47 +179,29 @@ __device__ __forceinline__ void ray_set(RayState& s, float ox, float oy, float o
     s.gx = dx < 0.0f ? -1 : 0;
     s.gy = dy < 0.0f ? -1 : 0;
     s.gz = dz < 0.0f ? -1 : 0;
-    s.sx = s.sy = s.sz = s.tb = s.t_lo = 0.0f;
-}
-__device__ __forceinline__ bool ray_finite(const RayState& s) {
-    return fabsf(s.ix) < kSafeInvDir && fabsf(s.iy) < kSafeInvDir && fabsf(s.iz) < kSafeInvDir;
+    s.sx = s.sy = s.sz = 0.0f;
+    s.fast = fabsf(s.ix) < kFastInvDir && fabsf(s.iy) < kFastInvDir && fabsf(s.iz) < kFastInvDir;
 }
 
-// Start of a ray whose origin is inside and near.  Such an origin never clips: per axis
-// l - o < 0 < h - o, so min(t1, t2) of the slab test is negative (or -inf, or NaN when dir is
-// NaN, which minps/maxps drop) and tmin <= 0 on every path.
-__device__ __forceinline__ void ray_init_inside(RayState& s, const BoxSides& b, float ox, float oy, float oz, float dx,
-                                                float dy, float dz) {
-    ray_set(s, ox, oy, oz, dx, dy, dz);
-    const float t = fminf(fminf(__fmul_rn(dx < 0.0f ? b.lo[0] : b.hi[0], s.ix), __fmul_rn(dy < 0.0f ? b.lo[1] : b.hi[1], s.iy)),
-                          __fmul_rn(dz < 0.0f ? b.lo[2] : b.hi[2], s.iz));
-    s.t_hi = ray_finite(s) ? t : 0.0f;
-}
-
-// Start of any ray: the clipped start position (VoxelTraversal.glsl:133-145,163-167) and the
-// range of the fast step.
+// Start of any ray, with the clipped start position (VoxelTraversal.glsl:133-145,163-167).  An
+// origin inside and near never clips: per axis l - o < 0 < h - o, so min(t1, t2) is negative
+// (or -inf, or NaN when dir is NaN, which minps/maxps drop) and tmin <= 0 on every path; for
+// one known to be, ray_set is the whole start.
 __device__ __forceinline__ void ray_init(RayState& s, const ClipBox& b, float ox, float oy, float oz, float dx,
                                          float dy, float dz) {
-    const BoxSides d = box_sides(b, ox, oy, oz);
-    if (origin_inside_near(b, ox, oy, oz)) {
-        ray_init_inside(s, d, ox, oy, oz, dx, dy, dz);
-        return;
-    }
     ray_set(s, ox, oy, oz, dx, dy, dz);
-    const float t1x = __fmul_rn(d.lo[0], s.ix), t1y = __fmul_rn(d.lo[1], s.iy), t1z = __fmul_rn(d.lo[2], s.iz);
-    const float t2x = __fmul_rn(d.hi[0], s.ix), t2y = __fmul_rn(d.hi[1], s.iy), t2z = __fmul_rn(d.hi[2], s.iz);
+    if (origin_inside_near(b, ox, oy, oz)) return;
+    const float t1x = __fmul_rn(__fsub_rn(b.lo[0], ox), s.ix), t2x = __fmul_rn(__fsub_rn(b.hi[0], ox), s.ix);
+    const float t1y = __fmul_rn(__fsub_rn(b.lo[1], oy), s.iy), t2y = __fmul_rn(__fsub_rn(b.hi[1], oy), s.iy);
+    const float t1z = __fmul_rn(__fsub_rn(b.lo[2], oz), s.iz), t2z = __fmul_rn(__fsub_rn(b.hi[2], oz), s.iz);
     const float tmin = max_x86(min_x86(t1x, t2x), max_x86(min_x86(t1y, t2y), min_x86(t1z, t2z)));
     const float tmax = min_x86(max_x86(t1x, t2x), min_x86(max_x86(t1y, t2y), max_x86(t1z, t2z)));
-    s.t_hi = 0.0f;
     if (tmin > 0.0f && tmin < tmax) {
         s.cx = __fadd_rn(ox, __fmul_rn(dx, tmin));
         s.cy = __fadd_rn(oy, __fmul_rn(dy, tmin));
         s.cz = __fadd_rn(oz, __fmul_rn(dz, tmin));
-        if (b.near && ray_finite(s) && fabsf(ox) < kNearOrigin && fabsf(oy) < kNearOrigin && fabsf(oz) < kNearOrigin) {
-            s.tb = s.t_lo = tmin;
-            s.t_hi = tmax;
-        }
     }
+    s.fast = s.fast && b.near && fabsf(ox) < kFastOrigin && fabsf(oy) < kFastOrigin && fabsf(oz) < kFastOrigin;
 }
 
 // GLSL mode: the step's distance and position from its side distances.  tmin + 5 ulp as
@@ -274,10 +209,10 @@ __device__ __forceinline__ void ray_init(RayState& s, const ClipBox& b, float ox
 // platforms: the GPU's 0x7FFFFFFF would wrap to a denormal).  A rayCastCoarse ray takes
 // tmin + 0.001 (VoxelTraversal.glsl:213).  Kept as the hit distance, so min keeps the minps
 // rule.
-template <bool kSafe>
+template <bool kFast>
 __device__ __forceinline__ void glsl_advance(RayState& s, bool coarse_ray) {
     const float m = min_x86(min_x86(s.sx, s.sy), s.sz);
-    const float t = coarse_ray ? __fadd_rn(m, 0.001f) : (!kSafe && m != m) ? m : __uint_as_float(__float_as_uint(m) + 5u);
+    const float t = coarse_ray ? __fadd_rn(m, 0.001f) : (!kFast && m != m) ? m : __uint_as_float(__float_as_uint(m) + 5u);
     s.tb = t;
     s.cx = __fadd_rn(s.ox, __fmul_rn(t, s.dx));
     s.cy = __fadd_rn(s.oy, __fmul_rn(t, s.dy));
@@ -301,9 +236,6 @@ __device__ __forceinline__ void glsl_start(RayState& s, int32_t wox, int32_t woy
         s.tsx = __fmul_rn(__fsub_rn(s.dx < 0.0f ? 0.0f : 1.0f, s.ox), s.ix);
         s.tsy = __fmul_rn(__fsub_rn(s.dy < 0.0f ? 0.0f : 1.0f, s.oy), s.iy);
         s.tsz = __fmul_rn(__fsub_rn(s.dz < 0.0f ? 0.0f : 1.0f, s.oz), s.iz);
-        // distances count from the clipped start, and so do the range's ends
-        s.t_hi = s.t_hi > 0.0f ? __fsub_rn(s.t_hi, s.t_lo) : 0.0f;
-        s.t_lo = 0.0f;
     }
     // (voxel - worldOrigin in wrapping arithmetic, where the start voxel saturated)
     s.sx = __fadd_rn(s.tsx, __fmul_rn(rel_voxel(wadd(wox, floor2i(s.cx)), wox), s.ix));
@@ -321,9 +253,9 @@ __device__ __forceinline__ void ray_start(RayState& s, const ClipBox& b, float o
     glsl_start<kGlsl>(s, wox, woy, woz, coarse_origin);
 }
 template <bool kGlsl>
-__device__ __forceinline__ void ray_start_inside(RayState& s, const BoxSides& b, float ox, float oy, float oz, float dx,
+__device__ __forceinline__ void ray_start_inside(RayState& s, float ox, float oy, float oz, float dx,
                                                  float dy, float dz, int32_t wox, int32_t woy, int32_t woz) {
-    ray_init_inside(s, b, ox, oy, oz, dx, dy, dz);
+    ray_set(s, ox, oy, oz, dx, dy, dz);
     glsl_start<kGlsl>(s, wox, woy, woz, false);
 }
 
@@ -366,27 +298,26 @@ __device__ __forceinline__ uint32_t coarse_bits(bool coarse_ray, uint32_t i) {
     return coarse_ray ? (kCoarseRay | (i >= kCoarseFrom ? kCoarseNow : 0u)) : 0u;
 }
 
-// The end of a step: from the voxel (of a safe ray in its biased form) and the alignment
+// The end of a step: from the voxel (of a fast ray in its biased form) and the alignment
 // mask of its cell to the cell's side distances, tmin and the next position.
-template <bool kSafe, bool kGlsl, bool kCoarse>
+template <bool kFast, bool kGlsl, bool kCoarse>
 __device__ __forceinline__ void step_on(RayState& s, uint32_t vx, uint32_t vy, uint32_t vz, uint32_t m, int32_t wox,
                                         int32_t woy, int32_t woz, uint32_t coarse) {
     // dir < 0 ? pos & ~m : pos | m, as (pos | m) ^ (g & m) with g = -1 for dir < 0
     vx = (vx | m) ^ ((uint32_t)s.gx & m);
     vy = (vy | m) ^ ((uint32_t)s.gy & m);
     vz = (vz | m) ^ ((uint32_t)s.gz & m);
-    const float fx = kSafe ? __fsub_rn(__uint_as_float(vx), voxel_frame(wox)) : rel_voxel((int32_t)vx, wox);
-    const float fy = kSafe ? __fsub_rn(__uint_as_float(vy), voxel_frame(woy)) : rel_voxel((int32_t)vy, woy);
-    const float fz = kSafe ? __fsub_rn(__uint_as_float(vz), voxel_frame(woz)) : rel_voxel((int32_t)vz, woz);
+    const float fx = kFast ? __fsub_rn(__uint_as_float(vx), voxel_frame(wox)) : rel_voxel((int32_t)vx, wox);
+    const float fy = kFast ? __fsub_rn(__uint_as_float(vy), voxel_frame(woy)) : rel_voxel((int32_t)vy, woy);
+    const float fz = kFast ? __fsub_rn(__uint_as_float(vz), voxel_frame(woz)) : rel_voxel((int32_t)vz, woz);
     s.sx = __fadd_rn(s.tsx, __fmul_rn(fx, s.ix));
     s.sy = __fadd_rn(s.tsy, __fmul_rn(fy, s.iy));
     s.sz = __fadd_rn(s.tsz, __fmul_rn(fz, s.iz));
     if (kGlsl) {
-        glsl_advance<kSafe>(s, kCoarse && (coarse & kCoarseRay) != 0);
+        glsl_advance<kFast>(s, kCoarse && (coarse & kCoarseRay) != 0);
     } else {
-        const float t = kSafe ? __fadd_rn(fminf(fminf(s.sx, s.sy), s.sz), 0.001f)
+        const float t = kFast ? __fadd_rn(fminf(fminf(s.sx, s.sy), s.sz), 0.001f)
                               : __fadd_rn(min_x86(min_x86(s.sx, s.sy), s.sz), 0.001f);
-        s.tb = t;
         s.cx = __fadd_rn(s.ox, __fmul_rn(t, s.dx));
         s.cy = __fadd_rn(s.oy, __fmul_rn(t, s.dy));
         s.cz = __fadd_rn(s.oz, __fmul_rn(t, s.dz));
@@ -396,10 +327,9 @@ __device__ __forceinline__ void step_on(RayState& s, uint32_t vx, uint32_t vy, u
 // One iteration of RayCast (CpuRenderer.cpp:186-201) with GetStepPos (:135-171): the voxel
 // of the current position, its bounds and table entries, then the side distances of the cell
 // reached, tmin and the next position.
-// kSafe: the distance lies in the ray's range of ray_init, so the position is in the grid, no
-// NaN can occur and voxels are kept in the biased form of kVoxelBias; min uses fminf, which
-// equals the minps rule on non-NaN operands up to the sign of a zero result, which the +0.001
-// bias removes.
+// kFast: the ray passed the bounds of ray_init, so no NaN can occur and voxels are kept in the
+// biased form of kVoxelBias; min uses fminf, which equals the minps rule on non-NaN operands
+// up to the sign of a zero result, which the +0.001 bias removes.
 // kGlsl: rayCast (VoxelTraversal.glsl:170-199), whose iteration takes its position first
 // (ray_start has iteration 0's): bounds, then getStepPos (:100-131), whose empty sectors take
 // the 4th-level mask from the brick table.  kCoarse (with kGlsl): the step may belong to a
@@ -410,23 +340,15 @@ __device__ __forceinline__ void step_on(RayState& s, uint32_t vx, uint32_t vy, u
 // kAniso (with kGlsl): anisotropic LODs (u_UseAnisotropicLods, :116-121): the mask of
 // the current level (cell, sector or sector group, read raw instead of through the
 // precomputed codes) is restricted to the cells ahead of the ray before its LOD is taken.
-template <bool kCount, bool kSafe = false, bool kGlsl = false, bool kCoarse = false, bool kAniso = false>
-__device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, const uint32_t* biased, int32_t wox,
-                                             int32_t woy, int32_t woz, TraceCounters& cnt, uint32_t coarse = 0) {
-    uint32_t vx, vy, vz;  // the voxel; of a safe ray its biased form
-    uint32_t bx, by, bz;  // its brick, likewise
-    uint32_t e;
-    constexpr uint32_t kBias = kSafe ? kVoxelBias : 0u;
-    if (kSafe) {
-        const float rx = add_rd(s.cx, voxel_frame(wox)), ry = add_rd(s.cy, voxel_frame(woy)),
-                    rz = add_rd(s.cz, voxel_frame(woz));
-        vx = __float_as_uint(rx);
-        vy = __float_as_uint(ry);
-        vz = __float_as_uint(rz);
-        bx = biased_brick(rx);
-        by = biased_brick(ry);
-        bz = biased_brick(rz);
-        e = __ldg(biased + imad(by, w.bsxz, imad(bz, w.bsx, bx)));
+template <bool kCount, bool kFast = false, bool kGlsl = false, bool kCoarse = false, bool kAniso = false>
+__device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int32_t wox, int32_t woy, int32_t woz,
+                                             TraceCounters& cnt, uint32_t coarse = 0) {
+    uint32_t vx, vy, vz;  // the voxel; of a fast ray its biased form
+    constexpr uint32_t kBias = kFast ? kVoxelBias : 0u;
+    if (kFast) {
+        vx = __float_as_uint(add_rd(s.cx, voxel_frame(wox)));
+        vy = __float_as_uint(add_rd(s.cy, voxel_frame(woy)));
+        vz = __float_as_uint(add_rd(s.cz, voxel_frame(woz)));
     } else {
         // floor2i: a NaN coordinate converts to INT32_MIN on x86 and leaves the grid;
         // cvt.rmi saturates infinities and out-of-range values, which leave the grid
@@ -437,12 +359,11 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, con
         vx = (uint32_t)wadd(__float2int_rd(s.cx), wox);
         vy = (uint32_t)wadd(__float2int_rd(s.cy), woy);
         vz = (uint32_t)wadd(__float2int_rd(s.cz), woz);
-        if (!(vx < w.size_x && vy < w.size_y && vz < w.size_z)) return kStepOut;
-        bx = vx >> 3;
-        by = vy >> 3;
-        bz = vz >> 3;
-        e = __ldg(w.bricks + bx + bz * w.bsx + by * w.bsxz);
     }
+    const uint32_t ux = vx - kBias, uy = vy - kBias, uz = vz - kBias;
+    if (!(ux < w.size_x && uy < w.size_y && uz < w.size_z)) return kStepOut;
+    const uint32_t bx = ux >> 3, by = uy >> 3, bz = uz >> 3;
+    const uint32_t e = __ldg(w.bricks + bx + bz * w.bsx + by * w.bsxz);
     if (kCount) cnt.step_calls++;
     // The brick table holds the slot of an allocated brick, or for an empty one the
     // alignment mask of the level GetStepPos reaches from the sector mask
@@ -453,11 +374,11 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, con
     if (kGlsl && kAniso) {
         if (e < kBrickEmpty) {
             if (kCount) cnt.occ_fetches++;
-            const uint32_t lx = vx & 7u, ly = vy & 7u, lz = vz & 7u;
+            const uint32_t lx = ux & 7u, ly = uy & 7u, lz = uz & 7u;
             const uint64_t cm = __ldg(w.cells + (size_t)e * 8 + ((lx >> 2) | (lz >> 2) << 1 | (ly >> 2) << 2));
             const uint32_t idx = (lx & 3u) | (lz & 3u) << 2 | (ly & 3u) << 4;
             if ((cm >> idx) & 1u) {
-                s.set_hit(vx - kBias, vy - kBias, vz - kBias, e);
+                s.set_hit(ux, uy, uz, e);
                 return kStepHit;
             }
             const uint32_t li = idx + 64u * ((uint32_t)(s.gx + 1) | (uint32_t)(s.gy + 1) << 1 | (uint32_t)(s.gz + 1) << 2);
@@ -465,8 +386,8 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, con
             if (kCoarse && (coarse & kCoarseNow) && am != 0) {
                 // findAnyOccupiedPos on the masked cell mask: its lowest set bit
                 const uint32_t j = (uint32_t)__ffsll((long long)am) - 1u;
-                s.set_hit(((vx - kBias) & ~3u) | (j & 3u), ((vy - kBias) & ~3u) | (j >> 4),
-                          ((vz - kBias) & ~3u) | ((j >> 2) & 3u), e);
+                s.set_hit((ux & ~3u) | (j & 3u), (uy & ~3u) | (j >> 4),
+                          (uz & ~3u) | ((j >> 2) & 3u), e);
                 return kStepHit;
             }
             m = am == 0 ? 3u : ((cm & s_forward_lut[1][li]) == 0 ? 1u : 0u);
@@ -480,26 +401,22 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, con
         }
     } else if (e < kBrickEmpty) {
         if (kCount) cnt.occ_fetches++;
-        // voxel in brick v = x | z<<3 | y<<6 from v - 8*(v >> 3) per axis; its code byte.
-        // The biases of a safe ray's sum (a multiple of 2^22, so v < 512 does not carry)
-        // go into the base address.
-        constexpr uint32_t kViBias = kSafe ? 73u * (kVoxelBias - 8u * kBrickBias) : 0u;
-        const uint32_t lx = imad(bx, 0xFFFFFFF8u, vx), ly = imad(by, 0xFFFFFFF8u, vy), lz = imad(bz, 0xFFFFFFF8u, vz);
-        const uint32_t vi = imad(ly, 64u, imad(lz, 8u, lx));
-        const uint32_t code = __ldg(w.codes - (size_t)kViBias + (size_t)e * 512 + vi);
+        // voxel in brick x | z<<3 | y<<6
+        const uint32_t vi = (ux & 7u) | (uz & 7u) << 3 | (uy & 7u) << 6;
+        const uint32_t code = __ldg(w.codes + (size_t)e * 512 + vi);
         if (code == kCodeSolid) {
-            s.set_hit(vx - kBias, vy - kBias, vz - kBias, e);
+            s.set_hit(ux, uy, uz, e);
             return kStepHit;
         }
         if (kGlsl && kCoarse && (coarse & kCoarseNow) && code != 3u) {
             // the cell's mask is not empty (lod < 4): its first solid voxel, bit
             // x + z*4 + y*16 of the cell mask, is the hit (mask-order scan of the payload)
-            const size_t cell = (size_t)e * 512 + ((vx & 4u) | (vz & 4u) << 3 | (vy & 4u) << 6);
+            const size_t cell = (size_t)e * 512 + ((ux & 4u) | (uz & 4u) << 3 | (uy & 4u) << 6);
             for (uint32_t j = 0; j < 64; j++) {
                 const size_t c = cell + ((j & 3u) | ((j >> 2) & 3u) << 3 | (j >> 4) << 6);
                 if (__ldg(w.payload + c)) {
-                    s.set_hit(((vx - kBias) & ~3u) | (j & 3u), ((vy - kBias) & ~3u) | (j >> 4),
-                              ((vz - kBias) & ~3u) | ((j >> 2) & 3u), e);
+                    s.set_hit((ux & ~3u) | (j & 3u), (uy & ~3u) | (j >> 4),
+                              (uz & ~3u) | ((j >> 2) & 3u), e);
                     return kStepHit;
                 }
             }
@@ -508,30 +425,31 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, con
     } else {
         m = kGlsl ? (e >> 8) & 127u : e & 31u;
     }
-    step_on<kSafe, kGlsl, kCoarse>(s, vx, vy, vz, m, wox, woy, woz, coarse);
+    step_on<kFast, kGlsl, kCoarse>(s, vx, vy, vz, m, wox, woy, woz, coarse);
     return kStepContinue;
 }
 
 // Steps k = k .. kmax-1 of a ray whose first step here is its iteration i0 + k, until
-// one ends it (the returned status) or kmax is reached (kStepContinue): fast steps while the
-// distance lies in the ray's range, then general ones (a ray that misses takes one or two at
-// the grid's edge).  The loops follow each other; a choice between them cost the fast one ten
-// register moves a step (59 instead of 48 instructions).  coarse_ray: a rayCastCoarse ray
-// (kCoarse only).
+// one ends it (the returned status) or kmax is reached (kStepContinue).  The general step's loop
+// follows the fast one, which it leaves in place: a choice between the two cost the fast loop
+// ten register moves a step (59 instead of 49 instructions).  A test of the distance against
+// the grid's exit in place of the three bounds compares saved nothing, and lanes past the
+// exit, stepping in the second loop, doubled the time of warps with stalled rays.
+// coarse_ray: a rayCastCoarse ray (kCoarse only).
 template <bool kCount, bool kGlsl, bool kCoarse, bool kAniso>
 __device__ __forceinline__ uint32_t dda_steps(RayState& s, const DevWorld& w, int32_t wox, int32_t woy, int32_t woz,
                                               TraceCounters& cnt, bool coarse_ray, uint32_t i0, uint32_t& k,
                                               uint32_t kmax) {
     uint32_t st = kStepContinue;
-    const uint32_t* biased = biased_table(w);
-    while (k < kmax && s.tb >= s.t_lo && s.tb < s.t_hi) {
-        st = ray_step<kCount, true, kGlsl, kCoarse, kAniso>(s, w, biased, wox, woy, woz, cnt,
+    const uint32_t kfast = s.fast ? kmax : 0u;
+    while (k < kfast) {
+        st = ray_step<kCount, true, kGlsl, kCoarse, kAniso>(s, w, wox, woy, woz, cnt,
                                                             kCoarse ? coarse_bits(coarse_ray, i0 + k) : 0u);
         if (st != kStepContinue) return st;
         k++;
     }
     for (; k < kmax; k++) {
-        st = ray_step<kCount, false, kGlsl, kCoarse, kAniso>(s, w, nullptr, wox, woy, woz, cnt,
+        st = ray_step<kCount, false, kGlsl, kCoarse, kAniso>(s, w, wox, woy, woz, cnt,
                                                              kCoarse ? coarse_bits(coarse_ray, i0 + k) : 0u);
         if (st != kStepContinue) break;
     }

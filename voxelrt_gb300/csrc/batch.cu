@@ -272,7 +272,7 @@ __device__ __forceinline__ void resident_pixels_done(const BatchParams& p, uint3
 
 // kFull: the launch may hold views with the GPU renderer's whole path (a separate
 // instantiation, so the others keep their code and registers).  64 registers (32 warps a SM)
-// are enough for the CPU traversal (two 720p views of 4 bounces: 443 us against 450 us with
+// are enough for the CPU traversal (two 720p views of 4 bounces: 409 us against 429 us with
 // 72), not for the GLSL modes (two worlds' whole paths: 735 us against 717 us).
 template <bool kCount, bool kGlsl, bool kResident = false, bool kAniso = false, bool kFull = false>
 __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
@@ -593,7 +593,7 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
                 uint32_t k = 0;
                 // GLSL mode: the rayCastCoarse variant while some lane traces a shadow or
                 // bounce ray, the anisotropic one for views that ask for it
-                const uint32_t st = dda_steps_mode<kCount, kGlsl>(s, w, wv.x, wv.y, wv.z, cnt, any_coarse,
+                const uint32_t st = dda_steps_mode<kCount, kGlsl, true>(s, w, wv.x, wv.y, wv.z, cnt, any_coarse,
                                                                   (path & 0xFFu) != 0, kAniso, iter, k, kmax);
                 iter += k;  // the iteration a ray left on, or max_iters when the cap ran out
                 if (st != kStepContinue)

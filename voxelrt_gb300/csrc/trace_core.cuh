@@ -340,7 +340,14 @@ __device__ __forceinline__ void step_on(RayState& s, uint32_t vx, uint32_t vy, u
 // kAniso (with kGlsl): anisotropic LODs (u_UseAnisotropicLods, :116-121): the mask of
 // the current level (cell, sector or sector group, read raw instead of through the
 // precomputed codes) is restricted to the cells ahead of the ray before its LOD is taken.
-template <bool kCount, bool kFast = false, bool kGlsl = false, bool kCoarse = false, bool kAniso = false>
+// kFlat (not with kAniso): no branch on what the brick is.  A position outside reads no entry
+// and takes kOutside, whose masks are the solid code, so one test ends the ray either way,
+// and an allocated brick's code is a predicated load.  Fewer branches, more instructions for
+// an empty brick: for rays that diverge in any case (bounces of two 720p views: 423 -> 409 us;
+// 4.2 M random rays: 252 -> 248 us, 16,000: 20.2 -> 18.7 us); camera rays over terrain lose (six
+// 1080p views with sun rays 779 -> 816 us).
+constexpr uint32_t kOutside = kBrickEmpty | kCodeSolid | kCodeSolid << 8;
+template <bool kCount, bool kFast, bool kGlsl, bool kCoarse, bool kAniso, bool kFlat>
 __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int32_t wox, int32_t woy, int32_t woz,
                                              TraceCounters& cnt, uint32_t coarse = 0) {
     uint32_t vx, vy, vz;  // the voxel; of a fast ray its biased form
@@ -361,17 +368,20 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int
         vz = (uint32_t)wadd(__float2int_rd(s.cz), woz);
     }
     const uint32_t ux = vx - kBias, uy = vy - kBias, uz = vz - kBias;
-    if (!(ux < w.size_x && uy < w.size_y && uz < w.size_z)) return kStepOut;
-    const uint32_t bx = ux >> 3, by = uy >> 3, bz = uz >> 3;
-    const uint32_t e = __ldg(w.bricks + bx + bz * w.bsx + by * w.bsxz);
-    if (kCount) cnt.step_calls++;
+    const bool in = ux < w.size_x && uy < w.size_y && uz < w.size_z;
+    // (the sum in 32 bits: added to the pointer term by term it takes three wide adds)
+    const uint32_t ei = (uy >> 3) * w.bsxz + ((uz >> 3) * w.bsx + (ux >> 3));
+    const uint32_t vi = (ux & 7u) | (uz & 7u) << 3 | (uy & 7u) << 6;  // voxel in brick x | z<<3 | y<<6
     // The brick table holds the slot of an allocated brick, or for an empty one the
     // alignment mask of the level GetStepPos reaches from the sector mask
     // (3 + skip_levels).  An allocated brick's voxel code is kCodeSolid (the hit) or
     // the alignment mask of the skip level of the voxel's 4^3 cell; both replace the
     // two mask fetches of the reference with their precomputed outcome.
-    uint32_t m;
-    if (kGlsl && kAniso) {
+    uint32_t e, m;
+    if (kAniso) {
+        if (!in) return kStepOut;
+        if (kCount) cnt.step_calls++;
+        e = __ldg(w.bricks + ei);
         if (e < kBrickEmpty) {
             if (kCount) cnt.occ_fetches++;
             const uint32_t lx = ux & 7u, ly = uy & 7u, lz = uz & 7u;
@@ -386,8 +396,7 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int
             if (kCoarse && (coarse & kCoarseNow) && am != 0) {
                 // findAnyOccupiedPos on the masked cell mask: its lowest set bit
                 const uint32_t j = (uint32_t)__ffsll((long long)am) - 1u;
-                s.set_hit((ux & ~3u) | (j & 3u), (uy & ~3u) | (j >> 4),
-                          (uz & ~3u) | ((j >> 2) & 3u), e);
+                s.set_hit((ux & ~3u) | (j & 3u), (uy & ~3u) | (j >> 4), (uz & ~3u) | ((j >> 2) & 3u), e);
                 return kStepHit;
             }
             m = am == 0 ? 3u : ((cm & s_forward_lut[1][li]) == 0 ? 1u : 0u);
@@ -399,31 +408,43 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int
             const uint32_t skip = ((e >> (kAnisoShift + oct2)) & 3u) + ((e >> 4) & 2u);
             m = (8u << skip) - 1u;
         }
-    } else if (e < kBrickEmpty) {
-        if (kCount) cnt.occ_fetches++;
-        // voxel in brick x | z<<3 | y<<6
-        const uint32_t vi = (ux & 7u) | (uz & 7u) << 3 | (uy & 7u) << 6;
-        const uint32_t code = __ldg(w.codes + (size_t)e * 512 + vi);
-        if (code == kCodeSolid) {
+    } else if (kFlat) {
+        e = kOutside;
+        if (in) e = __ldg(w.bricks + ei);
+        if (kCount && in) cnt.step_calls++;
+        m = kGlsl ? (e >> 8) & 127u : e & 31u;
+        if (e < kBrickEmpty) m = __ldg(w.codes + (size_t)e * 512 + vi);
+        if (kCount && e < kBrickEmpty) cnt.occ_fetches++;
+        if (m == kCodeSolid) {
+            if (e == kOutside) return kStepOut;
             s.set_hit(ux, uy, uz, e);
             return kStepHit;
         }
-        if (kGlsl && kCoarse && (coarse & kCoarseNow) && code != 3u) {
-            // the cell's mask is not empty (lod < 4): its first solid voxel, bit
-            // x + z*4 + y*16 of the cell mask, is the hit (mask-order scan of the payload)
-            const size_t cell = (size_t)e * 512 + ((ux & 4u) | (uz & 4u) << 3 | (uy & 4u) << 6);
-            for (uint32_t j = 0; j < 64; j++) {
-                const size_t c = cell + ((j & 3u) | ((j >> 2) & 3u) << 3 | (j >> 4) << 6);
-                if (__ldg(w.payload + c)) {
-                    s.set_hit((ux & ~3u) | (j & 3u), (uy & ~3u) | (j >> 4),
-                              (uz & ~3u) | ((j >> 2) & 3u), e);
-                    return kStepHit;
-                }
+    } else {
+        if (!in) return kStepOut;
+        if (kCount) cnt.step_calls++;
+        e = __ldg(w.bricks + ei);
+        if (e < kBrickEmpty) {
+            if (kCount) cnt.occ_fetches++;
+            m = __ldg(w.codes + (size_t)e * 512 + vi);
+            if (m == kCodeSolid) {
+                s.set_hit(ux, uy, uz, e);
+                return kStepHit;
+            }
+        } else {
+            m = kGlsl ? (e >> 8) & 127u : e & 31u;
+        }
+    }
+    if (kGlsl && kCoarse && !kAniso && (coarse & kCoarseNow) && e < kBrickEmpty && m != 3u) {
+        // the cell's mask is not empty (lod < 4): its first solid voxel, bit
+        // x + z*4 + y*16 of the cell mask, is the hit (mask-order scan of the payload)
+        const size_t cell = (size_t)e * 512 + ((ux & 4u) | (uz & 4u) << 3 | (uy & 4u) << 6);
+        for (uint32_t j = 0; j < 64; j++) {
+            if (__ldg(w.payload + cell + ((j & 3u) | ((j >> 2) & 3u) << 3 | (j >> 4) << 6))) {
+                s.set_hit((ux & ~3u) | (j & 3u), (uy & ~3u) | (j >> 4), (uz & ~3u) | ((j >> 2) & 3u), e);
+                return kStepHit;
             }
         }
-        m = code;
-    } else {
-        m = kGlsl ? (e >> 8) & 127u : e & 31u;
     }
     step_on<kFast, kGlsl, kCoarse>(s, vx, vy, vz, m, wox, woy, woz, coarse);
     return kStepContinue;
@@ -436,20 +457,20 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int
 // the grid's exit in place of the three bounds compares saved nothing, and lanes past the
 // exit, stepping in the second loop, doubled the time of warps with stalled rays.
 // coarse_ray: a rayCastCoarse ray (kCoarse only).
-template <bool kCount, bool kGlsl, bool kCoarse, bool kAniso>
+template <bool kCount, bool kGlsl, bool kCoarse, bool kAniso, bool kFlat>
 __device__ __forceinline__ uint32_t dda_steps(RayState& s, const DevWorld& w, int32_t wox, int32_t woy, int32_t woz,
                                               TraceCounters& cnt, bool coarse_ray, uint32_t i0, uint32_t& k,
                                               uint32_t kmax) {
     uint32_t st = kStepContinue;
     const uint32_t kfast = s.fast ? kmax : 0u;
     while (k < kfast) {
-        st = ray_step<kCount, true, kGlsl, kCoarse, kAniso>(s, w, wox, woy, woz, cnt,
+        st = ray_step<kCount, true, kGlsl, kCoarse, kAniso, kFlat>(s, w, wox, woy, woz, cnt,
                                                             kCoarse ? coarse_bits(coarse_ray, i0 + k) : 0u);
         if (st != kStepContinue) return st;
         k++;
     }
     for (; k < kmax; k++) {
-        st = ray_step<kCount, false, kGlsl, kCoarse, kAniso>(s, w, wox, woy, woz, cnt,
+        st = ray_step<kCount, false, kGlsl, kCoarse, kAniso, false>(s, w, wox, woy, woz, cnt,
                                                              kCoarse ? coarse_bits(coarse_ray, i0 + k) : 0u);
         if (st != kStepContinue) break;
     }
@@ -458,19 +479,19 @@ __device__ __forceinline__ uint32_t dda_steps(RayState& s, const DevWorld& w, in
 
 // dda_steps with the GLSL variants picked at run time: coarse (some ray of the caller's
 // group may be a rayCastCoarse ray; coarse_ray says whether this one is) and aniso.
-template <bool kCount, bool kGlsl>
+template <bool kCount, bool kGlsl, bool kFlat = false>
 __device__ __forceinline__ uint32_t dda_steps_mode(RayState& s, const DevWorld& w, int32_t wox, int32_t woy,
                                                    int32_t woz, TraceCounters& cnt, bool coarse,
                                                    bool coarse_ray, bool aniso, uint32_t i0, uint32_t& k,
                                                    uint32_t kmax) {
     if constexpr (!kGlsl) {
-        return dda_steps<kCount, false, false, false>(s, w, wox, woy, woz, cnt, false, i0, k, kmax);
+        return dda_steps<kCount, false, false, false, kFlat>(s, w, wox, woy, woz, cnt, false, i0, k, kmax);
     } else {
         if (aniso)
-            return coarse ? dda_steps<kCount, true, true, true>(s, w, wox, woy, woz, cnt, coarse_ray, i0, k, kmax)
-                          : dda_steps<kCount, true, false, true>(s, w, wox, woy, woz, cnt, false, i0, k, kmax);
-        return coarse ? dda_steps<kCount, true, true, false>(s, w, wox, woy, woz, cnt, coarse_ray, i0, k, kmax)
-                      : dda_steps<kCount, true, false, false>(s, w, wox, woy, woz, cnt, false, i0, k, kmax);
+            return coarse ? dda_steps<kCount, true, true, true, false>(s, w, wox, woy, woz, cnt, coarse_ray, i0, k, kmax)
+                          : dda_steps<kCount, true, false, true, false>(s, w, wox, woy, woz, cnt, false, i0, k, kmax);
+        return coarse ? dda_steps<kCount, true, true, false, kFlat>(s, w, wox, woy, woz, cnt, coarse_ray, i0, k, kmax)
+                      : dda_steps<kCount, true, false, false, kFlat>(s, w, wox, woy, woz, cnt, false, i0, k, kmax);
     }
 }
 

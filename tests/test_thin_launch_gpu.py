@@ -1,0 +1,42 @@
+"""Small launches (thin_lanes_log2 in trace.cu: 4 to 32 rays per warp) against the oracle, at
+the ray counts where the rays per warp change and at the remainders of a warp and a block;
+frames of odd shapes likewise.  Every record word is equal."""
+import numpy as np
+import pytest
+
+import voxelrt_gb300 as v
+from tests.helpers import both_worlds
+
+pytestmark = pytest.mark.gpu
+# n >> (l - 1) <= warps: casts 2432 warps (4 rays a warp up to 9728 rays, 8 to 19456, 16 to 38912)
+COUNTS = [1, 3, 4, 5, 31, 33, 127, 2000, 9728, 9731, 19456, 19459, 38911, 38915]
+# frames 1216 warps (4 up to 4864 pixels, 8 to 9728, 16 to 19456)
+SHAPES = [(1, 1), (3, 2), (64, 64), (76, 64), (77, 64), (4864, 1), (1, 4866), (139, 70), (128, 76), (195, 100), (140, 139)]
+
+
+@pytest.fixture(scope="module")
+def world(gpu):
+    w, o = both_worlds(v.synth_mix(96, seed=5))
+    yield w, o
+    w.close()
+
+
+def words(a):
+    return np.ascontiguousarray(a).view(np.uint32)
+
+
+@pytest.mark.parametrize("mode", [{}, dict(glsl=True), dict(coarse=True), dict(aniso=True)], ids=lambda m: "+".join(m) or "cpu")
+def test_casts(world, mode):
+    w, o = world
+    rays = v.random_rays((96, 96, 96), seed=9, n=max(COUNTS))
+    want = words(o.cast(rays, glsl=bool(mode), coarse=mode.get("coarse", False), aniso=mode.get("aniso", False)))
+    for n in COUNTS:
+        assert np.array_equal(words(w.cast(rays[:n], **mode)), want[: 4 * n]), n
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_frames(world, shape):
+    w, o = world
+    for pos in ((50.3, 70.1, 20.7), (-30.0, 60.0, 48.0)):  # inside, outside the world
+        cam = v.look_at(pos, (48, 40, 48), 70.0, *shape)
+        assert np.array_equal(words(w.render_view(cam)), words(o.render_view(cam)))

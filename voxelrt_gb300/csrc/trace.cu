@@ -21,14 +21,31 @@ uint32_t eff_iters(uint32_t max_iters, bool glsl = false) {
     return max_iters > 65535u ? 65535u : max_iters;
 }
 
+// Rays per warp of a small launch (log2, 2..5): as few as keep the launch within `warps` warps.
+// A launch that leaves most of the chip idle lasts as long as its longest ray, and a ray's
+// step waits for the slowest lane of its warp: with 4 rays a warp a 64x64 frame of a
+// 256-voxel terrain takes 12.5 us against 14.5, 2,000 random rays 16.4 us against 18.6 (one ray a
+// warp: 12.7 and 15.6, but 2,000 GLSL rays 55 us against 41).  `warps` where the gain ends:
+// casts 32,000 rays; frames earlier, as one whose rays end at once lasts as long as its
+// blocks take to launch (192x192 from within a solid voxel: 4.0 us, thinned 5.2 us).
+constexpr uint32_t kThinFrameWarps = 1216, kThinCastWarps = 2432;
+uint32_t thin_lanes_log2(uint64_t rays, uint32_t warps) {
+    uint32_t l = 5;
+    while (l > 2 && rays >> (l - 1) <= warps) l--;
+    return l;
+}
+
+// One thread per pixel, 2 warps per block, each an area of 2^lanes_log2 pixels (8x4 for 32).
 // inside: the camera origin is (origin_inside_near)
 __global__ void __launch_bounds__(64) render_view_kernel(const __grid_constant__ DevWorld w,
                                                         const __grid_constant__ vrt_camera cam,
                                                         const __grid_constant__ ClipBox clip, bool inside,
-                                                        uint32_t max_iters,
+                                                        uint32_t lanes_log2, uint32_t max_iters,
                                                         uint4* __restrict__ out) {
-    const uint32_t px = blockIdx.x * 8 + threadIdx.x;
-    const uint32_t py = blockIdx.y * 8 + threadIdx.y;
+    const uint32_t lane = threadIdx.x & 31, wl = (lanes_log2 + 1) / 2;
+    if (lane >> lanes_log2) return;
+    const uint32_t px = (blockIdx.x << wl) + (lane & ((1u << wl) - 1u));
+    const uint32_t py = ((blockIdx.y * 2 + (threadIdx.x >> 5)) << (lanes_log2 - wl)) + (lane >> wl);
     if (px >= cam.width || py >= cam.height) return;
     float dx, dy, dz;
     camera_ray(cam, px, py, dx, dy, dz);
@@ -49,16 +66,19 @@ template <bool kGlsl, bool kAniso = false>
 __global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ClipBox clip,
                                                   const float4* __restrict__ rays, uint32_t n,
                                                   int32_t wox, int32_t woy, int32_t woz, uint32_t max_iters,
-                                                  uint4* __restrict__ out, bool coarse) {
+                                                  uint4* __restrict__ out, bool coarse, uint32_t lanes_log2) {
     if constexpr (kAniso) fill_forward_lut();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31;
+    if (lane >> lanes_log2) return;
+    const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5 << lanes_log2) + lane;
     if (i >= n) return;
     const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
     RayState s;
     ray_start<kGlsl>(s, clip, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, coarse);
     TraceCounters cnt;
     uint32_t k = 0;
-    const bool hit = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, k, max_iters) == kStepHit;
+    const bool hit = dda_steps_mode<false, kGlsl, true>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, k,
+                                                                max_iters) == kStepHit;
     out[i] = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, k, __float_as_uint(b.z));
 }
 
@@ -123,7 +143,7 @@ __global__ void __maxnreg__(48) cast_persistent_kernel(const __grid_constant__ D
             const uint32_t kmax = min(inner, max_iters - iter);
             uint32_t k = 0;
             // GLSL variants (rayCastCoarse, anisotropic LODs) are uniform over the launch
-            const uint32_t st = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, iter, k,
+            const uint32_t st = dda_steps_mode<false, kGlsl, true>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, iter, k,
                                                              kmax);
             iter += k;
             if (st != kStepContinue || iter >= max_iters) {
@@ -145,24 +165,25 @@ vrt_status check_camera(const vrt_camera* cam) {
 
 vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters, vrt_hit* hits,
                          cudaStream_t stream) {
-    dim3 block(8, 8);
-    dim3 grid((cam->width + 7) / 8, (cam->height + 7) / 8);
+    const uint32_t ll = thin_lanes_log2((uint64_t)cam->width * cam->height, kThinFrameWarps), wl = (ll + 1) / 2;
+    const uint32_t tw = 1u << wl, th = 2u << (ll - wl);  // pixels of a block
+    const dim3 grid((cam->width + tw - 1) / tw, (cam->height + th - 1) / th);
     L2Window l2;
     vrt_status st = l2.enter(w, stream);
     if (st != VRT_OK) return st;
     const DevWorld dw = w->dev();
     const float* o = cam->origin;
     const ClipBox clip = clip_box(dw, cam->world_origin);
-    render_view_kernel<<<grid, block, 0, stream>>>(dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]),
-                                                   eff_iters(max_iters), reinterpret_cast<uint4*>(hits));
+    render_view_kernel<<<grid, 64, 0, stream>>>(dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]), ll,
+                                                eff_iters(max_iters), reinterpret_cast<uint4*>(hits));
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }
 
 // Launch shape of cast_persistent_kernel (also capped at 48 registers, for more warps to hide
 // L2 latency: 40 and 56 measured 301 and 292 us against 286).  On 4.2 M random rays in a
-// 512-voxel world, slices of 8 steps take 268 us, of 12 steps (the best of the step before)
-// 285 us and of 16 steps 291 us.
+// 512-voxel world, slices of 8 steps took 268 us, of 12 steps 285 us and of 16 steps 291 us;
+// with the flat step 248 us.
 constexpr uint32_t kCastThreads = 128, kCastInner = 8, kCastRefill = 28;
 // Below this many rays the thread-per-ray kernel is used (too few rays to fill the
 // persistent grid's lanes twice).
@@ -184,8 +205,10 @@ vrt_status launch_cast(vrt_world* w, const vrt_ray* rays, uint32_t n, const vrt_
     if (st != VRT_OK) return st;
     if (n < kCastPersistentMin) {
         auto kernel = glsl ? (aniso ? cast_kernel<true, true> : cast_kernel<true>) : cast_kernel<false>;
-        kernel<<<(n + 255) / 256, 256, 0, stream>>>(dw, clip, r4, n, p->world_origin[0], p->world_origin[1],
-                                                    p->world_origin[2], iters, o4, coarse);
+        const uint32_t ll = thin_lanes_log2(n, kThinCastWarps), per_block = 8u << ll;
+        kernel<<<(n + per_block - 1) / per_block, 256, 0, stream>>>(dw, clip, r4, n, p->world_origin[0],
+                                                                    p->world_origin[1], p->world_origin[2], iters, o4,
+                                                                    coarse, ll);
     } else {
         auto kernel = glsl ? (aniso ? cast_persistent_kernel<true, true> : cast_persistent_kernel<true>)
                            : cast_persistent_kernel<false>;

@@ -1,6 +1,7 @@
 """Batches without bounces (tile_kernel in batch.cu) against the oracle: tile shapes and
 remainders, cameras in solid, empty, border and outside voxels, near and far world origins,
-sun rays, iteration caps and the three traversal modes.  Every record word is equal."""
+sun rays, iteration caps and the three traversal modes.  Every record word is equal, in the
+12-byte form too."""
 import copy
 
 import numpy as np
@@ -61,5 +62,21 @@ def test_tiles_match_oracle(worlds, mode, cfg):
     hits = with_cfg.run()
     for i in range(len(views)):
         assert np.array_equal(words(with_cfg.view_hits(hits, i)), words(want[i])), i
+    # the kernel's own 12-byte records
+    assert np.array_equal(with_cfg.run_packed().view(np.uint32), v.pack_hits(hits).view(np.uint32))
     assert with_cfg.stats()["rays_cast"] == sum(int((w["tag"] != v.NO_RAY).sum()) for w in want)
     with_cfg.close()
+
+
+@pytest.mark.parametrize("n_views", [1, 2, 9])
+def test_parts_deliver_every_record(worlds, n_views):
+    """Batches of one, a few and several parts (vrt_batch_run cuts them by record count)."""
+    rng = np.random.default_rng(n_views)
+    views = [v.make_view(v.look_at(rng.uniform(0, 96, 3), rng.uniform(0, 96, 3), 70.0, 1280, 720), world=0,
+                         shadow_dir=SUN if i % 2 else None) for i in range(n_views)]
+    b = v.Batch([w for w, _ in worlds], views)
+    hits = b.run()
+    for i in range(n_views):
+        assert np.array_equal(words(b.view_hits(hits, i)), words(oracle_view(worlds[0][1], views[i]))), i
+    assert np.array_equal(b.run_packed().view(np.uint32), v.pack_hits(hits).view(np.uint32))
+    b.close()

@@ -51,20 +51,33 @@ VRT_HD inline ViewStart view_start(const DevWorld& w, const ViewDev& v) {
     return s;
 }
 
+// Store of record i: the 16-byte record, or with kPacked its 12-byte form (vrt_hit_packed).
+template <bool kPacked>
+__device__ __forceinline__ void store_record(uint4* __restrict__ out, uint64_t i, uint4 r) {
+    if constexpr (kPacked) {
+        uint32_t* o = reinterpret_cast<uint32_t*>(out) + 3 * i;
+        o[0] = r.x;
+        o[1] = r.w == VRT_NO_RAY ? (r.y & 0xFFFF00FFu) | (VRT_PACKED_NO_RAY << 8) : r.y;
+        o[2] = r.z;
+    } else {
+        out[i] = r;
+    }
+}
+
 // One pixel's whole path: the primary ray, then its sun ray or bounces, or with kFull the GPU
 // renderer's path (VoxelRender.comp:27-93); returns the rays traced.  One loop over the rays,
 // so that the step loop is compiled once.
-template <bool kGlsl, bool kAniso, bool kBounces>
+template <bool kGlsl, bool kAniso, bool kBounces, bool kPacked>
 __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld& w, const ViewStart& vs, uint32_t px,
                                                 uint32_t py, uint4* __restrict__ out) {
     const uint32_t pixel = py * v.width + px, last = v.last_kind();
-    uint4* o = out + v.out_base + pixel;
+    uint64_t o = v.out_base + pixel;
     float dx, dy, dz;
     camera_ray(v.d0, v.du, v.dv, px, py, dx, dy, dz);
     if (!kGlsl && !kBounces && vs.mask == kStartSolid && last == 0) {
         // the camera stands in a solid voxel: every ray hits it on iteration 0 at t = 0, face X
         const uint32_t x = vs.voxel[0] - kVoxelBias, y = vs.voxel[1] - kVoxelBias, z = vs.voxel[2] - kVoxelBias;
-        *o = make_uint4(x | y << 11 | z << 21, (dx < 0.0f ? 1u : 0u) | vs.material << 8, 0u, pixel);
+        store_record<kPacked>(out, o, make_uint4(x | y << 11 | z << 21, (dx < 0.0f ? 1u : 0u) | vs.material << 8, 0u, pixel));
         return 1;
     }
     const int32_t wox = v.wo[0], woy = v.wo[1], woz = v.wo[2];
@@ -88,14 +101,14 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
         const uint32_t iters = coarse ? min(v.max_iters, kCoarseMaxIters) : v.max_iters;
         const uint32_t st = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, i, iters);
         const bool hit = st == kStepHit;
-        *o = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, i, pixel);
+        store_record<kPacked>(out, o, pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, i, pixel));
         if (k == last) return k + 1;
         // the path goes on after a hit, and the whole path after a sun ray, hit or miss
         const bool go = hit || (full && full_is_sun(k));
         const size_t plane = (size_t)v.width * v.height;
         if (!go) {
             const uint32_t n = k + 1;
-            for (; k < last; k++) *(o += plane) = no_ray_hit();
+            for (; k < last; k++) store_record<kPacked>(out, o += plane, no_ray_hit());
             return n;
         }
         k++;
@@ -130,7 +143,7 @@ __global__ void __launch_bounds__(64) view_path_kernel(const __grid_constant__ D
     const uint32_t px = blockIdx.x * 8 + threadIdx.x;
     const uint32_t py = blockIdx.y * 8 + threadIdx.y;
     if (px >= v.width || py >= v.height) return;
-    trace_pixel<kGlsl, kAniso, true>(v, w, vs, px, py, out);
+    trace_pixel<kGlsl, kAniso, true, false>(v, w, vs, px, py, out);
 }
 
 // View-table loads: read-only through the non-coherent path, or at L2 (coherent with
@@ -633,7 +646,8 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
 // 44 M rays over 154 views of 16 mixed worlds: 701 us against 1109 us;
 // six 1080p terrain views with sun rays: 754 us against 1035 us.  72 registers, 28 warps a
 // SM: 64 spill (713 and 767 us), 56 more so (759 and 803 us), 80 leave 24 warps (735 and 788 us).
-template <bool kGlsl, bool kAniso>
+// kPacked: the records are stored in the 12-byte form.
+template <bool kGlsl, bool kAniso, bool kPacked>
 __global__ void __maxnreg__(72) tile_kernel(BatchParams p) {
     if constexpr (kAniso) fill_forward_lut();
     // what the warp's view needs at a ray's start (warps_per_block <= 16)
@@ -715,7 +729,7 @@ __global__ void __maxnreg__(72) tile_kernel(BatchParams p) {
         uint32_t y = ty * tile_h;
         for (;;) {
             const uint32_t px = (tx << p.tile_w_log2) + kx, py = y + ky;
-            if (px < v.width && py < v.height) rays += trace_pixel<kGlsl, kAniso, false>(v, w, sw.start, px, py, p.out);
+            if (px < v.width && py < v.height) rays += trace_pixel<kGlsl, kAniso, false, kPacked>(v, w, sw.start, px, py, p.out);
             __syncwarp();
             y += rows;
             if ((y & (tile_h - 1u)) == 0) {  // the tile is done
@@ -937,9 +951,13 @@ PersistentFn persistent_fn_mode(bool glsl, bool aniso) {
     if (glsl) return persistent_kernel<kCount, true, kResident, false, kFull>;
     return persistent_kernel<kCount, false, kResident, false, kFull>;
 }
+template <bool kPacked>
+PersistentFn tile_fn(bool glsl, bool aniso) {
+    return glsl ? (aniso ? tile_kernel<true, true, kPacked> : tile_kernel<true, false, kPacked>)
+                : tile_kernel<false, false, kPacked>;
+}
 PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, bool full, bool tiles) {
-    if (tiles && !count && !resident)
-        return glsl ? (aniso ? tile_kernel<true, true> : tile_kernel<true, false>) : tile_kernel<false, false>;
+    if (tiles && !count && !resident) return tile_fn<false>(glsl, aniso);
     if (resident) return full ? persistent_fn_mode<false, true, true>(glsl, aniso)
                               : persistent_fn_mode<false, true, false>(glsl, aniso);
     if (count) return full ? persistent_fn_mode<true, false, true>(glsl, aniso)
@@ -1005,9 +1023,10 @@ vrt_status launch_resident(const BatchParams& p, int blocks, int threads, cudaSt
 }
 
 vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool count, cudaStream_t stream,
-                             bool reset_counters) {
-    VRT_CUDA(cudaMemsetAsync(p.queue, 0, reset_counters ? 64 : 4, stream));
-    const PersistentFn fn = persistent_fn(count, p.glsl != 0, p.aniso != 0, false, p.full != 0, p.tiles != 0);
+                             size_t zero_bytes) {
+    if (zero_bytes) VRT_CUDA(cudaMemsetAsync(p.queue, 0, zero_bytes, stream));
+    const PersistentFn fn = p.tiles && p.packed ? tile_fn<true>(p.glsl != 0, p.aniso != 0)
+                                                : persistent_fn(count, p.glsl != 0, p.aniso != 0, false, p.full != 0, p.tiles != 0);
     fn<<<blocks, threads, pend_bytes(p, threads), stream>>>(p);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
@@ -1015,8 +1034,8 @@ vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool
 
 namespace {
 
-// vrt_batch_run_packed: records [0, n) of one part as 12-byte vrt_hit_packed, one thread per
-// record (three 4-byte stores: a warp's stores cover 384 contiguous bytes); the 16-byte
+// vrt_batch_run_packed of views with bounces (tile_kernel stores this form itself): records
+// [0, n) of one part as 12-byte vrt_hit_packed, one thread per record (three 4-byte stores: a warp's stores cover 384 contiguous bytes); the 16-byte
 // records are read once, so they are loaded as streaming
 static_assert(sizeof(vrt_hit_packed) == 12 && sizeof(vrt_hit) == 16, "record sizes");
 __global__ void __launch_bounds__(256)
@@ -1035,6 +1054,10 @@ __global__ void __launch_bounds__(256)
 
 using namespace vrt;
 
+// Device block of a batch's queue counter and launch counters, and the parts of vrt_batch_run.
+constexpr size_t kQueueBytes = 64;
+constexpr uint64_t kMaxParts = 32;
+
 struct vrt_batch {
     int device = 0;
     std::vector<vrt_world*> worlds;
@@ -1046,7 +1069,7 @@ struct vrt_batch {
     DevWorld* d_worlds = nullptr;
     ViewDev* d_views = nullptr;
     uint32_t* d_chunk_base = nullptr;
-    uint32_t* d_queue = nullptr;  // queue counter followed by 4 u64 counters (16-byte aligned)
+    uint32_t* d_queue = nullptr;  // queue counter, 4 u64 counters at byte 16, part counters at byte 64
     unsigned long long* d_counters = nullptr;
     cudaStream_t last_stream = nullptr;
     DevBuf d_out;     // record buffer of vrt_batch_run
@@ -1173,7 +1196,7 @@ vrt_status vrt_batch_create(vrt_world* const* worlds, uint32_t n_worlds, const v
     cudaError_t e = cudaMalloc(&b->d_worlds, sizeof(DevWorld) * n_worlds);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_views, sizeof(ViewDev) * n_views);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_chunk_base, sizeof(uint32_t) * (n_views + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_queue, 64);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_queue, kQueueBytes + kMaxParts * sizeof(uint32_t));
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_views, b->plan.views.data(), sizeof(ViewDev) * n_views, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
@@ -1320,23 +1343,34 @@ vrt_status vrt_batch_launch_per_view(vrt_batch* b, vrt_hit* hits, void* stream_)
 namespace {
 
 // vrt_batch_run and vrt_batch_run_packed: trace, (pack,) and copy to `host` part by part.
+uint64_t part_count(uint64_t records) {
+    uint64_t n = 1;
+    while (n < kMaxParts && (n + 1) * (n + 1) << 18 <= records) n++;
+    return n;
+}
+
 vrt_status run_parts(vrt_batch* b, void* host, bool packed, cudaStream_t stream) {
     DeviceScope ds;
     VRT_CUDA(ds.enter(b->device));
     const LaunchPlan& plan = b->plan;
     const size_t nv = plan.views.size();
-    VRT_CUDA(b->d_out.reserve(plan.records * sizeof(vrt_hit)));
+    const bool direct = packed && plan.tiles;  // the kernel stores packed records itself
+    if (!direct) VRT_CUDA(b->d_out.reserve(plan.records * sizeof(vrt_hit)));
     if (packed) VRT_CUDA(b->d_packed.reserve(plan.records * sizeof(vrt_hit_packed)));
     vrt_status st = refresh_worlds(b, stream);
     if (st != VRT_OK) return st;
     // Views are split into parts of about equal record count, at view boundaries.
     // All parts are launched first, one after another on `stream`; the copy of a
     // part's records (one contiguous range) waits for that part only, so the host
-    // transfer of finished parts overlaps the traversal of the later ones.
-    constexpr uint64_t kParts = 32;  // measured on GB300: 8 parts 30.99 ms, 32 parts 30.02, 128 parts 35.30
+    // transfer of finished parts overlaps the traversal of the later ones.  More parts start
+    // the copies earlier, but each launch ramps up and runs out (20-100 us): the best number
+    // grows with the root of the batch.  Times on GB300 for views of mixed worlds, 12-byte
+    // records, by parts: 3.0 M records 287 us (1), 249 (4); 9.3 M 655 (5), 662 (11), 695 (23);
+    // 24.6 M 1705 (7), 1760 (15), 2088 (32); 353 M as ever 32.
+    const uint64_t want = part_count(plan.records);
     std::vector<size_t> cut{0};
     for (size_t i = 1; i < nv; i++)
-        if (plan.views[i].out_base * kParts >= plan.records * cut.size()) cut.push_back(i);
+        if (plan.views[i].out_base * want >= plan.records * cut.size()) cut.push_back(i);
     cut.push_back(nv);
     const size_t parts = cut.size() - 1;
     if (!b->copy_stream) {
@@ -1353,18 +1387,21 @@ vrt_status run_parts(vrt_batch* b, void* host, bool packed, cudaStream_t stream)
     uint32_t* d_pack = (uint32_t*)b->d_packed.ptr;
     L2Window l2;
     if ((st = l2.enter(b->l2_world, stream)) != VRT_OK) return st;
+    VRT_CUDA(cudaMemsetAsync(b->d_queue, 0, kQueueBytes + parts * sizeof(uint32_t), stream));
     for (size_t k = 0; k < parts; k++) {
         const size_t a = cut[k], e = cut[k + 1];
         BatchParams p = make_params(plan, b->d_worlds, b->d_views, b->d_chunk_base, b->d_queue,
-                                    (vrt_hit*)b->d_out.ptr);
+                                    (vrt_hit*)(direct ? b->d_packed.ptr : b->d_out.ptr));
+        p.queue = b->d_queue + kQueueBytes / sizeof(uint32_t) + k;
+        p.packed = direct ? 1u : 0u;
         p.views = b->d_views + a;
         p.chunk_base = b->d_chunk_base + a;
         p.n_views = (uint32_t)(e - a);
         p.chunk_first = plan.chunk_base[a];
         p.total_chunks = plan.chunk_base[e] - plan.chunk_base[a];
-        if ((st = launch_persistent(p, b->blocks, b->threads, false, stream, k == 0)) != VRT_OK) return st;
+        if ((st = launch_persistent(p, b->blocks, b->threads, false, stream, 0)) != VRT_OK) return st;
         const uint64_t r0 = first_record(a), n = first_record(e) - r0;
-        if (packed && n) {
+        if (packed && !direct && n) {
             const uint32_t blocks = (uint32_t)std::min<uint64_t>((n + 255) / 256, 4096);
             pack_records_kernel<<<blocks, 256, 0, stream>>>(d_full + r0, d_pack + 3 * r0, n);
             VRT_CUDA(cudaGetLastError());

@@ -63,6 +63,7 @@ struct BatchParams {
     uint32_t glsl;  // traversal mode of every view (VRT_VIEW_GLSL)
     uint32_t aniso;  // ... with anisotropic LODs (VRT_VIEW_GLSL_ANISO)
     uint32_t tiles;  // no view has bounces: tile_kernel traces the launch
+    uint32_t packed; // (tiles) records are stored in the 12-byte form
     uint32_t full;   // some view traces the GPU renderer's whole path (sun rays among bounces)
     // resident launches (request server): views are published while the kernel runs
     unsigned long long* mailbox;  // host-mapped: published chunks | published views << 32 | closed << 63
@@ -137,10 +138,10 @@ vrt_status persistent_grid(int device, const vrt_batch_config& cfg, bool count, 
                            bool full, bool tiles, int& blocks, int& threads);
 BatchParams make_params(const LaunchPlan& plan, const DevWorld* worlds, const ViewDev* views,
                         const uint32_t* chunk_base, uint32_t* queue, vrt_hit* out);
-// Queue reset (the tile counter, and with reset_counters the launch counters: 64
-// bytes at params.queue) + persistent kernel launch.
+// Reset of the tile counter and the launch counters (64 bytes at params.queue; 0: the caller
+// has reset them) + launch of the kernel.
 vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool count, cudaStream_t stream,
-                             bool reset_counters = true);
+                             size_t zero_bytes = 64);
 // A resident launch: the kernel claims chunks the host publishes through p.mailbox
 // while it runs, and exits once the mailbox is closed and its work is done.  The
 // caller zeroes the block at p.queue (claim counter and launch counters in the first

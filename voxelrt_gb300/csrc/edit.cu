@@ -10,23 +10,24 @@
 //   host (geometry only, no device state): the sectors the edits' boxes touch, per
 //       sector the bricks inside a box (`visit`) and the bricks a fill sphere reaches
 //       (`create`), and the sector groups whose brick-table entries follow them;
-//   1. relayout_kernel<true>: sectors gaining bricks move to a fresh range from the
-//      device's bump allocator (alloc.cu) and zero-fill the new bricks;
-//   2. edit_bricks_kernel: one warp per visited allocated brick applies every edit of
-//      the batch in order, derives the 8 cell masks by ballot, stores the voxel codes
-//      and flags the brick when it is empty;
-//   3. relayout_kernel<false>: sectors with emptied bricks drop them in place;
-//   4. the group masks and brick-table entries of the touched groups.
+//   1. edit_sectors_kernel: a cluster of blocks per touched sector, a warp per brick: applies
+//      every edit of the batch in order to the visited bricks, drops the emptied ones, moves the
+//      sector to a fresh range from the device's bump allocator (alloc.cu) when it gained
+//      bricks or packs it in place when it lost some, and derives the cell masks and voxel
+//      codes of what it writes;
+//   2. the group masks and brick-table entries of the touched groups (world.cu).
 // The final state equals applying the edits one by one.  The call only enqueues this
-// work on the stream (one upload of the batch from pinned memory and the kernels); the
+// work on the stream (one upload of the batch from pinned memory and two kernels); the
 // host reads nothing back, except when its bound of the bump pointer says the pool may
 // be full, and then it compacts the pool first (alloc.cu).
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "brick_codes.cuh"
@@ -35,7 +36,7 @@
 namespace vrt {
 namespace {
 
-struct EditDev {
+struct alignas(16) EditDev {
     int32_t cx, cy, cz;
     int32_t r2;
     int32_t lo[3], hi[3];  // brick bounding box (inclusive)
@@ -51,134 +52,128 @@ struct EditSector {
 static_assert(sizeof(EditSector) == 24, "edit sector records are 24 bytes");
 
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
-constexpr int kEditWarps = 8;
 
-// Copy brick slot src to slot dst (payload, voxel codes, cell masks: 68 16-byte words),
-// or zero-fill dst (an empty brick) when src is kNoSlot; threads [0, n) share the words.
-__device__ __forceinline__ void move_brick(uint8_t* __restrict__ payload, uint4* __restrict__ codes,
-                                           uint64_t* __restrict__ cells, uint32_t src, uint32_t dst, uint32_t t,
-                                           uint32_t n) {
-    for (uint32_t k = t; k < 68; k += n) {
-        if (k < 32) {
-            uint4* d = reinterpret_cast<uint4*>(payload + (size_t)dst * 512) + k;
-            *d = src == kNoSlot ? make_uint4(0, 0, 0, 0)
-                                : reinterpret_cast<const uint4*>(payload + (size_t)src * 512)[k];
-        } else if (k < 64) {
-            codes[(size_t)dst * 32 + (k - 32)] =
-                src == kNoSlot ? empty_brick_codes() : codes[(size_t)src * 32 + (k - 32)];
-        } else {
-            uint4* d = reinterpret_cast<uint4*>(cells + (size_t)dst * 8) + (k - 64);
-            *d = src == kNoSlot ? make_uint4(0, 0, 0, 0)
-                                : reinterpret_cast<const uint4*>(cells + (size_t)src * 8)[k - 64];
-        }
-    }
-}
-
-// Relayout of the touched sectors whose mask the batch changes, one block per touched
-// sector.  kGrow: new mask = old | create; the sector takes popcount(new) slots at the
-// bump pointer, its bricks move there, created bricks are zero-filled, and its old
-// range is left as garbage.  Otherwise: new mask = old & ~emptied; the remaining bricks
-// move down in place in ascending order: every brick's destination lies at or below its
-// source, and a brick's source lies above the destinations of the bricks before it, so
-// moving one brick at a time in that order never overwrites a brick not yet moved.
-template <bool kGrow>
-__global__ void __launch_bounds__(96)
-    relayout_kernel(const EditSector* __restrict__ ts, uint32_t m, const unsigned long long* __restrict__ emptied,
-                    SectorRec* __restrict__ sectors, DevAlloc* __restrict__ alloc, uint8_t* __restrict__ payload,
-                    uint4* __restrict__ codes, uint64_t* __restrict__ cells) {
-    const uint32_t i = blockIdx.x, t = threadIdx.x;
-    if (i >= m) return;
-    const uint32_t s = ts[i].sector;
-    const SectorRec rec = sectors[s];
-    const uint64_t old = (uint64_t)rec.mask_hi << 32 | rec.mask_lo;
-    const uint64_t nm = kGrow ? (old | ts[i].create) : (old & ~emptied[i]);
-    if (nm == old) return;  // the whole block
-    __shared__ uint32_t s_dst;
-    if (t == 0) {
-        const uint32_t n_new = (uint32_t)__popcll(nm), n_old = (uint32_t)__popcll(old);
-        if (kGrow) {
-            const uint32_t b = atomicAdd(&alloc->top, n_new);
-            if ((uint64_t)b + n_new > alloc->cap) {
-                atomicExch(&alloc->overflow, 1u);  // never, while the host's bound of the pointer holds
-                s_dst = kNoSlot;
-            } else {
-                atomicAdd(&alloc->live, n_new - n_old);
-                s_dst = b;
-            }
-        } else {
-            atomicSub(&alloc->live, n_old - n_new);
-            s_dst = rec.base;
-        }
-    }
-    __syncthreads();
-    const uint32_t dst_base = s_dst;
-    if (dst_base == kNoSlot) return;
-    uint32_t k = 0;
-    for (uint64_t r = nm; r; r &= r - 1, k++) {
-        const uint64_t bit = r & (~r + 1);
-        const uint32_t src = (old & bit) ? rec.base + (uint32_t)__popcll(old & (bit - 1)) : kNoSlot;
-        if (src == dst_base + k) continue;
-        move_brick(payload, codes, cells, src, dst_base + k, t, blockDim.x);
-        __syncthreads();
-    }
-    if (t == 0) {
-        SectorRec out = rec;
-        out.mask_lo = (uint32_t)nm;
-        out.mask_hi = (uint32_t)(nm >> 32);
-        out.base = nm ? dst_base : 0;
-        sectors[s] = out;
-    }
-}
-
-// One warp per (touched sector i, brick b): a visited brick that is allocated takes every
-// edit of the batch in order; its cell masks and voxel codes are re-derived, and an
-// emptied brick is flagged in emptied[i].
-__global__ void __launch_bounds__(kEditWarps * 32)
-    edit_bricks_kernel(const EditSector* __restrict__ ts, uint32_t m, const EditDev* __restrict__ edits,
-                       uint32_t n_edits, const SectorRec* __restrict__ sectors, uint32_t sx, uint32_t sz,
-                       uint8_t* __restrict__ payload, uint4* __restrict__ codes, uint64_t* __restrict__ cell_masks,
-                       unsigned long long* __restrict__ emptied) {
+// A cluster of 8 blocks per touched sector, a warp for each of its up to 64 bricks (k-th set
+// bit of old | create).  Every brick is read before any is written, so a sector that loses
+// bricks is packed in place.  A sector that gains some takes popcount(final mask) slots at the
+// bump pointer and leaves its old range as garbage.
+// Bound by latency: a stroke touches some twenty sectors, and a brick is a load, a few dozen
+// instructions per edit that reaches it and a store.  In one kernel the bricks stay in
+// registers between the edits and the layout; as three (grow, edit, shrink, the layouts one
+// brick after another with a barrier each) a stroke of 24 spheres of radius 14 took 23 + 9 + 13 us,
+// and with the frame after it 107 us, now 50.  8 blocks of 8 warps: 200 spheres of radius 30 over
+// the same sectors 520 us, 4 of 16 557 us, 2 of 32 594 us.
+constexpr uint32_t kEditWarps = 8, kEditCluster = 8;
+__global__ void __cluster_dims__(kEditCluster, 1, 1) __launch_bounds__(kEditWarps * 32)
+    edit_sectors_kernel(const EditSector* __restrict__ ts, const EditDev* __restrict__ edits, uint32_t n_edits,
+                        SectorRec* __restrict__ sectors, uint32_t sx, uint32_t sz, DevAlloc* __restrict__ alloc,
+                        uint8_t* __restrict__ payload, uint4* __restrict__ codes, uint64_t* __restrict__ cell_masks) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
     __shared__ __align__(16) uint8_t sb[kEditWarps][512];
-    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint32_t gw = blockIdx.x * kEditWarps + wib;
-    const uint32_t i = gw >> 6, b = gw & 63u;
-    if (i >= m) return;  // whole warps
-    const unsigned long long bit = 1ull << b;
-    if (!(ts[i].visit & bit)) return;
-    const uint32_t s = ts[i].sector;
+    __shared__ uint32_t s_emptied[2], s_base;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5, rank = cluster.block_rank();
+    const EditSector es = ts[blockIdx.x / kEditCluster];
+    const uint32_t s = es.sector;
     const SectorRec rec = sectors[s];
-    const uint64_t mask = (uint64_t)rec.mask_hi << 32 | rec.mask_lo;
-    if (!(mask & bit)) return;
-    const uint32_t slot = rec.base + (uint32_t)__popcll(mask & (bit - 1));
-    const uint32_t bx = (s % sx) * 4 + (b & 3u), bz = ((s / sx) % sz) * 4 + ((b >> 2) & 3u),
-                   by = (s / (sx * sz)) * 4 + (b >> 4);
-    uint4 v = reinterpret_cast<const uint4*>(payload + (size_t)slot * 512)[lane];
-    uint8_t* bytes = reinterpret_cast<uint8_t*>(&v);
-    // lane holds voxels 16*lane .. 16*lane+15: y = lane>>2, z = 2*(lane&3) + (j>>3), x = j&7
-    const int32_t y = (int32_t)(by * 8 + (lane >> 2));
-    const int32_t z0 = (int32_t)(bz * 8 + 2 * (lane & 3));
-    const int32_t x0 = (int32_t)(bx * 8);
-    for (uint32_t e = 0; e < n_edits; e++) {
-        const EditDev ed = edits[e];
-        if ((int32_t)bx < ed.lo[0] || (int32_t)bx > ed.hi[0] || (int32_t)by < ed.lo[1] || (int32_t)by > ed.hi[1] ||
-            (int32_t)bz < ed.lo[2] || (int32_t)bz > ed.hi[2])
-            continue;
-        const int32_t dy = y - ed.cy;
-#pragma unroll
-        for (int j = 0; j < 16; j++) {
-            const int32_t dx = x0 + (j & 7) - ed.cx, dz = z0 + (j >> 3) - ed.cz;
-            if (dx * dx + dy * dy + dz * dz > ed.r2) continue;
-            if (ed.replace && bytes[j] == 0) continue;
-            bytes[j] = (uint8_t)ed.material;
-        }
+    const uint64_t old = (uint64_t)rec.mask_hi << 32 | rec.mask_lo, nm = old | es.create;
+    if (!(nm & es.visit)) return;  // the whole cluster
+    if (threadIdx.x < 2) s_emptied[threadIdx.x] = 0;
+    __syncthreads();
+    // this warp's brick
+    const uint32_t k = rank * kEditWarps + wib;
+    const bool mine = k < (uint32_t)__popcll(nm);
+    uint32_t b = 0;
+    if (mine) {  // the k-th set bit of nm: the one set bit with k set bits below it
+        const uint32_t lo = (uint32_t)nm, nlo = (uint32_t)__popc(lo), half = k < nlo ? lo : (uint32_t)(nm >> 32);
+        const uint32_t kk = k < nlo ? k : k - nlo;
+        b = (uint32_t)__ffs(__ballot_sync(0xffffffffu, ((half >> lane) & 1u) &&
+                                                           (uint32_t)__popc(half & ((1u << lane) - 1u)) == kk)) - 1u;
+        if (k >= nlo) b += 32u;
     }
-    reinterpret_cast<uint4*>(payload + (size_t)slot * 512)[lane] = v;
-    reinterpret_cast<uint4*>(sb[wib])[lane] = v;
-    __syncwarp();
-    const uint64_t cells = warp_cell_mask(sb[wib], lane);
-    codes[(size_t)slot * 32 + lane] = warp_voxel_codes(sb[wib], cells, lane);
-    if (lane < 8) cell_masks[(size_t)slot * 8 + lane] = cells;
-    if (!__any_sync(0xffffffffu, cells != 0) && lane == 0) atomicOr(emptied + i, bit);
+    const uint64_t bit = 1ull << b;
+    const bool had = mine && (old & bit), visited = mine && (es.visit & bit);
+    const uint32_t src = rec.base + (uint32_t)__popcll(old & (bit - 1));
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (visited) {
+        if (had) v = reinterpret_cast<const uint4*>(payload + (size_t)src * 512)[lane];
+        const int32_t bx = (int32_t)((s % sx) * 4 + (b & 3u)), bz = (int32_t)(((s / sx) % sz) * 4 + ((b >> 2) & 3u)),
+                      by = (int32_t)((s / (sx * sz)) * 4 + (b >> 4));
+        uint8_t* bytes = reinterpret_cast<uint8_t*>(&v);
+        // lane holds voxels 16*lane .. 16*lane+15: y = lane>>2, z = 2*(lane&3) + (j>>3), x = j&7
+        const int32_t y = by * 8 + (int32_t)(lane >> 2), z0 = bz * 8 + 2 * (int32_t)(lane & 3), x0 = bx * 8;
+        for (uint32_t e0 = 0; e0 < n_edits; e0 += 32) {
+            // 32 edits at a time: each lane tests one against the brick
+            EditDev ed{};
+            const bool valid = e0 + lane < n_edits;
+            if (valid) ed = edits[e0 + lane];
+            uint32_t todo = __ballot_sync(0xffffffffu, valid && bx >= ed.lo[0] && bx <= ed.hi[0] && by >= ed.lo[1] &&
+                                                           by <= ed.hi[1] && bz >= ed.lo[2] && bz <= ed.hi[2]);
+            for (; todo; todo &= todo - 1) {
+                const int l = __ffs(todo) - 1;
+                const int32_t dy = y - __shfl_sync(0xffffffffu, ed.cy, l), dz0 = z0 - __shfl_sync(0xffffffffu, ed.cz, l),
+                              dx0 = x0 - __shfl_sync(0xffffffffu, ed.cx, l);
+                const int32_t r2 = __shfl_sync(0xffffffffu, ed.r2, l);
+                const uint32_t paint = __shfl_sync(0xffffffffu, ed.material | ed.replace << 8, l);
+                const int32_t left[2] = {r2 - dy * dy - dz0 * dz0, r2 - dy * dy - (dz0 + 1) * (dz0 + 1)};
+                const bool replace = paint >> 8 != 0;
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const int32_t dx = dx0 + (j & 7);
+                    if (dx * dx > left[j >> 3]) continue;
+                    if (replace && bytes[j] == 0) continue;
+                    bytes[j] = (uint8_t)paint;
+                }
+            }
+        }
+        if (!__any_sync(0xffffffffu, (v.x | v.y | v.z | v.w) != 0) && lane == 0)
+            atomicOr(&s_emptied[b >> 5], 1u << (b & 31));
+    }
+    cluster.sync();
+    uint64_t emptied = 0;
+    for (uint32_t r = 0; r < kEditCluster; r++) {
+        const uint32_t* e = cluster.map_shared_rank(s_emptied, r);
+        emptied |= (uint64_t)e[0] | (uint64_t)e[1] << 32;
+    }
+    const uint64_t fm = nm & ~emptied;
+    uint32_t base = rec.base;
+    if (fm != old) {  // a new layout
+        if (rank == 0 && threadIdx.x == 0) {
+            const uint32_t n_new = (uint32_t)__popcll(fm), n_old = (uint32_t)__popcll(old);
+            if (fm & ~old) {
+                base = atomicAdd(&alloc->top, n_new);
+                if ((uint64_t)base + n_new > alloc->cap) {
+                    atomicExch(&alloc->overflow, 1u);  // never, while the host's bound of the pointer holds
+                    base = kNoSlot;
+                }
+            }
+            if (base != kNoSlot) {
+                atomicAdd(&alloc->live, n_new - n_old);
+                SectorRec out = rec;
+                out.mask_lo = (uint32_t)fm;
+                out.mask_hi = (uint32_t)(fm >> 32);
+                out.base = fm ? base : 0;
+                sectors[s] = out;
+            }
+            s_base = base;
+        }
+        // bricks no edit visits that change slots: read before anything is written
+        if (mine && !visited) v = reinterpret_cast<const uint4*>(payload + (size_t)src * 512)[lane];
+        cluster.sync();
+        base = *cluster.map_shared_rank(&s_base, 0);
+    }
+    // no block may leave while another reads its shared memory: said here, waited for at the end
+    auto token = cluster.barrier_arrive();
+    const uint32_t dst = base + (uint32_t)__popcll(fm & (bit - 1));
+    if (mine && (fm & bit) && base != kNoSlot && (visited || dst != src)) {
+        reinterpret_cast<uint4*>(payload + (size_t)dst * 512)[lane] = v;
+        reinterpret_cast<uint4*>(sb[wib])[lane] = v;
+        __syncwarp();
+        const uint64_t cells = warp_cell_mask(sb[wib], lane);
+        codes[(size_t)dst * 32 + lane] = warp_voxel_codes(sb[wib], cells, lane);
+        if (lane < 8) cell_masks[(size_t)dst * 8 + lane] = cells;
+    }
+    cluster.barrier_wait(std::move(token));
 }
 
 // Closest voxel of the brick to the center lies within the sphere.
@@ -308,20 +303,12 @@ extern "C" vrt_status vrt_world_edit(vrt_world* w, const vrt_edit* edits, uint32
     std::memcpy(h + soff, secs.data(), sb);
     std::memcpy(h + goff, groups.data(), groups.size() * sizeof(uint32_t));
     VRT_CUDA(w->d_edit.reserve(total, true));
-    VRT_CUDA(w->d_gc.reserve((size_t)m * 8, true));
     uint8_t* d = (uint8_t*)w->d_edit.ptr;
     VRT_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, stream));
     VRT_CUDA(stage.release(stream));
-    VRT_CUDA(cudaMemsetAsync(w->d_gc.ptr, 0, (size_t)m * 8, stream));
     const EditSector* d_secs = (const EditSector*)(d + soff);
-    auto* d_emptied = (unsigned long long*)w->d_gc.ptr;
-    if (growing)
-        relayout_kernel<true><<<m, 96, 0, stream>>>(d_secs, m, d_emptied, w->d_sectors, w->d_alloc, w->d_payload,
-                                                   w->d_codes, w->d_cells);
-    edit_bricks_kernel<<<(m * 64 + kEditWarps - 1) / kEditWarps, kEditWarps * 32, 0, stream>>>(
-        d_secs, m, (const EditDev*)d, n, w->d_sectors, w->sx, w->sz, w->d_payload, w->d_codes, w->d_cells, d_emptied);
-    relayout_kernel<false><<<m, 96, 0, stream>>>(d_secs, m, d_emptied, w->d_sectors, w->d_alloc, w->d_payload,
-                                                w->d_codes, w->d_cells);
+    edit_sectors_kernel<<<m * kEditCluster, kEditWarps * 32, 0, stream>>>(
+        d_secs, (const EditDev*)d, n, w->d_sectors, w->sx, w->sz, w->d_alloc, w->d_payload, w->d_codes, w->d_cells);
     VRT_CUDA(cudaGetLastError());
     if ((st = rebuild_table_groups(w, (const uint32_t*)(d + goff), (uint32_t)groups.size(), stream)) != VRT_OK)
         return st;

@@ -126,7 +126,6 @@ struct vrt_world {
     vrt::HostStage edit_stage[4];  // pinned uploads of the last edit batches, used in turn
     uint32_t edit_stage_next = 0;
     vrt::DevBuf d_edit;         // the edit batch on the device
-    vrt::DevBuf d_gc;           // per touched sector: bricks an edit emptied
     cudaEvent_t edited = nullptr;  // recorded behind the last device edit
     bool host_stale = false;    // slots / arena / h_table predate device edits
     uint64_t top_bound = 0;     // upper bound of d_alloc->top without reading it

@@ -55,11 +55,24 @@ __device__ __forceinline__ uint4 warp_voxel_codes(const uint8_t* sb, uint64_t ce
     return make_uint4(word[0], word[1], word[2], word[3]);
 }
 
-// Codes of an all-empty brick: every cell mask is 0, so every voxel skips 2 levels
-// (mask 3 in every byte).
-constexpr uint32_t kEmptyCodeWord = 0x03030303u;
-__device__ __forceinline__ uint4 empty_brick_codes() {
-    return make_uint4(kEmptyCodeWord, kEmptyCodeWord, kEmptyCodeWord, kEmptyCodeWord);
+// Position of the k-th set bit (from 0) of a mask with more than k, by a whole warp.
+__device__ __forceinline__ uint32_t warp_nth_bit(uint64_t mask, uint32_t k, uint32_t lane) {
+    const uint32_t lo = (uint32_t)mask, nlo = (uint32_t)__popc(lo);
+    const uint32_t half = k < nlo ? lo : (uint32_t)(mask >> 32), kk = k < nlo ? k : k - nlo;
+    const bool is = ((half >> lane) & 1u) && (uint32_t)__popc(half & ((1u << lane) - 1u)) == kk;
+    return (uint32_t)__ffs(__ballot_sync(0xffffffffu, is)) - 1u + (k < nlo ? 0u : 32u);
+}
+
+// A brick held 16 bytes per lane to its slot, with the cell masks and voxel codes derived
+// from it; sb: the warp's 512 bytes of shared memory.
+__device__ __forceinline__ void store_brick(uint8_t* sb, uint4 v, uint32_t slot, uint32_t lane, uint8_t* payload,
+                                            uint4* codes, uint64_t* cells) {
+    reinterpret_cast<uint4*>(payload + (size_t)slot * 512)[lane] = v;
+    reinterpret_cast<uint4*>(sb)[lane] = v;
+    __syncwarp();
+    const uint64_t m = warp_cell_mask(sb, lane);
+    codes[(size_t)slot * 32 + lane] = warp_voxel_codes(sb, m, lane);
+    if (lane < 8) cells[(size_t)slot * 8 + lane] = m;
 }
 
 }  // namespace vrt

@@ -83,14 +83,7 @@ __global__ void __cluster_dims__(kEditCluster, 1, 1) __launch_bounds__(kEditWarp
     // this warp's brick
     const uint32_t k = rank * kEditWarps + wib;
     const bool mine = k < (uint32_t)__popcll(nm);
-    uint32_t b = 0;
-    if (mine) {  // the k-th set bit of nm: the one set bit with k set bits below it
-        const uint32_t lo = (uint32_t)nm, nlo = (uint32_t)__popc(lo), half = k < nlo ? lo : (uint32_t)(nm >> 32);
-        const uint32_t kk = k < nlo ? k : k - nlo;
-        b = (uint32_t)__ffs(__ballot_sync(0xffffffffu, ((half >> lane) & 1u) &&
-                                                           (uint32_t)__popc(half & ((1u << lane) - 1u)) == kk)) - 1u;
-        if (k >= nlo) b += 32u;
-    }
+    const uint32_t b = mine ? warp_nth_bit(nm, k, lane) : 0u;
     const uint64_t bit = 1ull << b;
     const bool had = mine && (old & bit), visited = mine && (es.visit & bit);
     const uint32_t src = rec.base + (uint32_t)__popcll(old & (bit - 1));
@@ -165,14 +158,8 @@ __global__ void __cluster_dims__(kEditCluster, 1, 1) __launch_bounds__(kEditWarp
     // no block may leave while another reads its shared memory: said here, waited for at the end
     auto token = cluster.barrier_arrive();
     const uint32_t dst = base + (uint32_t)__popcll(fm & (bit - 1));
-    if (mine && (fm & bit) && base != kNoSlot && (visited || dst != src)) {
-        reinterpret_cast<uint4*>(payload + (size_t)dst * 512)[lane] = v;
-        reinterpret_cast<uint4*>(sb[wib])[lane] = v;
-        __syncwarp();
-        const uint64_t cells = warp_cell_mask(sb[wib], lane);
-        codes[(size_t)dst * 32 + lane] = warp_voxel_codes(sb[wib], cells, lane);
-        if (lane < 8) cell_masks[(size_t)dst * 8 + lane] = cells;
-    }
+    if (mine && (fm & bit) && base != kNoSlot && (visited || dst != src))
+        store_brick(sb[wib], v, dst, lane, payload, codes, cell_masks);
     cluster.barrier_wait(std::move(token));
 }
 

@@ -13,7 +13,6 @@
 #include <cstring>
 #include <map>
 #include <string>
-#include <unordered_set>
 #include <vector>
 
 #include "brick_codes.cuh"
@@ -78,91 +77,85 @@ vrt_status setup_l2_window(vrt_world* w) {
 }
 
 // ---------------------------------------------------------------------------
-// Brick operations, one warp per brick.
+// Sector sync.
 
-enum : uint32_t { kOpMove = 0u, kOpUpload = 1u, kOpZero = 2u };
+// One sector of a sync batch, in its new layout: bricks whose bytes were supplied, bricks that
+// keep their content but change slot (gathered to scratch before anything is written), and new
+// bricks without bytes (zero-filled); the other bricks of `mask` stay as they are.
+struct alignas(16) SectorOp {
+    uint64_t mask, dirty, moved, fresh;
+    uint32_t sector, base;   // 0-based slot of the first brick
+    uint32_t first_dirty;    // staged brick of the lowest dirty bit
+    uint32_t first_moved;    // scratch brick of the lowest moved bit
+};
+static_assert(sizeof(SectorOp) == 48, "sector ops are read as three 16-byte words");
 
-struct BrickOp {
-    uint32_t dst;  // 0-based destination slot
-    uint32_t src;  // kind << 30 | index (scratch brick or staged brick)
+// The device allocator's state after a batch (DevAlloc), written by its sync kernel.
+struct AllocState {
+    DevAlloc* alloc;
+    uint32_t top, live, cap;
 };
 
-constexpr int kOpsWarps = 8;
-
-__global__ void gather_bricks_kernel(const uint32_t* __restrict__ src_slots, uint32_t n,
-                                     const uint8_t* __restrict__ payload, const uint4* __restrict__ codes,
-                                     const uint64_t* __restrict__ cells, uint8_t* __restrict__ scratch_payload,
-                                     uint4* __restrict__ scratch_codes, uint64_t* __restrict__ scratch_cells) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t k = warp; k < n; k += nwarps) {
-        const size_t s = src_slots[k];
-        const uint4 v = reinterpret_cast<const uint4*>(payload + s * 512)[lane];
-        reinterpret_cast<uint4*>(scratch_payload + (size_t)k * 512)[lane] = v;
-        scratch_codes[(size_t)k * 32 + lane] = codes[s * 32 + lane];
-        if (lane < 8) scratch_cells[(size_t)k * 8 + lane] = cells[s * 8 + lane];
-    }
+// Payload of the listed slots to scratch, a warp per brick.
+__global__ void __launch_bounds__(256)
+    gather_bricks_kernel(const uint32_t* __restrict__ slots, uint32_t n, const uint8_t* __restrict__ payload,
+                         uint8_t* __restrict__ scratch) {
+    const uint32_t lane = threadIdx.x & 31, k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (k >= n) return;
+    reinterpret_cast<uint4*>(scratch + (size_t)k * 512)[lane] =
+        reinterpret_cast<const uint4*>(payload + (size_t)slots[k] * 512)[lane];
 }
 
-__global__ void __launch_bounds__(kOpsWarps * 32)
-    brick_ops_kernel(const BrickOp* __restrict__ ops, uint32_t n, const uint8_t* __restrict__ stage,
-                     const uint8_t* __restrict__ scratch_payload, const uint4* __restrict__ scratch_codes,
-                     const uint64_t* __restrict__ scratch_cells, uint8_t* __restrict__ payload,
-                     uint4* __restrict__ codes, uint64_t* __restrict__ cells) {
-    __shared__ __align__(16) uint8_t sbrick[kOpsWarps][512];
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t wib = threadIdx.x >> 5;
-    const uint32_t warp = blockIdx.x * kOpsWarps + wib;
-    const uint32_t nwarps = gridDim.x * kOpsWarps;
-    for (uint32_t k = warp; k < n; k += nwarps) {
-        const BrickOp op = ops[k];
-        const uint32_t kind = op.src >> 30, si = op.src & 0x3fffffffu;
-        const size_t d = op.dst;
-        if (kind == kOpMove) {
-            const uint4 v = reinterpret_cast<const uint4*>(scratch_payload + (size_t)si * 512)[lane];
-            reinterpret_cast<uint4*>(payload + d * 512)[lane] = v;
-            codes[d * 32 + lane] = scratch_codes[(size_t)si * 32 + lane];
-            if (lane < 8) cells[d * 8 + lane] = scratch_cells[(size_t)si * 8 + lane];
-        } else if (kind == kOpZero) {
-            reinterpret_cast<uint4*>(payload + d * 512)[lane] = make_uint4(0, 0, 0, 0);
-            codes[d * 32 + lane] = empty_brick_codes();
-            if (lane < 8) cells[d * 8 + lane] = 0;
-        } else {
-            const uint4 v = reinterpret_cast<const uint4*>(stage + (size_t)si * 512)[lane];
-            reinterpret_cast<uint4*>(payload + d * 512)[lane] = v;
-            reinterpret_cast<uint4*>(sbrick[wib])[lane] = v;
-            __syncwarp();
-            const uint64_t m = warp_cell_mask(sbrick[wib], lane);
-            codes[d * 32 + lane] = warp_voxel_codes(sbrick[wib], m, lane);
-            if (lane < 8) cells[d * 8 + lane] = m;
-            __syncwarp();
+// A block per sector op, each of its 16 warps every 16th brick to write (up to 4, loaded
+// before the first is stored): payload, cell masks and voxel codes, then the sector's record.
+// Bound by memory: 512 B in and 1088 B out a brick.  One op per sector, read from the
+// host's pinned list, where a list of 60,000 brick ops took the host longer to build than the
+// copy to upload: 60 k bricks of a 512x256x512 terrain synced and a 640x360 frame: 450 us with
+// brick ops, 272 us.
+constexpr uint32_t kSyncWarps = 16;
+__global__ void __launch_bounds__(kSyncWarps * 32)
+    sync_sectors_kernel(const SectorOp* __restrict__ ops, const uint8_t* __restrict__ stage,
+                        const uint8_t* __restrict__ scratch, AllocState state, SectorRec* __restrict__ sectors,
+                        uint8_t* __restrict__ payload, uint4* __restrict__ codes, uint64_t* __restrict__ cells) {
+    __shared__ __align__(16) uint8_t sb[kSyncWarps][512];
+    __shared__ SectorOp op;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    if (threadIdx.x < 3)
+        reinterpret_cast<uint4*>(&op)[threadIdx.x] = reinterpret_cast<const uint4*>(ops + blockIdx.x)[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sectors[op.sector] = SectorRec{(uint32_t)op.mask, (uint32_t)(op.mask >> 32), op.base, 0};
+        if (blockIdx.x == 0) {
+            state.alloc->top = state.top;
+            state.alloc->live = state.live;
+            state.alloc->cap = state.cap;
         }
     }
-}
-
-// Sector-group masks of the GLSL mode's 4th level (VoxelTraversal.glsl:114-118): per
-// group of 4^3 sectors, bit x | z<<2 | y<<4 set when that sector holds a brick
-// (GpuRenderer.cpp:139-149); groups indexed x + z*GX + y*GX*GZ, one warp each (lane l
-// tests sectors l and l + 32 of the group, a ballot gathers each half).
-__global__ void group_masks_kernel(const SectorRec* __restrict__ sectors, uint32_t sx, uint32_t sy, uint32_t sz,
-                                   unsigned long long* __restrict__ groups) {
-    const uint32_t gx = (sx + 3) / 4, gy = (sy + 3) / 4, gz = (sz + 3) / 4;
-    const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (g >= gx * gy * gz) return;  // whole warps leave together
-    const uint32_t x0 = (g % gx) * 4, z0 = ((g / gx) % gz) * 4, y0 = (g / (gx * gz)) * 4;
-    uint32_t half[2];
-    for (uint32_t h = 0; h < 2; h++) {
-        const uint32_t b = lane + 32 * h;
-        const uint32_t x = x0 + (b & 3), z = z0 + ((b >> 2) & 3), y = y0 + (b >> 4);
-        bool nonempty = false;
-        if (x < sx && y < sy && z < sz) {
-            const SectorRec r = sectors[x + z * sx + y * sx * sz];
-            nonempty = (r.mask_lo | r.mask_hi) != 0;
-        }
-        half[h] = __ballot_sync(0xffffffffu, nonempty);
+    const uint64_t write = op.dirty | op.moved | op.fresh;
+    const uint32_t n = (uint32_t)__popcll(write);
+    uint4 v[4];
+    uint32_t dst[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+        const uint32_t k = wib + j * kSyncWarps;
+        if (k >= n) break;
+        const uint32_t b = warp_nth_bit(write, k, lane);
+        const uint64_t bit = 1ull << b;
+        dst[j] = op.base + (uint32_t)__popcll(op.mask & (bit - 1));
+        v[j] = make_uint4(0, 0, 0, 0);
+        if (op.dirty & bit)
+            v[j] = __ldcs(reinterpret_cast<const uint4*>(
+                              stage + (size_t)(op.first_dirty + (uint32_t)__popcll(op.dirty & (bit - 1))) * 512) + lane);
+        else if (op.moved & bit)
+            v[j] = __ldcs(reinterpret_cast<const uint4*>(
+                              scratch + (size_t)(op.first_moved + (uint32_t)__popcll(op.moved & (bit - 1))) * 512) + lane);
     }
-    if (lane == 0) groups[g] = (unsigned long long)half[0] | (unsigned long long)half[1] << 32;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+        if (wib + j * kSyncWarps >= n) break;
+        store_brick(sb[wib], v[j], dst[j], lane, payload, codes, cells);
+        __syncwarp();
+    }
 }
 
 // The brick-table entry of brick b of sector s, written at its brick position; group_mask: the
@@ -201,30 +194,21 @@ __device__ __forceinline__ void write_table_entry(const SectorRec* __restrict__ 
     bricks[bx + bz * (sx * 4) + by * (sx * 4) * (sz * 4)] = e;
 }
 
-// Brick-table entries of sectors [s_lo, s_hi), one thread per brick position.
-__global__ void brick_table_kernel(const SectorRec* __restrict__ sectors, const unsigned long long* __restrict__ groups,
-                                   uint32_t s_lo, uint32_t s_hi, uint32_t sx, uint32_t sz,
-                                   uint32_t* __restrict__ bricks) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (s_hi - s_lo) * 64u) return;
-    const uint32_t s = s_lo + (i >> 6), gx = (sx + 3) / 4, gz = (sz + 3) / 4;
-    const uint32_t x = s % sx, z = (s / sx) % sz, y = s / (sx * sz);
-    write_table_entry(sectors, groups + (x >> 2) + (z >> 2) * gx + (y >> 2) * gx * gz, s, i & 63u, sx, sz, bricks);
-}
-
-// The masks of listed sector groups (4^3 sectors, index x + z*GX + y*GX*GZ) and the brick-table
-// entries of their sectors, 16 blocks of 256 threads per group: after an edit, only the groups
-// of the sectors it changed are re-derived (a sector's emptiness changes its group's mask,
-// which the GLSL entries of the group's empty sectors read).  Each block derives the mask
-// from the 64 sector records itself, so no pass over all groups goes before (1.4 us and a gap
-// of 3 us between the kernels).
+// Masks of sector groups, the GLSL mode's 4th level (VoxelTraversal.glsl:114-118): per group of
+// 4^3 sectors (index x + z*GX + y*GX*GZ) bit x | z<<2 | y<<4 set when that sector holds a brick
+// (GpuRenderer.cpp:139-149); and the brick-table entries of the groups' sectors, 16 blocks of
+// 256 threads per group of the list, or of every group without one.  After an edit, only the
+// groups of the sectors it changed are re-derived (a sector's emptiness changes its group's
+// mask, which the GLSL entries of the group's empty sectors read).  Each block derives the
+// mask from the 64 sector records itself, so no pass over all groups goes before (1.4 us and
+// a gap of 3 us between the kernels).
 __global__ void __launch_bounds__(256)
     brick_table_groups_kernel(const SectorRec* __restrict__ sectors, unsigned long long* __restrict__ groups,
                               const uint32_t* __restrict__ list, uint32_t sx, uint32_t sy, uint32_t sz,
                               uint32_t* __restrict__ bricks) {
     __shared__ uint32_t s_half[2];
     __shared__ unsigned long long s_mask;
-    const uint32_t g = list[blockIdx.x >> 4], gx = (sx + 3) / 4, gz = (sz + 3) / 4;
+    const uint32_t g = list ? list[blockIdx.x >> 4] : blockIdx.x >> 4, gx = (sx + 3) / 4, gz = (sz + 3) / 4;
     const uint32_t x0 = (g % gx) * 4, z0 = ((g / gx) % gz) * 4, y0 = (g / (gx * gz)) * 4;
     if (threadIdx.x < 64) {
         const uint32_t b = threadIdx.x, x = x0 + (b & 3u), z = z0 + ((b >> 2) & 3u), y = y0 + (b >> 4);
@@ -246,11 +230,6 @@ __global__ void __launch_bounds__(256)
     const uint32_t x = x0 + (si & 3u), z = z0 + ((si >> 2) & 3u), y = y0 + (si >> 4);
     if (x >= sx || y >= sy || z >= sz) return;
     write_table_entry(sectors, &s_mask, x + z * sx + y * sx * sz, i & 63u, sx, sz, bricks);
-}
-
-uint32_t ops_grid(uint32_t n) {
-    uint32_t blocks = (n + kOpsWarps - 1) / kOpsWarps;
-    return std::max(1u, std::min(blocks, 152u * 16u));
 }
 
 // ---------------------------------------------------------------------------
@@ -294,13 +273,12 @@ vrt_status grow_pool(vrt_world* w, uint32_t min_capacity, cudaStream_t stream) {
     return VRT_OK;
 }
 
-// One self-consistent batch of sector updates: plan, then move, upload, zero.
+// One self-consistent batch of sector updates: plan, then gather, then write.
 struct SyncBatch {
-    std::vector<uint32_t> gathers;   // old slots copied to scratch first
-    std::vector<BrickOp> ops;
+    std::vector<SectorOp> ops;
+    std::vector<uint32_t> gathers;   // old slots of moved bricks, copied to scratch first
     const uint8_t* src = nullptr;    // first input brick of the batch
     uint64_t n_stage = 0;            // bricks staged from the input
-    std::vector<uint32_t> touched;   // sector linear indices
 };
 
 vrt_status plan_sector(vrt_world* w, SyncBatch& b, uint32_t s, uint64_t am, uint64_t dm, uint64_t stage_first,
@@ -312,134 +290,83 @@ vrt_status plan_sector(vrt_world* w, SyncBatch& b, uint32_t s, uint64_t am, uint
         vrt_status st = grow_pool(w, w->capacity + 64, stream);
         if (st != VRT_OK) return st;
     }
-    uint64_t rank_in = 0;
-    for (uint64_t r = cur.mask; r; r &= r - 1) {
-        const uint32_t brick = (uint32_t)__builtin_ctzll(r);
-        const uint32_t dst = cur.slot_of(brick) - 1;
-        const uint64_t bit = 1ull << brick;
-        if (dm & bit) {
-            rank_in = (uint64_t)__builtin_popcountll(dm & (bit - 1));
-            b.ops.push_back({dst, kOpUpload << 30 | (uint32_t)(stage_first + rank_in)});
-        } else if (old.mask & bit) {
-            const uint32_t src = old.slot_of(brick) - 1;
-            if (src != dst) {
-                b.ops.push_back({dst, kOpMove << 30 | (uint32_t)b.gathers.size()});
-                b.gathers.push_back(src);
-            }
-        } else {
-            b.ops.push_back({dst, kOpZero << 30});
-        }
+    SectorOp op{};
+    op.mask = cur.mask;
+    op.dirty = dm & cur.mask;
+    op.fresh = cur.mask & ~op.dirty & ~old.mask;
+    op.sector = s;
+    op.base = cur.base ? cur.base - 1 : 0;
+    op.first_dirty = (uint32_t)stage_first;
+    op.first_moved = (uint32_t)b.gathers.size();
+    for (uint64_t r = cur.mask & ~op.dirty & old.mask; r; r &= r - 1) {
+        const uint32_t brick = (uint32_t)__builtin_ctzll(r), src = old.slot_of(brick) - 1;
+        if (src == cur.slot_of(brick) - 1) continue;
+        op.moved |= 1ull << brick;
+        b.gathers.push_back(src);
     }
-    SectorRec& rec = w->h_table[s];
-    rec.mask_lo = (uint32_t)cur.mask;
-    rec.mask_hi = (uint32_t)(cur.mask >> 32);
-    rec.base = cur.base ? cur.base - 1 : 0;
-    rec.flags = 0;
-    b.touched.push_back(s);
-    return VRT_OK;
-}
-
-// Re-derive the sector-group masks and the whole brick table from the device sector
-// table (a sector's emptiness changes the GLSL-mode entries of its whole group).
-cudaError_t rebuild_brick_table(vrt_world* w, cudaStream_t stream) {
-    const uint32_t ng = w->num_groups();
-    group_masks_kernel<<<(ng + 3) / 4, 128, 0, stream>>>(w->d_sectors, w->sx, w->sy, w->sz,
-                                                       (unsigned long long*)w->d_groups);
-    const uint32_t ns = w->num_sectors(), n = ns * 64;
-    brick_table_kernel<<<(n + 255) / 256, 256, 0, stream>>>(w->d_sectors, (const unsigned long long*)w->d_groups, 0,
-                                                           ns, w->sx, w->sz, w->d_bricks);
-    return cudaGetLastError();
-}
-
-// The same for the groups of the given sectors only (device list in `list`, at most
-// num_groups entries); the whole table when they are most of the world.
-vrt_status rebuild_brick_table_for(vrt_world* w, const std::vector<uint32_t>& sectors, cudaStream_t stream) {
-    const uint32_t gx = (w->sx + 3) / 4, gz = (w->sz + 3) / 4;
-    std::vector<uint32_t> gl;
-    gl.reserve(sectors.size());
-    for (uint32_t s : sectors) {
-        const uint32_t x = s % w->sx, z = (s / w->sx) % w->sz, y = s / (w->sx * w->sz);
-        gl.push_back((x >> 2) + (z >> 2) * gx + (y >> 2) * gx * gz);
-    }
-    std::sort(gl.begin(), gl.end());
-    gl.erase(std::unique(gl.begin(), gl.end()), gl.end());
-    if ((uint64_t)gl.size() * 4 >= w->num_groups()) {
-        VRT_CUDA(rebuild_brick_table(w, stream));
-        return VRT_OK;
-    }
-    VRT_CUDA(w->d_glist.reserve(gl.size() * sizeof(uint32_t)));
-    VRT_CUDA(cudaMemcpyAsync(w->d_glist.ptr, gl.data(), gl.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
-    brick_table_groups_kernel<<<(uint32_t)gl.size() * 16u, 256, 0, stream>>>(
-        w->d_sectors, (unsigned long long*)w->d_groups, (const uint32_t*)w->d_glist.ptr, w->sx, w->sy, w->sz,
-        w->d_bricks);
-    VRT_CUDA(cudaGetLastError());
+    b.ops.push_back(op);
+    w->h_table[s] = SectorRec{(uint32_t)cur.mask, (uint32_t)(cur.mask >> 32), op.base, 0};
     return VRT_OK;
 }
 
 }  // namespace
 
-vrt_status rebuild_table_groups(vrt_world* w, const uint32_t* d_groups, uint32_t n, cudaStream_t stream) {
-    if (!d_groups || (uint64_t)n * 4 >= w->num_groups()) {
-        VRT_CUDA(rebuild_brick_table(w, stream));
-        return VRT_OK;
-    }
-    if (n == 0) return VRT_OK;
-    brick_table_groups_kernel<<<n * 16u, 256, 0, stream>>>(w->d_sectors, (unsigned long long*)w->d_groups, d_groups,
-                                                          w->sx, w->sy, w->sz, w->d_bricks);
+vrt_status rebuild_table_groups(vrt_world* w, const uint32_t* groups, uint32_t n, cudaStream_t stream) {
+    if (groups && n == 0) return VRT_OK;
+    const bool all = !groups || (uint64_t)n * 4 >= w->num_groups();
+    brick_table_groups_kernel<<<(all ? w->num_groups() : n) * 16u, 256, 0, stream>>>(
+        w->d_sectors, (unsigned long long*)w->d_groups, all ? nullptr : groups, w->sx, w->sy, w->sz, w->d_bricks);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }
 
 namespace {
 
+size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
+
 vrt_status run_batch(vrt_world* w, SyncBatch& b, cudaStream_t stream) {
-    if (b.ops.empty() && b.touched.empty()) return VRT_OK;
+    if (b.ops.empty()) return VRT_OK;
     const size_t stage_bytes = (size_t)b.n_stage * 512;
     if (stage_bytes) {
         VRT_CUDA(w->d_stage.reserve(stage_bytes));
         VRT_CUDA(cudaMemcpyAsync(w->d_stage.ptr, b.src, stage_bytes, cudaMemcpyHostToDevice, stream));
     }
-    const size_t gbytes = b.gathers.size() * sizeof(uint32_t);
-    const size_t obytes = b.ops.size() * sizeof(BrickOp);
-    const size_t ooff = (gbytes + 15) & ~size_t(15);
-    if (gbytes + obytes) {
-        VRT_CUDA(w->d_ops.reserve(ooff + obytes, true));
-        if (gbytes) VRT_CUDA(cudaMemcpyAsync(w->d_ops.ptr, b.gathers.data(), gbytes, cudaMemcpyHostToDevice, stream));
-        if (obytes)
-            VRT_CUDA(cudaMemcpyAsync((uint8_t*)w->d_ops.ptr + ooff, b.ops.data(), obytes, cudaMemcpyHostToDevice, stream));
+    // sector groups whose brick-table entries follow the sectors
+    const uint32_t gx = (w->sx + 3) / 4, gz = (w->sz + 3) / 4;
+    std::vector<uint32_t> groups;
+    groups.reserve(b.ops.size());
+    for (const SectorOp& op : b.ops) {
+        const uint32_t x = op.sector % w->sx, z = (op.sector / w->sx) % w->sz, y = op.sector / (w->sx * w->sz);
+        groups.push_back((x >> 2) + (z >> 2) * gx + (y >> 2) * gx * gz);
     }
-    const size_t ng = b.gathers.size();
+    std::sort(groups.begin(), groups.end());
+    groups.erase(std::unique(groups.begin(), groups.end()), groups.end());
+    // the kernels read the lists where they are, in pinned memory (a few bytes per sector)
+    const size_t ng = b.gathers.size(), ob = b.ops.size() * sizeof(SectorOp);
+    const size_t goff = align16(ob), loff = align16(goff + ng * sizeof(uint32_t));
+    VRT_CUDA(w->sync_stage.acquire(loff + groups.size() * sizeof(uint32_t)));
+    uint8_t* h = (uint8_t*)w->sync_stage.ptr;
+    std::memcpy(h, b.ops.data(), ob);
+    if (ng) std::memcpy(h + goff, b.gathers.data(), ng * sizeof(uint32_t));
+    std::memcpy(h + loff, groups.data(), groups.size() * sizeof(uint32_t));
     if (ng) {
-        VRT_CUDA(w->d_scratch.reserve(ng * 1088, true));
-        uint8_t* sp = (uint8_t*)w->d_scratch.ptr;
-        uint4* sc = (uint4*)(sp + ng * 512);
-        uint64_t* sm = (uint64_t*)(sp + ng * 1024);
-        gather_bricks_kernel<<<ops_grid((uint32_t)ng), kOpsWarps * 32, 0, stream>>>(
-            (const uint32_t*)w->d_ops.ptr, (uint32_t)ng, w->d_payload, w->d_codes, w->d_cells, sp, sc, sm);
+        VRT_CUDA(w->d_scratch.reserve(ng * 512, true));
+        gather_bricks_kernel<<<(uint32_t)((ng + 7) / 8), 256, 0, stream>>>((const uint32_t*)(h + goff), (uint32_t)ng,
+                                                                          w->d_payload, (uint8_t*)w->d_scratch.ptr);
         VRT_CUDA(cudaGetLastError());
     }
-    if (!b.ops.empty()) {
-        uint8_t* sp = (uint8_t*)w->d_scratch.ptr;
-        uint4* sc = sp ? (uint4*)(sp + ng * 512) : nullptr;
-        uint64_t* sm = sp ? (uint64_t*)(sp + ng * 1024) : nullptr;
-        brick_ops_kernel<<<ops_grid((uint32_t)b.ops.size()), kOpsWarps * 32, 0, stream>>>(
-            (const BrickOp*)((uint8_t*)w->d_ops.ptr + ooff), (uint32_t)b.ops.size(), (const uint8_t*)w->d_stage.ptr,
-            sp, sc, sm, w->d_payload, w->d_codes, w->d_cells);
-        VRT_CUDA(cudaGetLastError());
-    }
-    // sector headers: copy the span of touched records
-    if (!b.touched.empty()) {
-        auto mm = std::minmax_element(b.touched.begin(), b.touched.end());
-        const uint32_t lo = *mm.first, hi = *mm.second + 1;
-        VRT_CUDA(cudaMemcpyAsync(w->d_sectors + lo, w->h_table.data() + lo, (size_t)(hi - lo) * sizeof(SectorRec),
-                                 cudaMemcpyHostToDevice, stream));
-        vrt_status st = rebuild_brick_table_for(w, b.touched, stream);
-        if (st != VRT_OK) return st;
-    }
-    vrt_status st = alloc_publish(w, stream);
+    w->top_bound = w->arena.high_water() - 1;  // as alloc_publish
+    const AllocState state{w->d_alloc, (uint32_t)w->top_bound, w->arena.allocated(), w->capacity};
+    sync_sectors_kernel<<<(uint32_t)b.ops.size(), kSyncWarps * 32, 0, stream>>>(
+        (const SectorOp*)h, (const uint8_t*)w->d_stage.ptr, (const uint8_t*)w->d_scratch.ptr, state, w->d_sectors,
+        w->d_payload, w->d_codes, w->d_cells);
+    VRT_CUDA(cudaGetLastError());
+    vrt_status st = rebuild_table_groups(w, (const uint32_t*)(h + loff), (uint32_t)groups.size(), stream);
     if (st != VRT_OK) return st;
     VRT_CUDA(cudaStreamSynchronize(stream));
-    b = SyncBatch();
+    b.ops.clear();
+    b.gathers.clear();
+    b.n_stage = 0;
     return VRT_OK;
 }
 
@@ -500,9 +427,6 @@ vrt_status vrt_world_create(const vrt_world_desc* desc, vrt_world** out) {
         if (e == cudaSuccess) e = cudaMemset(w->d_sectors, 0, (size_t)w->num_sectors() * sizeof(SectorRec));
         if (e == cudaSuccess) e = cudaMalloc(&w->d_bricks, w->num_brick_positions() * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMalloc(&w->d_groups, (size_t)w->num_groups() * sizeof(uint64_t));
-        // the group list of incremental table rebuilds, at its largest size: it never
-        // grows (a growing buffer's cudaFree would wait for the whole device)
-        if (e == cudaSuccess) e = w->d_glist.reserve((size_t)w->num_groups() * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMalloc(&w->d_alloc, sizeof(DevAlloc));
         if (e == cudaSuccess) e = cudaMemset(w->d_alloc, 0, sizeof(DevAlloc));
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->edited, cudaEventDisableTiming);
@@ -511,9 +435,10 @@ vrt_status vrt_world_create(const vrt_world_desc* desc, vrt_world** out) {
         if (e == cudaSuccess) e = w->d_edit.reserve(256 << 10);
         for (auto& stage : w->edit_stage)
             if (e == cudaSuccess) e = stage.acquire(64 << 10);
-        if (e == cudaSuccess) e = rebuild_brick_table(w, 0);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+        if (e == cudaSuccess) e = w->sync_stage.acquire(64 << 10);
         if (e != cudaSuccess) st = cuda_fail(e, "allocate sector table");
+        if (st == VRT_OK) st = rebuild_table_groups(w, nullptr, 0, 0);
+        if (st == VRT_OK && (e = cudaStreamSynchronize(0)) != cudaSuccess) st = cuda_fail(e, "build brick table");
     }
     if (st == VRT_OK) st = grow_pool(w, desc->brick_capacity ? desc->brick_capacity : 4096, 0);
     if (st == VRT_OK) st = alloc_publish(w, 0);
@@ -539,10 +464,9 @@ vrt_status vrt_world_destroy(vrt_world* w) {
     if (w->d_payload) cudaFree(w->d_payload);
     if (w->d_cells) cudaFree(w->d_cells);
     w->d_stage.release();
-    w->d_ops.release();
     w->d_scratch.release();
     w->d_io.release();
-    w->d_glist.release();
+    w->sync_stage.destroy();
     w->d_edit.release();
     for (auto& stage : w->edit_stage) stage.destroy();
     if (w->d_alloc) cudaFree(w->d_alloc);
@@ -576,7 +500,7 @@ vrt_status vrt_world_get_stats(const vrt_world* cw, vrt_world_stats* out) {
     // 64 B cell masks, and the scratch buffers
     out->device_bytes = (uint64_t)w->num_sectors() * sizeof(SectorRec) + (uint64_t)w->num_brick_positions() * 4 +
                         (uint64_t)w->num_groups() * 8 + (uint64_t)w->capacity * 1088 + w->d_stage.bytes +
-                        w->d_ops.bytes + w->d_scratch.bytes + w->d_io.bytes + w->d_glist.bytes + w->d_edit.bytes;
+                        w->d_scratch.bytes + w->d_io.bytes + w->d_edit.bytes;
     return VRT_OK;
 }
 
@@ -594,7 +518,8 @@ vrt_status vrt_world_sync_sectors(vrt_world* w, uint32_t n, const int32_t* secto
     cudaStream_t stream = (cudaStream_t)stream_;
     const uint64_t kBatchBricks = 1ull << 19;  // 256 MiB of staged bricks per batch
     SyncBatch batch;
-    std::unordered_set<uint32_t> seen;
+    batch.ops.reserve(std::min<uint32_t>(n, 1u << 16));
+    std::vector<uint8_t> seen(w->num_sectors());  // sectors of the current batch
     uint64_t in_brick = 0;  // index of the next brick in the input stream
     for (uint32_t i = 0; i < n; i++) {
         const uint64_t am = alloc_mask[i];
@@ -608,11 +533,11 @@ vrt_status vrt_world_sync_sectors(vrt_world* w, uint32_t n, const int32_t* secto
         sector_index_unpack(sector_idx[i], x, y, z);
         if (w->sector_in(x, y, z)) {
             const uint32_t s = w->lin(x, y, z);
-            if (seen.count(s) || batch.n_stage + cnt > kBatchBricks) {
+            if (seen[s] || batch.n_stage + cnt > kBatchBricks) {
                 if ((st = run_batch(w, batch, stream)) != VRT_OK) return st;
-                seen.clear();
+                std::fill(seen.begin(), seen.end(), 0);
             }
-            if (batch.ops.empty() && batch.touched.empty()) {
+            if (batch.ops.empty()) {
                 batch.src = bricks ? bricks + in_brick * 512 : nullptr;
                 batch.n_stage = 0;
             }
@@ -620,7 +545,7 @@ vrt_status vrt_world_sync_sectors(vrt_world* w, uint32_t n, const int32_t* secto
             const uint64_t first = (bricks ? (in_brick - (uint64_t)(batch.src - bricks) / 512) : 0);
             if ((st = plan_sector(w, batch, s, am, dm, first, stream)) != VRT_OK) return st;
             batch.n_stage = first + cnt;
-            seen.insert(s);
+            seen[s] = 1;
         }
         in_brick += cnt;
     }

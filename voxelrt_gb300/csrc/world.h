@@ -114,9 +114,8 @@ struct vrt_world {
 
     // scratch reused across sync/edit calls
     vrt::DevBuf d_stage;    // uploaded brick bytes
-    vrt::DevBuf d_ops;      // brick operation lists
     vrt::DevBuf d_scratch;  // bricks in flight during a repack
-    vrt::DevBuf d_glist;    // sector groups whose brick-table entries an edit re-derives
+    vrt::HostStage sync_stage;  // sector ops, gather list and group list of a sync batch (pinned)
     vrt::DevBuf d_io;       // ray/hit staging for host-buffer calls
     std::vector<vrt::SectorRec> h_table;  // host copy of the sector table
 
@@ -206,7 +205,7 @@ vrt_status alloc_publish(vrt_world* w, cudaStream_t stream);
 vrt_status ensure_headroom(vrt_world* w, uint64_t need, cudaStream_t stream);
 // Pack the live bricks from slot 0 in sector order into a pool of `capacity` slots.
 vrt_status world_compact(vrt_world* w, uint32_t capacity, cudaStream_t stream);
-// Brick-table entries of the listed sector groups (device list of n groups), or of the
-// whole world when they are a quarter of it or more.
-vrt_status rebuild_table_groups(vrt_world* w, const uint32_t* d_groups, uint32_t n, cudaStream_t stream);
+// Masks and brick-table entries of the listed sector groups (n of them, in device or pinned
+// memory), or of the whole world without a list or when they are a quarter of it or more.
+vrt_status rebuild_table_groups(vrt_world* w, const uint32_t* groups, uint32_t n, cudaStream_t stream);
 }  // namespace vrt

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWo
     ray_start<kGlsl>(s, clip, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, coarse);
     TraceCounters cnt;
     uint32_t k = 0;
-    const bool hit = dda_steps_mode<false, kGlsl, true>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, k,
+    const bool hit = dda_steps_mode<false, kGlsl, !kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, k,
                                                                 max_iters) == kStepHit;
     out[i] = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, k, __float_as_uint(b.z));
 }
@@ -143,7 +143,7 @@ __global__ void __maxnreg__(48) cast_persistent_kernel(const __grid_constant__ D
             const uint32_t kmax = min(inner, max_iters - iter);
             uint32_t k = 0;
             // GLSL variants (rayCastCoarse, anisotropic LODs) are uniform over the launch
-            const uint32_t st = dda_steps_mode<false, kGlsl, true>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, iter, k,
+            const uint32_t st = dda_steps_mode<false, kGlsl, !kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, iter, k,
                                                              kmax);
             iter += k;
             if (st != kStepContinue || iter >= max_iters) {

@@ -41,6 +41,33 @@ __device__ __forceinline__ float add_rd(float a, float b) {
 #endif
 }
 
+// Two float adds in one instruction (sm_100 and later), each rounded as its scalar form: the step
+// loop is bound by instruction issue, and x and y take the same operations. 1080p GLSL frame with
+// a shadow ray 126.7 -> 121.8 us, 1080p x 8 views 754 -> 742, 64 mixed views 679 -> 671, an
+// anisotropic path batch 710 -> 694. The products stay scalar: a packed multiply that feeds a
+// packed add is contracted to a fused multiply-add also where both ask for rounding and the
+// build turns contraction off, and other results follow.
+struct F2 {
+    float x, y;
+};
+#ifdef __CUDA_ARCH__
+#define VRT_F2_ADD(name, op)                                                                 \
+    __device__ __forceinline__ F2 name(F2 a, F2 b) {                                         \
+        F2 r;                                                                                \
+        asm("{\n.reg .b64 a, b, r;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\n" op         \
+            " r, a, b;\nmov.b64 {%0, %1}, r;\n}"                                             \
+            : "=f"(r.x), "=f"(r.y)                                                           \
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                       \
+        return r;                                                                            \
+    }
+VRT_F2_ADD(add2, "add.rn.f32x2")
+VRT_F2_ADD(add2_rd, "add.rm.f32x2")
+#undef VRT_F2_ADD
+#else
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { return F2{__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)}; }
+__device__ __forceinline__ F2 add2_rd(F2 a, F2 b) { return F2{add_rd(a.x, b.x), add_rd(a.y, b.y)}; }
+#endif
+
 // Voxel coordinates as floats with an integer part in the low bits.  kVoxelBias is the
 // bit pattern of M = 1.5 * 2^23, where one ulp is 1: for an integer |n| < 2^22 the float
 // M + n has the bits kVoxelBias + n.  With a near world origin the float K = M + worldOrigin
@@ -204,6 +231,14 @@ __device__ __forceinline__ void ray_init(RayState& s, const ClipBox& b, float ox
     s.fast = s.fast && b.near && fabsf(ox) < kFastOrigin && fabsf(oy) < kFastOrigin && fabsf(oz) < kFastOrigin;
 }
 
+// The position at distance t.
+__device__ __forceinline__ void set_position(RayState& s, float t) {
+    const F2 c = add2(F2{s.ox, s.oy}, F2{__fmul_rn(t, s.dx), __fmul_rn(t, s.dy)});
+    s.cx = c.x;
+    s.cy = c.y;
+    s.cz = __fadd_rn(s.oz, __fmul_rn(t, s.dz));
+}
+
 // GLSL mode: the step's distance and position from its side distances.  tmin + 5 ulp as
 // an integer add on the bits; a NaN tmin stays NaN (its bit pattern differs between
 // platforms: the GPU's 0x7FFFFFFF would wrap to a denormal).  A rayCastCoarse ray takes
@@ -214,9 +249,7 @@ __device__ __forceinline__ void glsl_advance(RayState& s, bool coarse_ray) {
     const float m = min_x86(min_x86(s.sx, s.sy), s.sz);
     const float t = coarse_ray ? __fadd_rn(m, 0.001f) : (!kFast && m != m) ? m : __uint_as_float(__float_as_uint(m) + 5u);
     s.tb = t;
-    s.cx = __fadd_rn(s.ox, __fmul_rn(t, s.dx));
-    s.cy = __fadd_rn(s.oy, __fmul_rn(t, s.dy));
-    s.cz = __fadd_rn(s.oz, __fmul_rn(t, s.dz));
+    set_position(s, t);
 }
 
 // GLSL mode (VoxelTraversal.glsl rayCast): the start voxel worldOrigin + floor(start), and
@@ -307,20 +340,24 @@ __device__ __forceinline__ void step_on(RayState& s, uint32_t vx, uint32_t vy, u
     vx = (vx | m) ^ ((uint32_t)s.gx & m);
     vy = (vy | m) ^ ((uint32_t)s.gy & m);
     vz = (vz | m) ^ ((uint32_t)s.gz & m);
-    const float fx = kFast ? __fsub_rn(__uint_as_float(vx), voxel_frame(wox)) : rel_voxel((int32_t)vx, wox);
-    const float fy = kFast ? __fsub_rn(__uint_as_float(vy), voxel_frame(woy)) : rel_voxel((int32_t)vy, woy);
-    const float fz = kFast ? __fsub_rn(__uint_as_float(vz), voxel_frame(woz)) : rel_voxel((int32_t)vz, woz);
-    s.sx = __fadd_rn(s.tsx, __fmul_rn(fx, s.ix));
-    s.sy = __fadd_rn(s.tsy, __fmul_rn(fy, s.iy));
-    s.sz = __fadd_rn(s.tsz, __fmul_rn(fz, s.iz));
+    if (kFast) {
+        const F2 f = add2(F2{__uint_as_float(vx), __uint_as_float(vy)}, F2{-voxel_frame(wox), -voxel_frame(woy)});
+        const float fz = __fsub_rn(__uint_as_float(vz), voxel_frame(woz));
+        const F2 d = add2(F2{s.tsx, s.tsy}, F2{__fmul_rn(f.x, s.ix), __fmul_rn(f.y, s.iy)});
+        s.sx = d.x;
+        s.sy = d.y;
+        s.sz = __fadd_rn(s.tsz, __fmul_rn(fz, s.iz));
+    } else {
+        s.sx = __fadd_rn(s.tsx, __fmul_rn(rel_voxel((int32_t)vx, wox), s.ix));
+        s.sy = __fadd_rn(s.tsy, __fmul_rn(rel_voxel((int32_t)vy, woy), s.iy));
+        s.sz = __fadd_rn(s.tsz, __fmul_rn(rel_voxel((int32_t)vz, woz), s.iz));
+    }
     if (kGlsl) {
         glsl_advance<kFast>(s, kCoarse && (coarse & kCoarseRay) != 0);
     } else {
         const float t = kFast ? __fadd_rn(fminf(fminf(s.sx, s.sy), s.sz), 0.001f)
                               : __fadd_rn(min_x86(min_x86(s.sx, s.sy), s.sz), 0.001f);
-        s.cx = __fadd_rn(s.ox, __fmul_rn(t, s.dx));
-        s.cy = __fadd_rn(s.oy, __fmul_rn(t, s.dy));
-        s.cz = __fadd_rn(s.oz, __fmul_rn(t, s.dz));
+        set_position(s, t);
     }
 }
 
@@ -353,8 +390,9 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int
     uint32_t vx, vy, vz;  // the voxel; of a fast ray its biased form
     constexpr uint32_t kBias = kFast ? kVoxelBias : 0u;
     if (kFast) {
-        vx = __float_as_uint(add_rd(s.cx, voxel_frame(wox)));
-        vy = __float_as_uint(add_rd(s.cy, voxel_frame(woy)));
+        const F2 r = add2_rd(F2{s.cx, s.cy}, F2{voxel_frame(wox), voxel_frame(woy)});
+        vx = __float_as_uint(r.x);
+        vy = __float_as_uint(r.y);
         vz = __float_as_uint(add_rd(s.cz, voxel_frame(woz)));
     } else {
         // floor2i: a NaN coordinate converts to INT32_MIN on x86 and leaves the grid;

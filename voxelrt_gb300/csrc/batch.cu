@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "batch_internal.h"
+#include "thin_launch.cuh"
 #include "trace_core.cuh"
 #include "world.h"
 
@@ -135,14 +136,14 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
     }
 }
 
-// One thread per pixel, whole path (VoxelRender.comp:27-93 structure).
-template <bool kGlsl, bool kAniso = false>
+// One thread per pixel (thin_pixel), whole path (VoxelRender.comp:27-93 structure).
+template <bool kGlsl, bool kAniso, bool kThin>
 __global__ void __launch_bounds__(64) view_path_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
-                                                       const __grid_constant__ ViewStart vs, uint4* __restrict__ out) {
+                                                       const __grid_constant__ ViewStart vs, uint32_t lanes_log2,
+                                                       uint4* __restrict__ out) {
     if constexpr (kAniso) fill_forward_lut();
-    const uint32_t px = blockIdx.x * 8 + threadIdx.x;
-    const uint32_t py = blockIdx.y * 8 + threadIdx.y;
-    if (px >= v.width || py >= v.height) return;
+    uint32_t px, py;
+    if (!thin_pixel<kThin>(lanes_log2, px, py) || px >= v.width || py >= v.height) return;
     trace_pixel<kGlsl, kAniso, true, false>(v, w, vs, px, py, out);
 }
 
@@ -786,19 +787,19 @@ ViewDev make_view_dev(const vrt_view& v) {
 namespace {
 
 vrt_status launch_view_path(vrt_world* w, const ViewDev& v, bool glsl, vrt_hit* hits, cudaStream_t stream) {
-    dim3 block(8, 8), grid((v.width + 7) / 8, (v.height + 7) / 8);
+    const uint32_t ll = thin_lanes_log2((uint64_t)v.width * v.height, kThinFrameWarps);
+    const dim3 grid = thin_grid(ll, v.width, v.height);
     L2Window l2;
     vrt_status st = l2.enter(w, stream);
     if (st != VRT_OK) return st;
     uint4* out = reinterpret_cast<uint4*>(hits);
     const DevWorld dw = w->dev();
     const ViewStart vs = view_start(dw, v);
-    if (glsl && v.aniso)
-        view_path_kernel<true, true><<<grid, block, 0, stream>>>(dw, v, vs, out);
-    else if (glsl)
-        view_path_kernel<true><<<grid, block, 0, stream>>>(dw, v, vs, out);
-    else
-        view_path_kernel<false><<<grid, block, 0, stream>>>(dw, v, vs, out);
+    auto kernel = ll < 5 ? (glsl ? (v.aniso ? view_path_kernel<true, true, true> : view_path_kernel<true, false, true>)
+                                 : view_path_kernel<false, false, true>)
+                         : (glsl ? (v.aniso ? view_path_kernel<true, true, false> : view_path_kernel<true, false, false>)
+                                 : view_path_kernel<false, false, false>);
+    kernel<<<grid, 64, 0, stream>>>(dw, v, vs, ll, out);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }

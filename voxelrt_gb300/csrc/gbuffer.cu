@@ -15,6 +15,7 @@
 #include <cstring>
 
 #include "batch_internal.h"
+#include "thin_launch.cuh"
 #include "trace_core.cuh"
 #include "world.h"
 
@@ -53,20 +54,20 @@ __device__ __forceinline__ void gbuffer_texel(const RayState& s, bool hit, uint3
     depth = __fdiv_rn(z, w);
 }
 
-// 8x8 pixels per block.  The palette is read where it lies, in the parameters' constant bank: a
+// 8x8 pixels per block, fewer of a small frame (thin_pixel).  The palette is read where it lies, in the parameters' constant bank: a
 // load takes a turn per distinct material of a warp's hits, a few in most scenes.  (Staging
 // it in shared memory cost every block 256 constant reads at 32 addresses a warp, and a
 // barrier: the address divergence unit was busy half the time.  1280x720 GLSL G-buffer of a
 // 512-voxel terrain: 51.5 us staged, 41.9 us direct; 35.9 us with the step of trace_core.cuh.)
-template <bool kGlsl, bool kAniso>
+template <bool kGlsl, bool kAniso, bool kThin>
 __global__ void __launch_bounds__(64) gbuffer_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
-                                                    const __grid_constant__ ClipBox clip, bool inside,
+                                                    const __grid_constant__ ClipBox clip, bool inside, uint32_t lanes_log2,
                                                     const __grid_constant__ GbufferParams gp,
                                                     uint32_t* __restrict__ tex, float* __restrict__ depth,
                                                     uint4* __restrict__ out) {
     if constexpr (kAniso) fill_forward_lut();
-    const uint32_t px = blockIdx.x * 8 + threadIdx.x, py = blockIdx.y * 8 + threadIdx.y;
-    if (px >= v.width || py >= v.height) return;
+    uint32_t px, py;
+    if (!thin_pixel<kThin>(lanes_log2, px, py) || px >= v.width || py >= v.height) return;
     const uint32_t pixel = py * v.width + px;
     float dx, dy, dz;
     camera_ray(v.d0, v.du, v.dv, px, py, dx, dy, dz);
@@ -96,17 +97,18 @@ vrt_status launch_gbuffer(vrt_world* w, const vrt_view* view, const uint32_t* pa
     std::memcpy(gp.palette, palette, sizeof(gp.palette));
     std::memcpy(gp.proj, proj, sizeof(gp.proj));
     const ViewDev v = make_view_dev(*view);
-    dim3 block(8, 8), grid((v.width + 7) / 8, (v.height + 7) / 8);
+    const uint32_t ll = thin_lanes_log2((uint64_t)v.width * v.height, kThinFrameWarps);
+    const dim3 grid = thin_grid(ll, v.width, v.height);
     uint4* out = reinterpret_cast<uint4*>(hits);
     const DevWorld dw = w->dev();
     const ClipBox clip = clip_box(dw, v.wo);
     const bool inside = origin_inside_near(clip, v.ox, v.oy, v.oz);
-    if (view_glsl(*view) && view_aniso(*view))
-        gbuffer_kernel<true, true><<<grid, block, 0, stream>>>(dw, v, clip, inside, gp, tex, depth, out);
-    else if (view_glsl(*view))
-        gbuffer_kernel<true, false><<<grid, block, 0, stream>>>(dw, v, clip, inside, gp, tex, depth, out);
-    else
-        gbuffer_kernel<false, false><<<grid, block, 0, stream>>>(dw, v, clip, inside, gp, tex, depth, out);
+    const bool aniso = view_aniso(*view);
+    auto kernel = ll < 5 ? (view_glsl(*view) ? (aniso ? gbuffer_kernel<true, true, true> : gbuffer_kernel<true, false, true>)
+                                             : gbuffer_kernel<false, false, true>)
+                         : (view_glsl(*view) ? (aniso ? gbuffer_kernel<true, true, false> : gbuffer_kernel<true, false, false>)
+                                             : gbuffer_kernel<false, false, false>);
+    kernel<<<grid, 64, 0, stream>>>(dw, v, clip, inside, ll, gp, tex, depth, out);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }

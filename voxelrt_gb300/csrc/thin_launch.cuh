@@ -1,0 +1,43 @@
+// Small launches: fewer rays per warp.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace vrt {
+
+// Rays per warp of a small launch (log2, 2..5): as few as keep the launch within `warps` warps.
+// A launch that leaves most of the chip idle lasts as long as its longest ray, and a ray's
+// step waits for the slowest lane of its warp: with 4 rays a warp a 64x64 frame of a
+// 256-voxel terrain takes 12.5 us against 14.5, 2,000 random rays 16.4 us against 18.6 (one ray a
+// warp: 12.7 and 15.6, but 2,000 GLSL rays 55 us against 41).  `warps` where the gain ends:
+// casts 32,000 rays; frames, whole paths and G-buffers earlier, as one whose rays end at once
+// lasts as long as its blocks take to launch (192x192 from within a solid voxel: 4.0 us,
+// thinned 5.2 us).  64x64 paths of the terrain: sun rays 20.1 -> 17.6 us, 3 bounces 41.4 -> 30.4,
+// anisotropic with both 51.4 -> 35.5; G-buffers 15.3 -> 13.3.
+constexpr uint32_t kThinFrameWarps = 1216, kThinCastWarps = 2432;
+inline uint32_t thin_lanes_log2(uint64_t rays, uint32_t warps) {
+    uint32_t l = 5;
+    while (l > 2 && rays >> (l - 1) <= warps) l--;
+    return l;
+}
+
+// The pixel of this thread in such a launch's frame: blocks of 2 warps, one above the other,
+// each an area of 2^lanes_log2 pixels (8x4 for 32).  False for a lane without one.  kThin: fewer
+// than 32, an instantiation of its own where the test costs the large launches (1 % of a
+// 720p G-buffer).
+template <bool kThin>
+__device__ __forceinline__ bool thin_pixel(uint32_t lanes_log2, uint32_t& px, uint32_t& py) {
+    if (!kThin) lanes_log2 = 5;
+    const uint32_t lane = threadIdx.x & 31, wl = (lanes_log2 + 1) / 2;
+    px = (blockIdx.x << wl) + (lane & ((1u << wl) - 1u));
+    py = ((blockIdx.y * 2 + (threadIdx.x >> 5)) << (lanes_log2 - wl)) + (lane >> wl);
+    return (lane >> lanes_log2) == 0;
+}
+inline dim3 thin_grid(uint32_t lanes_log2, uint32_t width, uint32_t height) {
+    const uint32_t wl = (lanes_log2 + 1) / 2, tw = 1u << wl, th = 2u << (lanes_log2 - wl);
+    return dim3((width + tw - 1) / tw, (height + th - 1) / th);
+}
+
+}  // namespace vrt

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "thin_launch.cuh"
 #include "trace_core.cuh"
 #include "world.h"
 
@@ -21,32 +22,15 @@ uint32_t eff_iters(uint32_t max_iters, bool glsl = false) {
     return max_iters > 65535u ? 65535u : max_iters;
 }
 
-// Rays per warp of a small launch (log2, 2..5): as few as keep the launch within `warps` warps.
-// A launch that leaves most of the chip idle lasts as long as its longest ray, and a ray's
-// step waits for the slowest lane of its warp: with 4 rays a warp a 64x64 frame of a
-// 256-voxel terrain takes 12.5 us against 14.5, 2,000 random rays 16.4 us against 18.6 (one ray a
-// warp: 12.7 and 15.6, but 2,000 GLSL rays 55 us against 41).  `warps` where the gain ends:
-// casts 32,000 rays; frames earlier, as one whose rays end at once lasts as long as its
-// blocks take to launch (192x192 from within a solid voxel: 4.0 us, thinned 5.2 us).
-constexpr uint32_t kThinFrameWarps = 1216, kThinCastWarps = 2432;
-uint32_t thin_lanes_log2(uint64_t rays, uint32_t warps) {
-    uint32_t l = 5;
-    while (l > 2 && rays >> (l - 1) <= warps) l--;
-    return l;
-}
-
-// One thread per pixel, 2 warps per block, each an area of 2^lanes_log2 pixels (8x4 for 32).
+// One thread per pixel (thin_pixel).
 // inside: the camera origin is (origin_inside_near)
 __global__ void __launch_bounds__(64) render_view_kernel(const __grid_constant__ DevWorld w,
                                                         const __grid_constant__ vrt_camera cam,
                                                         const __grid_constant__ ClipBox clip, bool inside,
                                                         uint32_t lanes_log2, uint32_t max_iters,
                                                         uint4* __restrict__ out) {
-    const uint32_t lane = threadIdx.x & 31, wl = (lanes_log2 + 1) / 2;
-    if (lane >> lanes_log2) return;
-    const uint32_t px = (blockIdx.x << wl) + (lane & ((1u << wl) - 1u));
-    const uint32_t py = ((blockIdx.y * 2 + (threadIdx.x >> 5)) << (lanes_log2 - wl)) + (lane >> wl);
-    if (px >= cam.width || py >= cam.height) return;
+    uint32_t px, py;
+    if (!thin_pixel<true>(lanes_log2, px, py) || px >= cam.width || py >= cam.height) return;
     float dx, dy, dz;
     camera_ray(cam, px, py, dx, dy, dz);
     const int32_t wox = cam.world_origin[0], woy = cam.world_origin[1], woz = cam.world_origin[2];
@@ -165,16 +149,14 @@ vrt_status check_camera(const vrt_camera* cam) {
 
 vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters, vrt_hit* hits,
                          cudaStream_t stream) {
-    const uint32_t ll = thin_lanes_log2((uint64_t)cam->width * cam->height, kThinFrameWarps), wl = (ll + 1) / 2;
-    const uint32_t tw = 1u << wl, th = 2u << (ll - wl);  // pixels of a block
-    const dim3 grid((cam->width + tw - 1) / tw, (cam->height + th - 1) / th);
+    const uint32_t ll = thin_lanes_log2((uint64_t)cam->width * cam->height, kThinFrameWarps);
     L2Window l2;
     vrt_status st = l2.enter(w, stream);
     if (st != VRT_OK) return st;
     const DevWorld dw = w->dev();
     const float* o = cam->origin;
     const ClipBox clip = clip_box(dw, cam->world_origin);
-    render_view_kernel<<<grid, 64, 0, stream>>>(dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]), ll,
+    render_view_kernel<<<thin_grid(ll, cam->width, cam->height), 64, 0, stream>>>(dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]), ll,
                                                 eff_iters(max_iters), reinterpret_cast<uint4*>(hits));
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;

@@ -433,10 +433,10 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
         const uint32_t act = __ballot_sync(0xffffffffu, active);
         bool q_wait = false;  // resident: nothing published right now
         if ((uint32_t)__popc(act) < p.refill && !q_empty) {
-            uint32_t idle = ~act;
+            uint32_t idle = kResident ? ~act : ~act & p.lanes;
             while (idle) {
                 if (q_next >= q_end) {
-                    uint32_t c = 0, nv = p.n_views;
+                    uint32_t c = 0, nv = p.n_views, part = 0;
                     if (kResident) {
                         if (lane == 0) {
                             c = resident_claim(p, rw, act != 0);
@@ -455,6 +455,8 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
                     } else {
                         if (lane == 0) c = atomicAdd(p.queue, 1u);
                         c = __shfl_sync(0xffffffffu, c, 0);
+                        part = c & ((1u << p.split_log2) - 1u);
+                        c >>= p.split_log2;
                         if (c >= p.total_chunks) {
                             q_empty = true;
                             break;
@@ -477,6 +479,7 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
                     }
                     q_view = lo;
                     q_next = (c - ldv<kResident>(p.chunk_base + lo)) * p.chunk_rays;
+                    if (!kResident) q_next += part * (p.chunk_rays >> p.split_log2);
                     if (kResident && lo != rw.cached_view) {
                         // every lane is done with the old copy, and the loads below are
                         // ordered after lane 0's acquire of the hint that published lo
@@ -488,7 +491,7 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
                         __syncwarp();
                     }
                     const ViewDev* qv = kResident ? &sview : p.views + lo;
-                    q_end = min(q_next + p.chunk_rays, vget<kResident>(&qv->n_rays, true));
+                    q_end = min(q_next + (kResident ? p.chunk_rays : p.chunk_rays >> p.split_log2), vget<kResident>(&qv->n_rays, true));
                     // the view's camera origin, shared by its rays: inside the clip box?
                     // (a resident view's world index is checked before it is used)
                     const int4 qwv = vget4<kResident>(reinterpret_cast<const int4*>(qv->wo));  // origin xyz, world
@@ -647,8 +650,9 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
 // 44 M rays over 154 views of 16 mixed worlds: 701 us against 1109 us;
 // six 1080p terrain views with sun rays: 754 us against 1035 us.  72 registers, 28 warps a
 // SM: 64 spill (713 and 767 us), 56 more so (759 and 803 us), 80 leave 24 warps (735 and 788 us).
-// kPacked: the records are stored in the 12-byte form.
-template <bool kGlsl, bool kAniso, bool kPacked>
+// kPacked: the records are stored in the 12-byte form.  kSplit: claims are parts of a tile
+// (launch_persistent), an instantiation of its own as their arithmetic cost the others 0.5 %.
+template <bool kGlsl, bool kAniso, bool kPacked, bool kSplit>
 __global__ void __maxnreg__(72) tile_kernel(BatchParams p) {
     if constexpr (kAniso) fill_forward_lut();
     // what the warp's view needs at a ray's start (warps_per_block <= 16)
@@ -662,21 +666,31 @@ __global__ void __maxnreg__(72) tile_kernel(BatchParams p) {
     const ViewDev& v = sw.v;
     DevWorld w{};  // a copy in registers: the step loop reads its table addresses and strides
     const uint32_t lane = threadIdx.x & 31;
-    // the lane's pixel in a tile's first 32; the next 32 lie `rows` rows below
-    uint32_t kx, ky;
-    if (p.morton) {
-        kx = compact_even_bits(lane);
-        ky = compact_even_bits(lane >> 1);
-    } else {
-        kx = lane & ((1u << p.tile_w_log2) - 1u);
-        ky = lane >> p.tile_w_log2;
-    }
-    const uint32_t rows = 32u >> p.tile_w_log2, tile_h = 1u << (p.tile_size_log2 - p.tile_w_log2);
+    // the lane's pixel in a tile's first 32 (the next 32 lie `rows` rows below), or in the part of a
+    // tile that the warp has claimed (split_log2 > 0); outside every view where the lane has none
+    uint32_t kx = 0, ky = 0;
+    const auto place = [&](uint32_t first) {
+        const uint32_t k = first + lane;
+        if (p.morton) {
+            kx = compact_even_bits(k);
+            ky = compact_even_bits(k >> 1);
+        } else {
+            kx = k & ((1u << p.tile_w_log2) - 1u);
+            ky = k >> p.tile_w_log2;
+        }
+        if (kSplit && !((p.lanes >> lane) & 1u)) kx = 1u << 16;
+    };
+    place(0);
+    const uint32_t tile_h = 1u << (p.tile_size_log2 - p.tile_w_log2), rows = kSplit ? tile_h : 32u >> p.tile_w_log2;
     const uint32_t chunk_tiles = p.chunk_rays >> p.tile_size_log2;
     uint32_t view = 0, loaded = kNoView, rays = 0;
     for (;;) {
         uint32_t c = lane == 0 ? atomicAdd(p.queue, 1u) : 0u;
         c = __shfl_sync(0xffffffffu, c, 0);
+        if (kSplit) {
+            place((c & ((1u << p.split_log2) - 1u)) << (p.tile_size_log2 - p.split_log2));
+            c >>= p.split_log2;
+        }
         if (c >= p.total_chunks) break;
         c += p.chunk_first;
         // a warp's claims only grow, so the chunk lies in the last view or a later one
@@ -952,13 +966,13 @@ PersistentFn persistent_fn_mode(bool glsl, bool aniso) {
     if (glsl) return persistent_kernel<kCount, true, kResident, false, kFull>;
     return persistent_kernel<kCount, false, kResident, false, kFull>;
 }
-template <bool kPacked>
+template <bool kPacked, bool kSplit>
 PersistentFn tile_fn(bool glsl, bool aniso) {
-    return glsl ? (aniso ? tile_kernel<true, true, kPacked> : tile_kernel<true, false, kPacked>)
-                : tile_kernel<false, false, kPacked>;
+    return glsl ? (aniso ? tile_kernel<true, true, kPacked, kSplit> : tile_kernel<true, false, kPacked, kSplit>)
+                : tile_kernel<false, false, kPacked, kSplit>;
 }
 PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, bool full, bool tiles) {
-    if (tiles && !count && !resident) return tile_fn<false>(glsl, aniso);
+    if (tiles && !count && !resident) return tile_fn<false, false>(glsl, aniso);
     if (resident) return full ? persistent_fn_mode<false, true, true>(glsl, aniso)
                               : persistent_fn_mode<false, true, false>(glsl, aniso);
     if (count) return full ? persistent_fn_mode<true, false, true>(glsl, aniso)
@@ -1023,12 +1037,34 @@ vrt_status launch_resident(const BatchParams& p, int blocks, int threads, cudaSt
     return VRT_OK;
 }
 
+// Claims smaller than a tile, of launches whose chunks are one tile of 64.  A launch of few tiles
+// leaves most of the chip idle, and a warp that traces 64 rays takes twice as long as one with
+// 32: half tiles up to kHalfTileChunks tiles (768x768, 9,216 tiles, primary rays from within a
+// solid voxel: 23.6 us against 21.2 whole; 512x512 terrain frames 27.7 -> 23.1 us).  Launches
+// with bounces take half tiles at any size, as their warps end far apart (two 720p views of 4
+// bounces 372 -> 355 us, 1024x1024 131 -> 118; quarter tiles 370 and 133 us).  Below
+// kThinBatchWarps warps also fewer rays a warp, down to 4, as in thin_launch.cuh (64x64
+// terrain views: primary rays 25.1 -> 17.7 us, 3 bounces 68 -> 36, anisotropic with sun rays and
+// bounces 86 -> 40; 4,864 warps are faster still there by 2 to 4 us, and slower by as much where
+// rays end at once).
+constexpr uint32_t kHalfTileChunks = 7296, kThinBatchWarps = 2432;
 vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool count, cudaStream_t stream,
                              size_t zero_bytes) {
     if (zero_bytes) VRT_CUDA(cudaMemsetAsync(p.queue, 0, zero_bytes, stream));
-    const PersistentFn fn = p.tiles && p.packed ? tile_fn<true>(p.glsl != 0, p.aniso != 0)
-                                                : persistent_fn(count, p.glsl != 0, p.aniso != 0, false, p.full != 0, p.tiles != 0);
-    fn<<<blocks, threads, pend_bytes(p, threads), stream>>>(p);
+    const bool tiles = p.tiles && !count;
+    BatchParams q = p;
+    q.split_log2 = 0;
+    q.lanes = 0xffffffffu;
+    if (p.chunk_rays == 64 && p.tile_size_log2 == 6 && (!tiles || p.total_chunks <= kHalfTileChunks)) {
+        q.split_log2 = 1;
+        while (q.split_log2 < 4 && (uint64_t)p.total_chunks << (q.split_log2 + 1) <= kThinBatchWarps) q.split_log2++;
+        q.lanes >>= 32 - (64 >> q.split_log2);
+    }
+    const bool glsl = p.glsl != 0, aniso = p.aniso != 0;
+    const PersistentFn fn = !tiles ? persistent_fn(count, glsl, aniso, false, p.full != 0, false)
+                            : q.split_log2 ? (p.packed ? tile_fn<true, true>(glsl, aniso) : tile_fn<false, true>(glsl, aniso))
+                            : p.packed ? tile_fn<true, false>(glsl, aniso) : tile_fn<false, false>(glsl, aniso);
+    fn<<<blocks, threads, pend_bytes(p, threads), stream>>>(q);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }

@@ -58,6 +58,8 @@ struct BatchParams {
     uint4* out;
     uint32_t tile_w_log2, tile_size_log2, morton;
     uint32_t chunk_rays;
+    // set by launch_persistent: claims per chunk of one tile (log2), and the lanes that take rays
+    uint32_t split_log2, lanes;
     uint32_t refill;
     uint32_t inner;
     uint32_t glsl;  // traversal mode of every view (VRT_VIEW_GLSL)

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWo
 // cast_kernel: a lane's steps continue from where its ray left off, and a ray's record
 // is packed from the state at its exit.
 template <bool kGlsl, bool kAniso = false>
-__global__ void __maxnreg__(48) cast_persistent_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ClipBox clip,
+__global__ void __maxnreg__(56) cast_persistent_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ClipBox clip,
                                                              const float4* __restrict__ rays, uint32_t n,
                                                              int32_t wox, int32_t woy, int32_t woz, uint32_t max_iters,
                                                              uint32_t inner, uint32_t refill, uint4* __restrict__ out,
@@ -91,12 +91,15 @@ __global__ void __maxnreg__(48) cast_persistent_kernel(const __grid_constant__ D
     RayState s;
     TraceCounters cnt{0, 0};
     for (;;) {
+        // The material of a ray that ended and the ray that takes its lane are loaded together,
+        // before the record is stored: one wait for memory a round in place of two.
+        uint32_t material = 0, rn = 0;
         if (ended) {
-            out[ri] = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, iter, tag);
-            ended = false;
+            material = hit_material(s, w.payload, hit);
             active = false;
         }
         const uint32_t act = __ballot_sync(0xffffffffu, active);
+        bool mine = false;
         if ((uint32_t)__popc(act) < refill) {
             uint32_t idle = ~act;
             while (idle) {
@@ -108,19 +111,30 @@ __global__ void __maxnreg__(48) cast_persistent_kernel(const __grid_constant__ D
                 }
                 const uint32_t take = min(q_end - q_next, (uint32_t)__popc(idle));
                 const uint32_t rank = __popc(idle & lt);
-                const bool mine = ((idle >> lane) & 1u) && rank < take;
-                const uint32_t assigned = __ballot_sync(0xffffffffu, mine);
-                if (mine) {
-                    ri = q_next + rank;
-                    const float4 a = __ldg(rays + 2 * (size_t)ri), b = __ldg(rays + 2 * (size_t)ri + 1);
-                    tag = __float_as_uint(b.z);
-                    ray_start<kGlsl>(s, clip, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, coarse);
-                    iter = 0;
-                    active = true;
+                const bool now = ((idle >> lane) & 1u) && rank < take;
+                if (now) {
+                    rn = q_next + rank;
+                    mine = true;
                 }
-                idle &= ~assigned;
+                idle &= ~__ballot_sync(0xffffffffu, now);
                 q_next += take;
             }
+        }
+        float4 a{}, b{};
+        if (mine) {
+            a = __ldg(rays + 2 * (size_t)rn);
+            b = __ldg(rays + 2 * (size_t)rn + 1);
+        }
+        if (ended) {
+            out[ri] = pack_state<kGlsl>(s, material, hit, iter, tag);
+            ended = false;
+        }
+        if (mine) {
+            ri = rn;
+            tag = __float_as_uint(b.z);
+            ray_start<kGlsl>(s, clip, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, coarse);
+            iter = 0;
+            active = true;
         }
         if (__ballot_sync(0xffffffffu, active) == 0) break;
         if (active) {
@@ -162,10 +176,10 @@ vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters
     return VRT_OK;
 }
 
-// Launch shape of cast_persistent_kernel (also capped at 48 registers, for more warps to hide
-// L2 latency: 40 and 56 measured 301 and 292 us against 286).  On 4.2 M random rays in a
-// 512-voxel world, slices of 8 steps took 268 us, of 12 steps 285 us and of 16 steps 291 us;
-// with the flat step 248 us.
+// Launch shape of cast_persistent_kernel.  On 4.2 M random rays in a 512-voxel world, slices of
+// 8 steps took 268 us, of 12 steps 285 us and of 16 steps 291 us (48 registers); with the flat
+// step 248 us; with the records' and the new rays' loads together and 56 registers 241 us (48:
+// 243).  Slices of 4 steps: 236 us, but 435 us against 390 for 700,000 anisotropic rays.
 constexpr uint32_t kCastThreads = 128, kCastInner = 8, kCastRefill = 28;
 // Below this many rays the thread-per-ray kernel is used (too few rays to fill the
 // persistent grid's lanes twice).

@@ -10,8 +10,8 @@ namespace vrt {
 // Rays per warp of a small launch (log2, 2..5): as few as keep the launch within `warps` warps.
 // A launch that leaves most of the chip idle lasts as long as its longest ray, and a ray's
 // step waits for the slowest lane of its warp: with 4 rays a warp a 64x64 frame of a
-// 256-voxel terrain takes 12.5 us against 14.5, 2,000 random rays 16.4 us against 18.6 (one ray a
-// warp: 12.7 and 15.6, but 2,000 GLSL rays 55 us against 41).  `warps` where the gain ends:
+// 256-voxel terrain takes 12.5 us against 14.5, 2,000 random rays 16.4 us against 18.6 (two rays a
+// warp: another 2 % at 1,000 to 2,000 rays, nothing elsewhere).  `warps` where the gain ends:
 // casts 32,000 rays; frames, whole paths and G-buffers earlier, as one whose rays end at once
 // lasts as long as its blocks take to launch (192x192 from within a solid voxel: 4.0 us,
 // thinned 5.2 us).  64x64 paths of the terrain: sun rays 20.1 -> 17.6 us, 3 bounces 41.4 -> 30.4,

@@ -59,10 +59,8 @@ __global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWo
     const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
     RayState s;
     ray_start<kGlsl>(s, clip, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, coarse);
-    TraceCounters cnt;
     uint32_t k = 0;
-    const bool hit = dda_steps_mode<false, kGlsl, !kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, k,
-                                                                max_iters) == kStepHit;
+    const bool hit = dda_trace<kGlsl, !kGlsl, kGlsl ? 8 : 16>(s, w, wox, woy, woz, coarse, coarse, kAniso, k, max_iters) == kStepHit;
     out[i] = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, k, __float_as_uint(b.z));
 }
 
@@ -88,6 +86,7 @@ __global__ void __maxnreg__(56) cast_persistent_kernel(const __grid_constant__ D
     uint32_t q_next = 0, q_end = 0;
     bool active = false, ended = false, hit = false;
     uint32_t ri = 0, iter = 0, tag = 0;
+    float t0 = 0.0f;
     RayState s;
     TraceCounters cnt{0, 0};
     for (;;) {
@@ -134,6 +133,7 @@ __global__ void __maxnreg__(56) cast_persistent_kernel(const __grid_constant__ D
             tag = __float_as_uint(b.z);
             ray_start<kGlsl>(s, clip, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, coarse);
             iter = 0;
+            t0 = no_t();
             active = true;
         }
         if (__ballot_sync(0xffffffffu, active) == 0) break;
@@ -144,6 +144,8 @@ __global__ void __maxnreg__(56) cast_persistent_kernel(const __grid_constant__ D
             const uint32_t st = dda_steps_mode<false, kGlsl, !kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, iter, k,
                                                              kmax);
             iter += k;
+            if (st == kStepContinue && stalled<kGlsl>(s, t0, coarse, iter - k)) iter = max_iters;
+            t0 = last_t<kGlsl>(s);
             if (st != kStepContinue || iter >= max_iters) {
                 ended = true;
                 hit = st == kStepHit;
@@ -179,11 +181,15 @@ vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters
 // Launch shape of cast_persistent_kernel.  On 4.2 M random rays in a 512-voxel world, slices of
 // 8 steps took 268 us, of 12 steps 285 us and of 16 steps 291 us (48 registers); with the flat
 // step 248 us; with the records' and the new rays' loads together and 56 registers 241 us (48:
-// 243).  Slices of 4 steps: 236 us, but 435 us against 390 for 700,000 anisotropic rays.
-constexpr uint32_t kCastThreads = 128, kCastInner = 8, kCastRefill = 28;
-// Below this many rays the thread-per-ray kernel is used (too few rays to fill the
-// persistent grid's lanes twice).
-constexpr uint32_t kCastPersistentMin = 1u << 18;
+// 243).  With rays that stand still ended early (stalled) slices of 4 steps are the best: 229 us (8:
+// 242, 3: 228, 2: 234), 4 M random rays of a terrain 176 us (3: 185, 2: 208), 2.5 M anisotropic
+// 128 us (8: 164).
+constexpr uint32_t kCastThreads = 128, kCastInner = 4, kCastRefill = 28;
+// Below this many rays the thread-per-ray kernel is used: too few rays to fill the persistent
+// grid's lanes several times.  400,000 random CPU rays 36 us against 40 (terrain) and 20 against
+// 24 (mixed world), 800,000 rays 60 and 34 against 57 and 35, and twice as fast on coherent ones at
+// any count; 400,000 anisotropic rays 42 and 34 us against 40 and 27.
+constexpr uint32_t kCastPersistentMin = 3u << 18, kCastPersistentMinGlsl = 1u << 18;
 
 vrt_status launch_cast(vrt_world* w, const vrt_ray* rays, uint32_t n, const vrt_cast_params* p, vrt_hit* hits,
                        cudaStream_t stream) {
@@ -199,7 +205,7 @@ vrt_status launch_cast(vrt_world* w, const vrt_ray* rays, uint32_t n, const vrt_
     L2Window l2;
     vrt_status st = l2.enter(w, stream);
     if (st != VRT_OK) return st;
-    if (n < kCastPersistentMin) {
+    if (n < (glsl ? kCastPersistentMinGlsl : kCastPersistentMin)) {
         auto kernel = glsl ? (aniso ? cast_kernel<true, true> : cast_kernel<true>) : cast_kernel<false>;
         const uint32_t ll = thin_lanes_log2(n, kThinCastWarps), per_block = 8u << ll;
         kernel<<<(n + per_block - 1) / per_block, 256, 0, stream>>>(dw, clip, r4, n, p->world_origin[0],

@@ -533,6 +533,47 @@ __device__ __forceinline__ uint32_t dda_steps_mode(RayState& s, const DevWorld& 
     }
 }
 
+// Rays that stand still.  Where the bias of a step's distance (0.001, or 5 ulp in GLSL mode) is lost
+// in the rounding of the position, a ray stays before the cell's face and repeats its step up
+// to the iteration cap: an explicit ray has its origin in world coordinates, and of random rays
+// through a 256-voxel terrain one in four stands still in GLSL mode (256 steps each) and one in 500
+// in CPU mode.  A step is a function of the position, and the position of the distance alone, so a
+// ray back at the distance it had some steps before repeats those steps, none of which ended
+// it: its record is that of the cap.  In CPU mode only for fast rays, whose distances are no
+// NaN; of a rayCastCoarse ray (coarse_ray) once its steps no longer depend on their number.
+// Looked at between slices of steps: 2,000 random GLSL rays 49 -> 13 us, 2.5 M 653 -> 112, 2.5 M
+// anisotropic 841 -> 128, 60,000 CPU rays in a mixed world 22.9 -> 12.1.  Frames and batches
+// look for none: camera rays start near the world origin and do not stand still, and the
+// slices' loop cost them 2 to 8 %.
+template <bool kGlsl>
+__device__ __forceinline__ float last_t(const RayState& s) {
+    return kGlsl ? s.tb : fminf(fminf(s.sx, s.sy), s.sz);
+}
+__device__ __forceinline__ float no_t() { return __uint_as_float(0x7FFFFFFFu); }  // equals no distance
+// t0: last_t before iteration `first`, with one step or more since.
+template <bool kGlsl>
+__device__ __forceinline__ bool stalled(const RayState& s, float t0, bool coarse_ray, uint32_t first) {
+    return last_t<kGlsl>(s) == t0 && (kGlsl || s.fast) && (!kGlsl || !coarse_ray || first >= kCoarseFrom);
+}
+
+// dda_steps_mode from iteration i to the ray's end or `iters`, kSlice steps at a time.
+template <bool kGlsl, bool kFlat, uint32_t kSlice>
+__device__ __forceinline__ uint32_t dda_trace(RayState& s, const DevWorld& w, int32_t wox, int32_t woy, int32_t woz,
+                                              bool coarse, bool coarse_ray, bool aniso, uint32_t& i, uint32_t iters) {
+    TraceCounters cnt{0, 0};
+    float t0 = no_t();
+    for (;;) {
+        const uint32_t first = i, lim = iters - i < kSlice ? iters : i + kSlice;
+        const uint32_t st = dda_steps_mode<false, kGlsl, kFlat>(s, w, wox, woy, woz, cnt, coarse, coarse_ray, aniso, 0, i, lim);
+        if (st != kStepContinue || i >= iters) return st;
+        if (stalled<kGlsl>(s, t0, coarse_ray, first)) {
+            i = iters;
+            return st;
+        }
+        t0 = last_t<kGlsl>(s);
+    }
+}
+
 // Voxel id of a hit (0 on a miss), read once its ray has ended.
 __device__ __forceinline__ uint32_t hit_material(const RayState& s, const uint8_t* payload, bool hit) {
     return hit ? __ldg(payload + s.hit_byte()) : 0u;

@@ -58,9 +58,10 @@ __device__ __forceinline__ void gbuffer_texel(const RayState& s, bool hit, uint3
 // load takes a turn per distinct material of a warp's hits, a few in most scenes.  (Staging
 // it in shared memory cost every block 256 constant reads at 32 addresses a warp, and a
 // barrier: the address divergence unit was busy half the time.  1280x720 GLSL G-buffer of a
-// 512-voxel terrain: 51.5 us staged, 41.9 us direct; 35.9 us with the step of trace_core.cuh.)
+// 512-voxel terrain: 51.5 us staged, 41.9 us direct; 35.6 us with the step of trace_core.cuh, 35.0
+// with leave for 48 registers (the compiler's own choice is 32).)
 template <bool kGlsl, bool kAniso, bool kThin>
-__global__ void __launch_bounds__(64) gbuffer_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
+__global__ void __maxnreg__(48) gbuffer_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
                                                     const __grid_constant__ ClipBox clip, bool inside, uint32_t lanes_log2,
                                                     const __grid_constant__ GbufferParams gp,
                                                     uint32_t* __restrict__ tex, float* __restrict__ depth,

@@ -22,9 +22,11 @@ uint32_t eff_iters(uint32_t max_iters, bool glsl = false) {
     return max_iters > 65535u ? 65535u : max_iters;
 }
 
-// One thread per pixel (thin_pixel).
+// One thread per pixel (thin_pixel).  Bound by the latency of its steps: with leave for 48 registers
+// (the compiler's choice is 32) frames of a terrain take 3 to 8 % less (64x64 of a 256-voxel one
+// 14.3 -> 13.8 us, 192x192 15.3 -> 14.0, 512x512 16.1 -> 15.5).
 // inside: the camera origin is (origin_inside_near)
-__global__ void __launch_bounds__(64) render_view_kernel(const __grid_constant__ DevWorld w,
+__global__ void __maxnreg__(48) render_view_kernel(const __grid_constant__ DevWorld w,
                                                         const __grid_constant__ vrt_camera cam,
                                                         const __grid_constant__ ClipBox clip, bool inside,
                                                         uint32_t lanes_log2, uint32_t max_iters,

@@ -649,13 +649,14 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
 // share (ViewStart) belong to the warp: in shared memory, read at a ray's start, the step
 // loop's part in registers.  Warp instructions for 32 primary rays, against the persistent
 // kernel: 240 and 48 a step, against 335 and 52, and 170 in all for a camera in a solid voxel.
-// 44 M rays over 154 views of 16 mixed worlds: 701 us against 1109 us;
-// six 1080p terrain views with sun rays: 754 us against 1035 us.  72 registers, 28 warps a
-// SM: 64 spill (713 and 767 us), 56 more so (759 and 803 us), 80 leave 24 warps (735 and 788 us).
+// 44 M rays over 154 views of 16 mixed worlds: 701 us against 1109 us, 658 us with the packed adds
+// and 64 registers; six 1080p terrain views with sun rays: 754 us against 1035 us, 718 us.  64
+// registers, 32 warps a SM, in the CPU traversal (72, 28 warps: 670 and 740 us, 56: 714 and 767);
+// 72 in the GLSL modes (64 cost an anisotropic 1800x1800 batch 9 %).
 // kPacked: the records are stored in the 12-byte form.  kSplit: claims are parts of a tile
 // (launch_persistent), an instantiation of its own as their arithmetic cost the others 0.5 %.
 template <bool kGlsl, bool kAniso, bool kPacked, bool kSplit>
-__global__ void __maxnreg__(72) tile_kernel(BatchParams p) {
+__global__ void __maxnreg__(kGlsl ? 72 : 64) tile_kernel(BatchParams p) {
     if constexpr (kAniso) fill_forward_lut();
     // what the warp's view needs at a ray's start (warps_per_block <= 16)
     struct Warp {

@@ -113,6 +113,8 @@ def tune(worlds, views, hits, stream, log=print, passes: int = 2) -> tuple[dict,
          for r, i in itertools.product([1, 2, 4, 8, 12, 16, 20, 24, 28], [4, 8, 16, 32, 64, 128])],
         [dict(chunk_tiles=c) for c in (1, 2, 4, 8, 16, 32, 64)],
     ]
+    if not any(vw.n_bounces for vw in views):
+        del stages[1]  # read by launches with bounces alone
     tried = set()
     for _ in range(passes):
         for stage in stages:

@@ -889,8 +889,10 @@ uint32_t auto_chunk_tiles(uint64_t tiles, uint64_t warps) {
 // Tiles per claim of tile_kernel where the config leaves it open, at most: the launch ends with
 // the last claims, and 16 tiles (1,024 rays) of long rays run on for a third of a millisecond
 // after the queue is empty (44 M rays over 154 views: 1466 us with 16 tiles, 1041 with 4, 968
-// with 2, 950 with 1 in the kernel's first build; terrain views as well).  2 halve the claims.
-constexpr uint32_t kTileChunk = 2;
+// with 2, 950 with 1 in the kernel's first build; 658 with 2, 782 with 1 in the present one).
+// Pixels with a sun ray are twice the work, so one tile up to kOneTileWarps a warp (six 1080p
+// views 718 -> 697 us).
+constexpr uint32_t kTileChunk = 2, kOneTileWarps = 64;
 bool tile_launch(const vrt_view* views, uint32_t n) {
     for (uint32_t i = 0; i < n; i++)
         if (views[i].n_bounces) return false;
@@ -912,7 +914,14 @@ void resolve_batch_defaults(vrt_batch_config& cfg, const vrt_view* views, uint32
 void resolve_launch_config(vrt_batch_config& cfg, const vrt_view* views, uint32_t n, uint64_t warps) {
     const bool open = cfg.chunk_tiles == 0;
     resolve_batch_defaults(cfg, views, n, warps);
-    if (open && tile_launch(views, n)) cfg.chunk_tiles = std::min(cfg.chunk_tiles, kTileChunk);
+    if (!open || !tile_launch(views, n)) return;
+    bool sun = false;
+    uint64_t pixels = 0;
+    for (uint32_t i = 0; i < n; i++) {
+        sun |= (views[i].flags & VRT_VIEW_SHADOW) != 0;
+        pixels += (uint64_t)views[i].cam.width * views[i].cam.height;
+    }
+    cfg.chunk_tiles = sun && pixels / 64 < kOneTileWarps * warps ? 1 : std::min(cfg.chunk_tiles, kTileChunk);
 }
 
 vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, const vrt_batch_config& cfg_in,

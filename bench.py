@@ -251,8 +251,8 @@ def peak_hbm():
 
 # What bounds the persistent kernel on a workload, from the committed ncu summaries.
 LIMITERS = {
-    "uneven_batch": "instruction issue: 72.5 % of issue slots busy, wait (fixed-latency dependency) the first "
-                    "stall (profiles/persistent_kernel_uneven_batch_medium.md)",
+    "uneven_batch": "instruction issue: 79 % of issue slots busy, 28 of 32 lanes (tile_kernel, "
+                    "profiles/traversal_kernels.md)",
 }
 
 
@@ -534,7 +534,7 @@ class GpuEngine:
                 "world_bytes": int(sum(d.n_bricks for d in wl.worlds) * SLOT_BYTES),
                 "l2": "inputs larger than L2 (brick pools of all worlds); l2_flushed: the same launches, each after an L2 flush",
                 "batch_config": autotune.describe(self.cfg), "batch_config_source": self.cfg_src,
-                "launch": "persistent kernel + queue reset, CUDA graph replay",
+                "launch": "one kernel + queue reset, CUDA graph replay",
                 "traversal": traversal_name(self.args),
                 "l2_persist": bool(getattr(self.args, "l2_persist", False))}
 

@@ -418,8 +418,9 @@ typedef struct vrt_batch_config {
                                   launch with diffuse bounces, else 16); not used by a launch
                                   without bounces, whose warps trace 32 pixels to the end */
     uint32_t chunk_tiles;      /* tiles taken from the device queue per atomic (1..64; 0 = 1 for a
-                                  launch with diffuse bounces, else chosen per launch: about
-                                  eight fetches per warp, 1..2 tiles) */
+                                  launch with diffuse bounces, else 1 or 2 by the launch's size).
+                                  With 1, a tile of 64 rays is taken by halves in a launch with
+                                  bounces, and by halves or less in one of few tiles */
     uint32_t inner_iters;      /* DDA iterations between checks for ended rays (0 = 16); not used by
                                   a launch without bounces */
 } vrt_batch_config;

@@ -137,7 +137,7 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
 }
 
 // One thread per pixel (thin_pixel), whole path (VoxelRender.comp:27-93 structure).  kBounces: the
-// view has bounces; without them 48 registers in place of 56 (a 1080p GLSL frame with its sun
+// view has bounces; without them 48 registers in place of 56 (a 1080p frame with its sun
 // ray: 121.6 -> 118.0 us).
 template <bool kGlsl, bool kAniso, bool kBounces, bool kThin>
 __global__ void __launch_bounds__(64) view_path_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,

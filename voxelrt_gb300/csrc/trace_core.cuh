@@ -42,7 +42,7 @@ __device__ __forceinline__ float add_rd(float a, float b) {
 }
 
 // Two float adds in one instruction (sm_100 and later), each rounded as its scalar form: the step
-// loop is bound by instruction issue, and x and y take the same operations. 1080p GLSL frame with
+// loop is bound by instruction issue, and x and y take the same operations. 1080p frame with
 // a shadow ray 126.7 -> 121.8 us, 1080p x 8 views 754 -> 742, 64 mixed views 679 -> 671, an
 // anisotropic path batch 710 -> 694. The products stay scalar: a packed multiply that feeds a
 // packed add is contracted to a fused multiply-add also where both ask for rounding and the

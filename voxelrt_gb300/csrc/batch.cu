@@ -288,8 +288,8 @@ __device__ __forceinline__ void resident_pixels_done(const BatchParams& p, uint3
 
 // kFull: the launch may hold views with the GPU renderer's whole path (a separate
 // instantiation, so the others keep their code and registers).  64 registers (32 warps a SM)
-// are enough for the CPU traversal (two 720p views of 4 bounces: 409 us against 429 us with
-// 72), not for the GLSL modes (two worlds' whole paths: 735 us against 717 us).
+// are enough for the CPU traversal (two 720p views of 4 bounces: 355 us against 382 us with
+// 72 and 379 us with 56), not for the GLSL modes (two worlds' whole paths: 654 us against 626 us).
 template <bool kCount, bool kGlsl, bool kResident = false, bool kAniso = false, bool kFull = false>
 __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
     if constexpr (kAniso) fill_forward_lut();
@@ -604,7 +604,7 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
         }
         // Steps until half the tracing lanes have ended, in slices of p.inner: the lanes left
         // keep the warp busy, and enough have ended to share a retirement.  Two 720p views of
-        // 4 bounces: 468 us, one slice a round 472 us, a quarter left 485 us.
+        // 4 bounces: 372 us, five eighths left 374 us, three eighths 377 us.
         const uint32_t stop = (uint32_t)__popc(__ballot_sync(0xffffffffu, active)) / 2u;
         do {
             if (active && !(path & kEnded)) {

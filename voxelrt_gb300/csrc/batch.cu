@@ -1073,14 +1073,16 @@ vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool
     BatchParams q = p;
     q.split_log2 = 0;
     q.lanes = 0xffffffffu;
-    if (p.chunk_rays == 64 && p.tile_size_log2 == 6 && (!tiles || p.total_chunks <= kHalfTileChunks)) {
+    // (the queue counts claims in 32 bits)
+    if (p.chunk_rays == 64 && p.tile_size_log2 == 6 && p.total_chunks <= (tiles ? kHalfTileChunks : 1u << 30)) {
         q.split_log2 = 1;
         while (q.split_log2 < 4 && (uint64_t)p.total_chunks << (q.split_log2 + 1) <= kThinBatchWarps) q.split_log2++;
         q.lanes >>= 32 - (64 >> q.split_log2);
     }
     // no more warps than claims: each takes a turn at the queue's counter and returns (64x64 views
     // 13.3 -> 11.3 us from within a solid voxel, 35.7 -> 33.5 with 3 bounces of a terrain)
-    blocks = (int)std::min<uint64_t>((uint64_t)blocks, (((uint64_t)p.total_chunks << q.split_log2) * 32 + threads - 1) / threads);
+    const uint64_t claims = std::max<uint64_t>(1, (uint64_t)p.total_chunks << q.split_log2);
+    blocks = (int)std::min<uint64_t>((uint64_t)blocks, (claims * 32 + threads - 1) / threads);
     const bool glsl = p.glsl != 0, aniso = p.aniso != 0;
     const PersistentFn fn = !tiles ? persistent_fn(count, glsl, aniso, false, p.full != 0, false)
                             : q.split_log2 ? (p.packed ? tile_fn<true, true>(glsl, aniso) : tile_fn<false, true>(glsl, aniso))

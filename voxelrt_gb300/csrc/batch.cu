@@ -140,7 +140,7 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
 // view has bounces; without them 48 registers in place of 56 (a 1080p frame with its sun
 // ray: 121.6 -> 118.0 us).
 template <bool kGlsl, bool kAniso, bool kBounces, bool kThin>
-__global__ void __launch_bounds__(64) view_path_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
+__global__ void __launch_bounds__(kFrameThreads) view_path_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
                                                        const __grid_constant__ ViewStart vs, uint32_t lanes_log2,
                                                        uint4* __restrict__ out) {
     if constexpr (kAniso) fill_forward_lut();
@@ -822,7 +822,7 @@ vrt_status launch_view_path(vrt_world* w, const ViewDev& v, bool glsl, vrt_hit* 
     const bool bounces = v.last_kind() > 1u || (v.last_kind() == 1u && !v.shadow());
     const ViewPathFn kernel = bounces ? (ll < 5 ? view_path_fn<true, true>(glsl, v.aniso) : view_path_fn<true, false>(glsl, v.aniso))
                                       : (ll < 5 ? view_path_fn<false, true>(glsl, v.aniso) : view_path_fn<false, false>(glsl, v.aniso));
-    kernel<<<grid, 64, 0, stream>>>(dw, v, vs, ll, out);
+    kernel<<<grid, kFrameThreads, 0, stream>>>(dw, v, vs, ll, out);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }

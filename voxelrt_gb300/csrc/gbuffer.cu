@@ -54,7 +54,7 @@ __device__ __forceinline__ void gbuffer_texel(const RayState& s, bool hit, uint3
     depth = __fdiv_rn(z, w);
 }
 
-// 8x8 pixels per block, fewer of a small frame (thin_pixel).  The palette is read where it lies, in the parameters' constant bank: a
+// 16x8 pixels per block, fewer of a small frame (thin_pixel).  The palette is read where it lies, in the parameters' constant bank: a
 // load takes a turn per distinct material of a warp's hits, a few in most scenes.  (Staging
 // it in shared memory cost every block 256 constant reads at 32 addresses a warp, and a
 // barrier: the address divergence unit was busy half the time.  1280x720 GLSL G-buffer of a
@@ -109,7 +109,7 @@ vrt_status launch_gbuffer(vrt_world* w, const vrt_view* view, const uint32_t* pa
                                              : gbuffer_kernel<false, false, true>)
                          : (view_glsl(*view) ? (aniso ? gbuffer_kernel<true, true, false> : gbuffer_kernel<true, false, false>)
                                              : gbuffer_kernel<false, false, false>);
-    kernel<<<grid, 64, 0, stream>>>(dw, v, clip, inside, ll, gp, tex, depth, out);
+    kernel<<<grid, kFrameThreads, 0, stream>>>(dw, v, clip, inside, ll, gp, tex, depth, out);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }

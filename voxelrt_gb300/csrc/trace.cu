@@ -174,7 +174,7 @@ vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters
     const DevWorld dw = w->dev();
     const float* o = cam->origin;
     const ClipBox clip = clip_box(dw, cam->world_origin);
-    render_view_kernel<<<thin_grid(ll, cam->width, cam->height), 64, 0, stream>>>(dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]), ll,
+    render_view_kernel<<<thin_grid(ll, cam->width, cam->height), kFrameThreads, 0, stream>>>(dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]), ll,
                                                 eff_iters(max_iters), reinterpret_cast<uint4*>(hits));
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;

@@ -8,10 +8,10 @@ import voxelrt_gb300 as v
 from tests.helpers import both_worlds, oracle_view
 
 pytestmark = pytest.mark.gpu
-# n >> (l - 1) <= warps: casts 2432 warps (4 rays a warp up to 9728 rays, 8 to 19456, 16 to 38912)
+# n >> (l - 1) <= 2432 warps (4 rays a warp up to 9728 rays, 8 to 19456, 16 to 38912)
 COUNTS = [1, 3, 4, 5, 31, 33, 127, 2000, 9728, 9731, 19456, 19459, 38911, 38915]
-# frames 1216 warps (4 up to 4864 pixels, 8 to 9728, 16 to 19456)
-SHAPES = [(1, 1), (3, 2), (64, 64), (76, 64), (77, 64), (4864, 1), (1, 4866), (139, 70), (128, 76), (195, 100), (140, 139)]
+SHAPES = [(1, 1), (3, 2), (64, 64), (76, 64), (77, 64), (4864, 1), (1, 4866), (139, 70), (128, 76), (195, 100), (140, 139), (256, 152),
+          (195, 200)]
 
 
 @pytest.fixture(scope="module")

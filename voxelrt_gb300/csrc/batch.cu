@@ -811,7 +811,7 @@ ViewPathFn view_path_fn(bool glsl, bool aniso) {
 }
 
 vrt_status launch_view_path(vrt_world* w, const ViewDev& v, bool glsl, vrt_hit* hits, cudaStream_t stream) {
-    const uint32_t ll = thin_lanes_log2((uint64_t)v.width * v.height, kThinFrameWarps);
+    const uint32_t ll = thin_lanes_log2((uint64_t)v.width * v.height);
     const dim3 grid = thin_grid(ll, v.width, v.height);
     L2Window l2;
     vrt_status st = l2.enter(w, stream);

@@ -33,8 +33,8 @@ __device__ __forceinline__ uint32_t compact_even_bits(uint32_t k) {
 }
 
 // What the rays of one view share, from its camera origin: whether that is inside and near
-// (origin_inside_near), and (tile_kernel, CPU traversal) what iteration 0 finds there: the origin's voxel in biased form and the alignment
-// mask of its cell, or that it is solid.
+// (origin_inside_near), and (tile_kernel, CPU traversal) what iteration 0 finds there: the
+// origin's voxel in biased form and the alignment mask of its cell, or that it is solid.
 constexpr uint32_t kStartUnknown = 0xFFFFFFFFu, kStartSolid = 0xFFFFFFFEu;
 struct ViewStart {
     ClipBox clip;

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "cast_queue.h"
 #include "thin_launch.cuh"
 #include "trace_core.cuh"
 #include "world.h"
@@ -107,8 +108,8 @@ __global__ void __maxnreg__(56) cast_persistent_kernel(const __grid_constant__ D
                 if (q_next >= q_end) {
                     if (next >= n) break;
                     q_next = next;
-                    q_end = min(next + 32u, n);
-                    next = next + stride < next ? n : next + stride;  // no wrap past 2^32
+                    q_end = chunk_end(next, n);
+                    next = chunk_after(next, stride, n);
                 }
                 const uint32_t take = min(q_end - q_next, (uint32_t)__popc(idle));
                 const uint32_t rank = __popc(idle & lt);

@@ -70,9 +70,9 @@ __global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWo
 // Explicit rays whose lengths vary widely (random origins and directions: some hit at
 // once, others run to the iteration cap) leave most lanes of a thread-per-ray warp idle
 // behind its longest ray.  Here each warp walks its own grid-strided sequence of 32-ray
-// chunks (warp g takes rays [32 (g + k G), +32) for k = 0, 1, ...), traces in rounds
-// of `inner` DDA steps, and between rounds stores the records of the rays that ended
-// and refills those lanes from its chunks once fewer than `refill` lanes trace.  No
+// chunks (warp g takes rays [32 (g + k G), +32) for k = 0, 1, ...), traces in slices
+// of `inner` DDA steps, and once fewer than `refill` lanes trace stores the records of the
+// rays that ended and refills those lanes from its chunks.  No
 // device queue: calls on different streams stay independent.  Same records as
 // cast_kernel: a lane's steps continue from where its ray left off, and a ray's record
 // is packed from the state at its exit.
@@ -140,20 +140,21 @@ __global__ void __maxnreg__(56) cast_persistent_kernel(const __grid_constant__ D
             active = true;
         }
         if (__ballot_sync(0xffffffffu, active) == 0) break;
-        if (active) {
-            const uint32_t kmax = min(inner, max_iters - iter);
-            uint32_t k = 0;
-            // GLSL variants (rayCastCoarse, anisotropic LODs) are uniform over the launch
-            const uint32_t st = dda_steps_mode<false, kGlsl, !kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, iter, k,
-                                                             kmax);
-            iter += k;
-            if (st == kStepContinue && stalled<kGlsl>(s, t0, coarse, iter - k)) iter = max_iters;
-            t0 = last_t<kGlsl>(s);
-            if (st != kStepContinue || iter >= max_iters) {
-                ended = true;
-                hit = st == kStepHit;
+        // slices until fewer than `refill` lanes are tracing
+        do {
+            if (active && !ended) {
+                const uint32_t first = iter, lim = max_iters - iter < inner ? max_iters : iter + inner;
+                // GLSL variants (rayCastCoarse, anisotropic LODs) are uniform over the launch
+                const uint32_t st = dda_steps_mode<false, kGlsl, true>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0,
+                                                                       iter, lim);
+                if (st == kStepContinue && stalled<kGlsl>(s, t0, coarse, first)) iter = max_iters;
+                t0 = last_t<kGlsl>(s);
+                if (st != kStepContinue || iter >= max_iters) {
+                    ended = true;
+                    hit = st == kStepHit;
+                }
             }
-        }
+        } while ((uint32_t)__popc(__ballot_sync(0xffffffffu, active && !ended)) >= refill);
     }
 }
 
@@ -181,13 +182,21 @@ vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters
     return VRT_OK;
 }
 
-// Launch shape of cast_persistent_kernel.  On 4.2 M random rays in a 512-voxel world, slices of
-// 8 steps took 268 us, of 12 steps 285 us and of 16 steps 291 us (48 registers); with the flat
-// step 248 us; with the records' and the new rays' loads together and 56 registers 241 us (48:
-// 243).  With rays that stand still ended early (stalled) slices of 4 steps are the best: 229 us (8:
-// 242, 3: 228, 2: 234), 4 M random rays of a terrain 176 us (3: 185, 2: 208), 2.5 M anisotropic
-// 128 us (8: 164).
-constexpr uint32_t kCastThreads = 128, kCastInner = 4, kCastRefill = 28;
+// Launch shape of cast_persistent_kernel.  A slice's end costs about as much as a step, and lanes
+// whose rays have ended, or stand still (stalled), wait for it: short slices where rays end early or
+// stand still, longer ones where they are long and no slice finds a stalled ray.  On 4.2 M random
+// rays, launches repeated on the same rays:
+// - CPU traversal, slices of 4 / 5 / 6 / 8: 512-voxel mixed world 238 / 241 / 243 / 251 us, terrain
+//   232 / 225 / 222 / 224, a world with 2 % of its voxels set 462 / 445 / 432 / 413 (1 M of them 150 /
+//   144 / 140 / 134, as 147 with slices of 12 and no test for stalled rays);
+// - GLSL, 4 / 6 / 8: 208 / 227 / 250, 198 / 211 / 227, 280 / 296 / 322 us; anisotropic LODs alike;
+// - rayCastCoarse, whose rays are looked at from iteration 31 on alone, 4 / 8 / 12: 255 / 270 /
+//   284, 242 / 246 / 271, 602 / 532 / 527; with anisotropic LODs, 4 / 5 / 8: 192 / 196 / 221,
+//   257 / 259 / 284, 497 / 480 / 453 (504 us before the slices went on until a refill).
+constexpr uint32_t kCastThreads = 128, kCastRefill = 28;
+constexpr uint32_t cast_slice(bool glsl, bool coarse, bool aniso) {
+    return coarse ? (aniso ? 5u : 8u) : glsl ? 4u : 5u;
+}
 // Below this many rays the thread-per-ray kernel is used: too few rays to fill the persistent
 // grid's lanes several times.  400,000 random CPU rays 36 us against 40 (terrain) and 20 against
 // 24 (mixed world), 800,000 rays 60 and 34 against 57 and 35, and twice as fast on coherent ones at
@@ -223,7 +232,8 @@ vrt_status launch_cast(vrt_world* w, const vrt_ray* rays, uint32_t n, const vrt_
         VRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kCastThreads, 0));
         const uint32_t blocks = (uint32_t)(sms * std::max(occ, 1));
         kernel<<<blocks, kCastThreads, 0, stream>>>(dw, clip, r4, n, p->world_origin[0], p->world_origin[1],
-                                                    p->world_origin[2], iters, kCastInner, kCastRefill, o4, coarse);
+                                                    p->world_origin[2], iters, cast_slice(glsl, coarse, aniso), kCastRefill, o4,
+                                                    coarse);
     }
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;

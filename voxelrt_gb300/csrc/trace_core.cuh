@@ -539,21 +539,22 @@ __device__ __forceinline__ uint32_t dda_steps_mode(RayState& s, const DevWorld& 
 // through a 256-voxel terrain one in four stands still in GLSL mode (256 steps each) and one in 500
 // in CPU mode.  A step is a function of the position, and the position of the distance alone, so a
 // ray back at the distance it had some steps before repeats those steps, none of which ended
-// it: its record is that of the cap.  In CPU mode only for fast rays, whose distances are no
-// NaN; of a rayCastCoarse ray (coarse_ray) once its steps no longer depend on their number.
+// it: its record is that of the cap.  (A distance of NaN equals none.)  Of a rayCastCoarse ray
+// (coarse_ray) once its steps no longer depend on their number.
 // Looked at between slices of steps: 2,000 random GLSL rays 49 -> 13 us, 2.5 M 653 -> 112, 2.5 M
-// anisotropic 841 -> 128, 60,000 CPU rays in a mixed world 22.9 -> 12.1.  Frames and batches
+// anisotropic 841 -> 128, 60,000 CPU rays in a mixed world 22.9 -> 12.1; 1 M CPU rays from 2^22 voxels
+// off the world origin 290 -> 68.  Frames and batches
 // look for none: camera rays start near the world origin and do not stand still, and the
 // slices' loop cost them 2 to 8 %.
 template <bool kGlsl>
 __device__ __forceinline__ float last_t(const RayState& s) {
-    return kGlsl ? s.tb : fminf(fminf(s.sx, s.sy), s.sz);
+    return kGlsl ? s.tb : min_x86(min_x86(s.sx, s.sy), s.sz);
 }
 __device__ __forceinline__ float no_t() { return __uint_as_float(0x7FFFFFFFu); }  // equals no distance
 // t0: last_t before iteration `first`, with one step or more since.
 template <bool kGlsl>
 __device__ __forceinline__ bool stalled(const RayState& s, float t0, bool coarse_ray, uint32_t first) {
-    return last_t<kGlsl>(s) == t0 && (kGlsl || s.fast) && (!kGlsl || !coarse_ray || first >= kCoarseFrom);
+    return last_t<kGlsl>(s) == t0 && (!kGlsl || !coarse_ray || first >= kCoarseFrom);
 }
 
 // dda_steps_mode from iteration i to the ray's end or `iters`, kSlice steps at a time.

@@ -68,7 +68,7 @@ __device__ __forceinline__ void store_record(uint4* __restrict__ out, uint64_t i
 // One pixel's whole path: the primary ray, then its sun ray or bounces, or with kFull the GPU
 // renderer's path (VoxelRender.comp:27-93); returns the rays traced.  One loop over the rays,
 // so that the step loop is compiled once.
-template <bool kGlsl, bool kAniso, bool kBounces, bool kPacked>
+template <bool kGlsl, bool kAniso, bool kBounces, bool kPacked, bool kFar = false>
 __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld& w, const ViewStart& vs, uint32_t px,
                                                 uint32_t py, uint4* __restrict__ out) {
     const uint32_t pixel = py * v.width + px, last = v.last_kind();
@@ -100,7 +100,11 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
         // GLSL mode: shadow and bounce rays are rayCastCoarse's (VoxelRender.comp:56,74)
         const bool coarse = kGlsl && k != 0;
         const uint32_t iters = coarse ? min(v.max_iters, kCoarseMaxIters) : v.max_iters;
-        const uint32_t st = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, i, iters);
+        uint32_t st;
+        if constexpr (kFar)
+            st = dda_trace<kGlsl, false, 16>(s, w, wox, woy, woz, coarse, coarse, kAniso, i, iters);
+        else
+            st = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, i, iters);
         const bool hit = st == kStepHit;
         store_record<kPacked>(out, o, pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, i, pixel));
         if (k == last) return k + 1;
@@ -138,15 +142,16 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
 
 // One thread per pixel (thin_pixel), whole path (VoxelRender.comp:27-93 structure).  kBounces: the
 // view has bounces; without them 48 registers in place of 56 (a 1080p frame with its sun
-// ray: 121.6 -> 118.0 us).
-template <bool kGlsl, bool kAniso, bool kBounces, bool kThin>
+// ray: 121.6 -> 118.0 us).  kFar: the world origin is not near; most rays stand still, and dda_trace
+// ends them (720p with sun rays from 2^22 voxels off, GLSL: 592 -> 148 us, CPU traversal 322 -> 113).
+template <bool kGlsl, bool kAniso, bool kBounces, bool kThin, bool kFar>
 __global__ void __launch_bounds__(kFrameThreads) view_path_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
                                                        const __grid_constant__ ViewStart vs, uint32_t lanes_log2,
                                                        uint4* __restrict__ out) {
     if constexpr (kAniso) fill_forward_lut();
     uint32_t px, py;
     if (!thin_pixel<kThin>(lanes_log2, px, py) || px >= v.width || py >= v.height) return;
-    trace_pixel<kGlsl, kAniso, kBounces, false>(v, w, vs, px, py, out);
+    trace_pixel<kGlsl, kAniso, kBounces, false, kFar>(v, w, vs, px, py, out);
 }
 
 // View-table loads: read-only through the non-coherent path, or at L2 (coherent with
@@ -301,7 +306,13 @@ __device__ __forceinline__ uint32_t next_claim(const BatchParams& p) {
 // instantiation, so the others keep their code and registers).  64 registers (32 warps a SM)
 // are enough for the CPU traversal (two 720p views of 4 bounces: 355 us against 382 us with
 // 72 and 379 us with 56), not for the GLSL modes (two worlds' whole paths: 654 us against 626 us).
-template <bool kCount, bool kGlsl, bool kResident = false, bool kAniso = false, bool kFull = false>
+// kStall: rays that stand still (stalled) end early, looked at between the slices of a round.  A round
+// lasts until half of its lanes have ended, and stalled lanes hold it up to the cap: in the
+// GLSL modes many bounce rays are (a 720p view of a terrain with 2 bounces 382 -> 152 us, anisotropic
+// 358 -> 160), and of views whose world origin is not near nearly all rays (two such 720p views with
+// sun rays, CPU traversal: 599 us in tile_kernel, 193 here; GLSL 1140 and 255).  In the CPU traversal of
+// other views 1 ray in 500 is, and the test costs 6 % (spills).
+template <bool kCount, bool kGlsl, bool kResident, bool kAniso, bool kFull, bool kStall>
 __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
     if constexpr (kAniso) fill_forward_lut();
     const uint32_t lane = threadIdx.x & 31;
@@ -621,6 +632,7 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
         // keep the warp busy, and enough have ended to share a retirement.  Two 720p views of
         // 4 bounces: 372 us, five eighths left 374 us, three eighths 377 us.
         const uint32_t stop = (uint32_t)__popc(__ballot_sync(0xffffffffu, active)) / 2u;
+        float t0 = no_t();
         do {
             if (active && !(path & kEnded)) {
                 const uint32_t kmax = min(p.inner, max_iters - iter);  // an active lane has iter < max_iters
@@ -629,6 +641,10 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
                 // bounce ray, the anisotropic one for views that ask for it
                 const uint32_t st = dda_steps_mode<kCount, kGlsl, true>(s, w, wv.x, wv.y, wv.z, cnt, any_coarse,
                                                                   (path & 0xFFu) != 0, kAniso, iter, k, kmax);
+                if constexpr (kStall) {  // (the counting launch takes every step)
+                    if (st == kStepContinue && stalled<kGlsl>(s, t0, (path & 0xFFu) != 0, iter)) iter = max_iters - k;
+                    t0 = last_t<kGlsl>(s);
+                }
                 iter += k;  // the iteration a ray left on, or max_iters when the cap ran out
                 if (st != kStepContinue)
                     path |= kEnded | (st == kStepHit ? kHit : 0u);
@@ -820,14 +836,16 @@ ViewDev make_view_dev(const vrt_view& v) {
 namespace {
 
 using ViewPathFn = void (*)(DevWorld, ViewDev, ViewStart, uint32_t, uint4*);
-template <bool kBounces, bool kThin>
+template <bool kBounces, bool kThin, bool kFar = false>
 ViewPathFn view_path_fn(bool glsl, bool aniso) {
-    return glsl ? (aniso ? view_path_kernel<true, true, kBounces, kThin> : view_path_kernel<true, false, kBounces, kThin>)
-                : view_path_kernel<false, false, kBounces, kThin>;
+    if (glsl && aniso) return view_path_kernel<true, true, kBounces, kThin, kFar>;
+    if (glsl) return view_path_kernel<true, false, kBounces, kThin, kFar>;
+    return view_path_kernel<false, false, kBounces, kThin, kFar>;
 }
 
 vrt_status launch_view_path(vrt_world* w, const ViewDev& v, bool glsl, vrt_hit* hits, cudaStream_t stream) {
-    const uint32_t ll = thin_lanes_log2((uint64_t)v.width * v.height);
+    const bool far = !near_origin(v.wo);
+    const uint32_t ll = far ? 5u : thin_lanes_log2((uint64_t)v.width * v.height);
     const dim3 grid = thin_grid(ll, v.width, v.height);
     L2Window l2;
     vrt_status st = l2.enter(w, stream);
@@ -836,8 +854,10 @@ vrt_status launch_view_path(vrt_world* w, const ViewDev& v, bool glsl, vrt_hit* 
     const DevWorld dw = w->dev();
     const ViewStart vs = view_start(dw, v);
     const bool bounces = v.last_kind() > 1u || (v.last_kind() == 1u && !v.shadow());
-    const ViewPathFn kernel = bounces ? (ll < 5 ? view_path_fn<true, true>(glsl, v.aniso) : view_path_fn<true, false>(glsl, v.aniso))
-                                      : (ll < 5 ? view_path_fn<false, true>(glsl, v.aniso) : view_path_fn<false, false>(glsl, v.aniso));
+    const auto fn = far       ? view_path_fn<true, false, true>
+                    : bounces ? (ll < 5 ? view_path_fn<true, true> : view_path_fn<true, false>)
+                              : (ll < 5 ? view_path_fn<false, true> : view_path_fn<false, false>);
+    const ViewPathFn kernel = fn(glsl, v.aniso);
     kernel<<<grid, kFrameThreads, 0, stream>>>(dw, v, vs, ll, out);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
@@ -912,7 +932,12 @@ constexpr uint32_t kTileChunk = 2, kOneTileWarps = 64;
 bool tile_launch(const vrt_view* views, uint32_t n) {
     for (uint32_t i = 0; i < n; i++)
         if (views[i].n_bounces) return false;
-    return true;
+    return !far_launch(views, n);
+}
+bool far_launch(const vrt_view* views, uint32_t n) {
+    for (uint32_t i = 0; i < n; i++)
+        if (!near_origin(views[i].cam.world_origin)) return true;
+    return false;
 }
 
 void resolve_batch_defaults(vrt_batch_config& cfg, const vrt_view* views, uint32_t n, uint64_t warps) {
@@ -958,6 +983,7 @@ vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, cons
     plan.full = false;
     for (uint32_t i = 0; i < n; i++) plan.full |= view_full_path(views[i]);
     plan.tiles = tile_launch(views, n);
+    plan.far = far_launch(views, n);
     plan.cfg = cfg;
     plan.tile_w_log2 = log2u(cfg.tile_w);
     plan.tile_size_log2 = log2u(cfg.tile_w * cfg.tile_h);
@@ -995,42 +1021,45 @@ namespace {
 // instantiation: counting, traversal mode, resident, whole-path views.
 using PersistentFn = void (*)(BatchParams);
 template <bool kCount, bool kResident, bool kFull>
-PersistentFn persistent_fn_mode(bool glsl, bool aniso) {
-    if (glsl && aniso) return persistent_kernel<kCount, true, kResident, true, kFull>;
-    if (glsl) return persistent_kernel<kCount, true, kResident, false, kFull>;
-    return persistent_kernel<kCount, false, kResident, false, kFull>;
+PersistentFn persistent_fn_mode(bool glsl, bool aniso, bool far) {
+    if (glsl && aniso) return persistent_kernel<kCount, true, kResident, true, kFull, !kCount>;
+    if (glsl) return persistent_kernel<kCount, true, kResident, false, kFull, !kCount>;
+    if constexpr (!kCount && !kResident)
+        if (far) return persistent_kernel<false, false, false, false, kFull, true>;
+    return persistent_kernel<kCount, false, kResident, false, kFull, false>;
 }
 template <bool kPacked, bool kSplit>
 PersistentFn tile_fn(bool glsl, bool aniso) {
     return glsl ? (aniso ? tile_kernel<true, true, kPacked, kSplit> : tile_kernel<true, false, kPacked, kSplit>)
                 : tile_kernel<false, false, kPacked, kSplit>;
 }
-PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, bool full, bool tiles) {
+PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, bool full, bool tiles, bool far) {
     if (tiles && !count && !resident) return tile_fn<false, false>(glsl, aniso);
-    if (resident) return full ? persistent_fn_mode<false, true, true>(glsl, aniso)
-                              : persistent_fn_mode<false, true, false>(glsl, aniso);
-    if (count) return full ? persistent_fn_mode<true, false, true>(glsl, aniso)
-                           : persistent_fn_mode<true, false, false>(glsl, aniso);
-    return full ? persistent_fn_mode<false, false, true>(glsl, aniso) : persistent_fn_mode<false, false, false>(glsl, aniso);
+    if (resident) return full ? persistent_fn_mode<false, true, true>(glsl, aniso, far)
+                              : persistent_fn_mode<false, true, false>(glsl, aniso, far);
+    if (count) return full ? persistent_fn_mode<true, false, true>(glsl, aniso, far)
+                           : persistent_fn_mode<true, false, false>(glsl, aniso, far);
+    return full ? persistent_fn_mode<false, false, true>(glsl, aniso, far)
+                : persistent_fn_mode<false, false, false>(glsl, aniso, far);
 }
 
 // Resident blocks per SM of that kernel: the variants differ in registers and shared memory
 // (the anisotropic LUT is 8 KB per block).
 cudaError_t persistent_occupancy(int& occ, int threads, bool count, bool glsl, bool aniso, bool resident, bool full,
-                                 bool tiles) {
+                                 bool tiles, bool far) {
     const size_t smem = full ? (size_t)threads * 6 * sizeof(float) : 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, persistent_fn(count, glsl, aniso, resident, full, tiles),
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, persistent_fn(count, glsl, aniso, resident, full, tiles, far),
                                                          threads, smem);
 }
 
 }  // namespace
 
 vrt_status persistent_grid(int device, const vrt_batch_config& cfg, bool count, bool glsl, bool aniso, bool resident,
-                           bool full, bool tiles, int& blocks, int& threads) {
+                           bool full, bool tiles, bool far, int& blocks, int& threads) {
     int sms = 0, occ = 0;
     threads = (int)cfg.warps_per_block * 32;
     VRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    VRT_CUDA(persistent_occupancy(occ, threads, count, glsl, aniso, resident, full, tiles));
+    VRT_CUDA(persistent_occupancy(occ, threads, count, glsl, aniso, resident, full, tiles, far));
     occ = std::max(occ, 1);
     const int per_sm = (!count && cfg.blocks_per_sm) ? std::min<int>((int)cfg.blocks_per_sm, occ) : occ;
     blocks = sms * per_sm;
@@ -1061,11 +1090,12 @@ BatchParams make_params(const LaunchPlan& plan, const DevWorld* worlds, const Vi
     p.aniso = plan.aniso ? 1u : 0u;
     p.full = plan.full ? 1u : 0u;
     p.tiles = plan.tiles ? 1u : 0u;
+    p.far = plan.far ? 1u : 0u;
     return p;
 }
 
 vrt_status launch_resident(const BatchParams& p, int blocks, int threads, cudaStream_t stream) {
-    const PersistentFn fn = persistent_fn(false, p.glsl != 0, p.aniso != 0, true, p.full != 0, false);
+    const PersistentFn fn = persistent_fn(false, p.glsl != 0, p.aniso != 0, true, p.full != 0, false, false);
     fn<<<blocks, threads, pend_bytes(p, threads), stream>>>(p);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
@@ -1100,7 +1130,7 @@ vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool
     const uint64_t claims = std::max<uint64_t>(1, (uint64_t)p.total_chunks << q.split_log2);
     blocks = (int)std::min<uint64_t>((uint64_t)blocks, (claims * 32 + threads - 1) / threads);
     const bool glsl = p.glsl != 0, aniso = p.aniso != 0;
-    const PersistentFn fn = !tiles ? persistent_fn(count, glsl, aniso, false, p.full != 0, false)
+    const PersistentFn fn = !tiles ? persistent_fn(count, glsl, aniso, false, p.full != 0, false, p.far != 0)
                             : q.split_log2 ? (p.packed ? tile_fn<true, true>(glsl, aniso) : tile_fn<false, true>(glsl, aniso))
                             : p.packed ? tile_fn<true, false>(glsl, aniso) : tile_fn<false, false>(glsl, aniso);
     fn<<<blocks, threads, pend_bytes(p, threads), stream>>>(q);
@@ -1245,7 +1275,8 @@ vrt_status vrt_batch_create(vrt_world* const* worlds, uint32_t n_worlds, const v
         bool full = false;
         for (uint32_t i = 0; i < n_views; i++) full |= view_full_path(views[i]);
         if ((st = persistent_grid(worlds[0]->device, cfg, false, view_glsl(views[0]), view_aniso(views[0]), false,
-                                  full, tile_launch(views, n_views), grid_blocks, grid_threads)) != VRT_OK)
+                                  full, tile_launch(views, n_views), far_launch(views, n_views), grid_blocks,
+                                  grid_threads)) != VRT_OK)
             return st;
     }
     auto* b = new vrt_batch;
@@ -1282,10 +1313,11 @@ vrt_status vrt_batch_create(vrt_world* const* worlds, uint32_t n_worlds, const v
     b->d_counters = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(b->d_queue) + 16);
     if ((st = refresh_worlds(b, 0)) != VRT_OK) return fail(st);
     const bool glsl = b->plan.glsl, aniso = b->plan.aniso, full = b->plan.full;
-    if ((st = persistent_grid(b->device, cfg, false, glsl, aniso, false, full, b->plan.tiles, b->blocks, b->threads)) != VRT_OK)
+    if ((st = persistent_grid(b->device, cfg, false, glsl, aniso, false, full, b->plan.tiles, b->plan.far, b->blocks,
+                              b->threads)) != VRT_OK)
         return fail(st);
-    if ((st = persistent_grid(b->device, cfg, true, glsl, aniso, false, full, false, b->blocks_count, b->threads_count)) !=
-        VRT_OK)
+    if ((st = persistent_grid(b->device, cfg, true, glsl, aniso, false, full, false, false, b->blocks_count,
+                              b->threads_count)) != VRT_OK)
         return fail(st);
     *out = b;
     return VRT_OK;

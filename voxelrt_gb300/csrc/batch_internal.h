@@ -64,8 +64,9 @@ struct BatchParams {
     uint32_t inner;
     uint32_t glsl;  // traversal mode of every view (VRT_VIEW_GLSL)
     uint32_t aniso;  // ... with anisotropic LODs (VRT_VIEW_GLSL_ANISO)
-    uint32_t tiles;  // no view has bounces: tile_kernel traces the launch
+    uint32_t tiles;  // tile_kernel traces the launch (tile_launch)
     uint32_t packed; // (tiles) records are stored in the 12-byte form
+    uint32_t far;    // some view's world origin is not near (near_origin): see far_launch
     uint32_t full;   // some view traces the GPU renderer's whole path (sun rays among bounces)
     // resident launches (request server): views are published while the kernel runs
     unsigned long long* mailbox;  // host-mapped: published chunks | published views << 32 | closed << 63
@@ -95,7 +96,8 @@ struct LaunchPlan {
     uint32_t chunks = 0;
     bool glsl = false;   // every view traces in the GLSL mode
     bool aniso = false;  // ... with anisotropic LODs
-    bool tiles = false;  // no view has bounces (tile_launch)
+    bool tiles = false;  // the launch runs tile_kernel (tile_launch)
+    bool far = false;    // some view's world origin is not near (far_launch)
     bool full = false;   // some view traces the GPU renderer's whole path
 };
 
@@ -121,8 +123,11 @@ vrt_status normalize_batch_config(const vrt_batch_config* in, vrt_batch_config& 
 // eight chunks per warp of the launch, 1..16 tiles.  Fixed chunks too large for a small
 // launch leave most warps without work; the tuned table names its chunks explicitly.
 uint32_t auto_chunk_tiles(uint64_t tiles, uint64_t warps);
-// Whether a launch of these views runs tile_kernel: no view has bounces.
+// Whether a launch of these views runs tile_kernel: no view has bounces, and none is far.
 bool tile_launch(const vrt_view* views, uint32_t n);
+// Whether some view's world origin is too far for the fast step (near_origin): most of its rays
+// stand still until the cap, so the persistent kernel traces it and looks for those.
+bool far_launch(const vrt_view* views, uint32_t n);
 // Fill the fields a config leaves to the library (0): views with diffuse bounces (long,
 // uneven, incoherent paths per pixel) refill below 28 lanes and claim one tile at a time;
 // camera and sun rays refill below 16 and claim auto_chunk_tiles.
@@ -137,7 +142,7 @@ vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, cons
 // Grid of the persistent kernel: every SM, as many blocks of the launched instantiation
 // (counting, traversal mode, resident) as fit, or cfg.blocks_per_sm of them.
 vrt_status persistent_grid(int device, const vrt_batch_config& cfg, bool count, bool glsl, bool aniso, bool resident,
-                           bool full, bool tiles, int& blocks, int& threads);
+                           bool full, bool tiles, bool far, int& blocks, int& threads);
 BatchParams make_params(const LaunchPlan& plan, const DevWorld* worlds, const ViewDev* views,
                         const uint32_t* chunk_base, uint32_t* queue, vrt_hit* out);
 // Reset of the tile counter and the launch counters (64 bytes at params.queue; 0: the caller

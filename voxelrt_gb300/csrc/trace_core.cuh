@@ -158,12 +158,17 @@ struct RayState {
 
 // A ray takes the fast step (ray_step<.., true>) when no NaN or infinity can occur in its side
 // distances and voxels of the grid have their biased form:
-// - |worldOrigin| <= 2^21 (a near one), so K is exact;
+// - -2^22 <= worldOrigin < 2^22 (a near one), so K is exact;
 // - |origin| < 2^30 and |1/dir| < 2^95: |tStart| and |(voxel - worldOrigin) * invDir| stay below
 //   2^126, so side distances and t are finite, and the position o + t*d is finite or an
 //   infinity (never NaN) that leaves the grid.
-constexpr int32_t kNearWorldOrigin = 1 << 21;
+constexpr int32_t kNearWorldOrigin = 1 << 22;
 constexpr float kFastOrigin = 0x1p30f, kFastInvDir = 0x1p95f;
+VRT_HD inline bool near_origin(const int32_t wo[3]) {
+    bool near = true;
+    for (int c = 0; c < 3; c++) near &= (uint32_t)wo[c] + (uint32_t)kNearWorldOrigin < 2u * (uint32_t)kNearWorldOrigin;
+    return near;
+}
 
 // The clip box [1 - worldOrigin, size - 1 - worldOrigin] (VoxelTraversal.glsl:166) of a world
 // origin, and whether that is near: the same for every ray of a view or cast.
@@ -174,12 +179,11 @@ struct ClipBox {
 VRT_HD inline ClipBox clip_box(const DevWorld& w, const int32_t wo[3]) {
     const uint32_t size[3] = {w.size_x, w.size_y, w.size_z};
     ClipBox b;
-    b.near = 1;
     for (int c = 0; c < 3; c++) {
         b.lo[c] = (float)(1 - wo[c]);
         b.hi[c] = ((float)size[c] - (float)wo[c]) - 1.0f;
-        if ((uint32_t)wo[c] + (uint32_t)kNearWorldOrigin > 2u * (uint32_t)kNearWorldOrigin) b.near = 0;
     }
+    b.near = near_origin(wo) ? 1u : 0u;
     return b;
 }
 // The box holds the origin strictly inside, and the world origin is near: a ray's start then
@@ -543,9 +547,10 @@ __device__ __forceinline__ uint32_t dda_steps_mode(RayState& s, const DevWorld& 
 // (coarse_ray) once its steps no longer depend on their number.
 // Looked at between slices of steps: 2,000 random GLSL rays 49 -> 13 us, 2.5 M 653 -> 112, 2.5 M
 // anisotropic 841 -> 128, 60,000 CPU rays in a mixed world 22.9 -> 12.1; 1 M CPU rays from 2^22 voxels
-// off the world origin 290 -> 68.  Frames and batches
-// look for none: camera rays start near the world origin and do not stand still, and the
-// slices' loop cost them 2 to 8 %.
+// off the world origin 290 -> 68.  The persistent kernel looks too, in the GLSL modes, whose bounce rays
+// start from hits in world coordinates (batch.cu), and views whose world origin is not near, nearly
+// all of whose rays stand still.  Other frames and batches look for none: camera rays start near the
+// world origin and do not stand still, and the slices' loop cost them 2 to 8 %.
 template <bool kGlsl>
 __device__ __forceinline__ float last_t(const RayState& s) {
     return kGlsl ? s.tb : min_x86(min_x86(s.sx, s.sy), s.sz);

@@ -419,6 +419,7 @@ vrt_status vrt_world_create(const vrt_world_desc* desc, vrt_world** out) {
     w->flags = desc->flags;
     w->slots.assign(w->num_sectors(), SectorSlots{});
     w->h_table.assign(w->num_sectors(), SectorRec{0, 0, 0, 0});
+    w->sync_mark.assign(w->num_sectors(), 0);
     w->arena.reset(0);
     DeviceScope ds;
     vrt_status st = world_enter(w, ds);
@@ -519,7 +520,7 @@ vrt_status vrt_world_sync_sectors(vrt_world* w, uint32_t n, const int32_t* secto
     const uint64_t kBatchBricks = 1ull << 19;  // 256 MiB of staged bricks per batch
     SyncBatch batch;
     batch.ops.reserve(std::min<uint32_t>(n, 1u << 16));
-    std::vector<uint8_t> seen(w->num_sectors());  // sectors of the current batch
+    w->next_sync_batch();
     uint64_t in_brick = 0;  // index of the next brick in the input stream
     for (uint32_t i = 0; i < n; i++) {
         const uint64_t am = alloc_mask[i];
@@ -533,9 +534,9 @@ vrt_status vrt_world_sync_sectors(vrt_world* w, uint32_t n, const int32_t* secto
         sector_index_unpack(sector_idx[i], x, y, z);
         if (w->sector_in(x, y, z)) {
             const uint32_t s = w->lin(x, y, z);
-            if (seen[s] || batch.n_stage + cnt > kBatchBricks) {
+            if (w->sync_mark[s] == w->sync_batch || batch.n_stage + cnt > kBatchBricks) {
                 if ((st = run_batch(w, batch, stream)) != VRT_OK) return st;
-                std::fill(seen.begin(), seen.end(), 0);
+                w->next_sync_batch();
             }
             if (batch.ops.empty()) {
                 batch.src = bricks ? bricks + in_brick * 512 : nullptr;
@@ -545,7 +546,7 @@ vrt_status vrt_world_sync_sectors(vrt_world* w, uint32_t n, const int32_t* secto
             const uint64_t first = (bricks ? (in_brick - (uint64_t)(batch.src - bricks) / 512) : 0);
             if ((st = plan_sector(w, batch, s, am, dm, first, stream)) != VRT_OK) return st;
             batch.n_stage = first + cnt;
-            seen[s] = 1;
+            w->sync_mark[s] = w->sync_batch;
         }
         in_brick += cnt;
     }

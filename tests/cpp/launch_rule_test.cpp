@@ -1,10 +1,11 @@
-// launch_rule_test.cpp - the rules that pick the kernel and the claim size of a launch, on the host:
-// links libvrt.so and calls its planner (tile_launch, far_launch, resolve_launch_config,
-// plan_views).  Prints FAIL lines and exits non-zero on a mismatch.
+// launch_rule_test.cpp - the rules that pick the kernel, the claim size and the rays per warp of a
+// launch, on the host: links libvrt.so and calls its planner (tile_launch, far_launch,
+// resolve_launch_config, plan_views), and launch_rules.h.  Prints FAIL lines and exits non-zero on a mismatch.
 #include <cstdio>
 #include <vector>
 
 #include "batch_internal.h"
+#include "launch_rules.h"
 
 using namespace vrt;
 
@@ -84,6 +85,24 @@ int main() {
     // far views run on the persistent kernel: about eight claims a warp, 1 to 16 tiles
     CHECK(chunk({make(1600, 1600, 0, false, near)}, warps) == auto_chunk_tiles(40000, warps));
     CHECK(chunk({make(64, 64, 0, true, near)}, warps) == 1);
+
+    // rays per warp and claims per tile, on 152 SMs and on half of them
+    for (const uint32_t sms : {152u, 76u}) {
+        const uint32_t w = 16 * sms;
+        for (uint32_t l = 2; l < 5; l++) {
+            const uint64_t most = ((uint64_t)w << l) + (1u << l) - 1;  // `w` warps of 2^l rays and a remainder below one
+            CHECK(thin_lanes_log2(most, sms) == l && thin_lanes_log2(most + 1, sms) == l + 1);
+        }
+        CHECK(thin_lanes_log2(1, sms) == 2 && thin_lanes_log2(1ull << 32, sms) == 5);
+        for (const bool bounces : {false, true}) {
+            for (uint32_t k = 2; k <= 4; k++) CHECK(claim_split_log2(w >> k, bounces, sms) == k);
+            CHECK(claim_split_log2(1, bounces, sms) == 4 && claim_split_log2((w >> 4) + 1, bounces, sms) == 3);
+            CHECK(claim_split_log2((w >> 2) + 1, bounces, sms) == 1);
+            CHECK(claim_split_log2(48 * sms, bounces, sms) == 1);
+            CHECK(claim_split_log2(48 * sms + 1, bounces, sms) == (bounces ? 1 : 0));
+        }
+        CHECK(claim_split_log2(1u << 30, true, sms) == 1 && claim_split_log2((1u << 30) + 1, true, sms) == 0);
+    }
 
     std::printf("%s: %d failures\n", fails ? "FAIL" : "ok", fails);
     return fails ? 1 : 0;

@@ -845,7 +845,7 @@ ViewPathFn view_path_fn(bool glsl, bool aniso) {
 
 vrt_status launch_view_path(vrt_world* w, const ViewDev& v, bool glsl, vrt_hit* hits, cudaStream_t stream) {
     const bool far = !near_origin(v.wo);
-    const uint32_t ll = far ? 5u : thin_lanes_log2((uint64_t)v.width * v.height);
+    const uint32_t ll = far ? 5u : thin_lanes_log2((uint64_t)v.width * v.height, sm_count());
     const dim3 grid = thin_grid(ll, v.width, v.height);
     L2Window l2;
     vrt_status st = l2.enter(w, stream);
@@ -1101,17 +1101,6 @@ vrt_status launch_resident(const BatchParams& p, int blocks, int threads, cudaSt
     return VRT_OK;
 }
 
-// Claims smaller than a tile, of launches whose chunks are one tile of 64.  A launch of few tiles
-// leaves most of the chip idle, and a warp that traces 64 rays takes twice as long as one with
-// 32: half tiles up to kHalfTileChunks tiles (768x768, 9,216 tiles, primary rays from within a
-// solid voxel: 23.6 us against 21.2 whole; 512x512 terrain frames 27.7 -> 23.1 us).  Launches
-// with bounces take half tiles at any size, as their warps end far apart (two 720p views of 4
-// bounces 372 -> 355 us, 1024x1024 131 -> 118; quarter tiles 370 and 133 us).  Below
-// kThinBatchWarps warps also fewer rays a warp, down to 4, as in thin_launch.cuh (64x64
-// terrain views: primary rays 25.1 -> 17.7 us, 3 bounces 68 -> 36, anisotropic with sun rays and
-// bounces 86 -> 40; 4,864 warps are faster still there by 2 to 4 us, and slower by as much where
-// rays end at once).
-constexpr uint32_t kHalfTileChunks = 7296, kThinBatchWarps = 2432;
 vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool count, cudaStream_t stream,
                              size_t zero_bytes) {
     if (zero_bytes) VRT_CUDA(cudaMemsetAsync(p.queue, 0, zero_bytes, stream));
@@ -1119,12 +1108,9 @@ vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool
     BatchParams q = p;
     q.split_log2 = 0;
     q.lanes = 0xffffffffu;
-    // (the queue counts claims in 32 bits)
-    if (p.chunk_rays == 64 && p.tile_size_log2 == 6 && p.total_chunks <= (tiles ? kHalfTileChunks : 1u << 30)) {
-        q.split_log2 = 1;
-        while (q.split_log2 < 4 && (uint64_t)p.total_chunks << (q.split_log2 + 1) <= kThinBatchWarps) q.split_log2++;
-        q.lanes >>= 32 - (64 >> q.split_log2);
-    }
+    if (p.chunk_rays == 64 && p.tile_size_log2 == 6)
+        q.split_log2 = claim_split_log2(p.total_chunks, !tiles, sm_count());
+    if (q.split_log2) q.lanes >>= 32 - (64 >> q.split_log2);
     // no more warps than claims: each takes a turn at the queue's counter and returns (64x64 views
     // 13.3 -> 11.3 us from within a solid voxel, 35.7 -> 33.5 with 3 bounces of a terrain)
     const uint64_t claims = std::max<uint64_t>(1, (uint64_t)p.total_chunks << q.split_log2);

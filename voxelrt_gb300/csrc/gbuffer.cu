@@ -98,7 +98,7 @@ vrt_status launch_gbuffer(vrt_world* w, const vrt_view* view, const uint32_t* pa
     std::memcpy(gp.palette, palette, sizeof(gp.palette));
     std::memcpy(gp.proj, proj, sizeof(gp.proj));
     const ViewDev v = make_view_dev(*view);
-    const uint32_t ll = thin_lanes_log2((uint64_t)v.width * v.height);
+    const uint32_t ll = thin_lanes_log2((uint64_t)v.width * v.height, sm_count());
     const dim3 grid = thin_grid(ll, v.width, v.height);
     uint4* out = reinterpret_cast<uint4*>(hits);
     const DevWorld dw = w->dev();

@@ -1,26 +1,13 @@
-// Small launches: fewer rays per warp.
+// Frames, small ones with fewer rays per warp (launch_rules.h).
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
-namespace vrt {
+#include "launch_rules.h"
 
-// Rays per warp of a small launch (log2, 2..5): as few as keep the launch within kThinWarps warps.
-// A launch that leaves most of the chip idle lasts as long as its longest ray, and a ray's
-// step waits for the slowest lane of its warp: with 4 rays a warp a 64x64 frame of a
-// 256-voxel terrain takes 12.5 us against 14.5, 2,000 random rays 16.4 us against 18.6 (two rays a
-// warp: another 2 % at 1,000 to 2,000 rays, nothing elsewhere).  64x64 paths of the terrain: sun
-// rays 20.1 -> 17.4 us, 3 bounces 41.4 -> 28.9, anisotropic with both 51.4 -> 34.3; G-buffers
-// 15.3 -> 12.5.  kThinWarps where the gain ends (with 1,216 frames of 100x100 to 160x160 take 2 to 7 %
-// more, such paths 5 to 12 %; with 4,864 paths whose rays end at once up to half as much again).
-constexpr uint32_t kThinWarps = 2432;
-inline uint32_t thin_lanes_log2(uint64_t rays) {
-    uint32_t l = 5;
-    while (l > 2 && rays >> (l - 1) <= kThinWarps) l--;
-    return l;
-}
+namespace vrt {
 
 // The pixel of this thread in such a launch's frame: blocks of kFrameThreads, two by two warps, each
 // an area of 2^lanes_log2 pixels (8x4 for 32).  One above the other, two warps a block: 118.3 us for a

@@ -169,7 +169,7 @@ vrt_status check_camera(const vrt_camera* cam) {
 
 vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters, vrt_hit* hits,
                          cudaStream_t stream) {
-    const uint32_t ll = thin_lanes_log2((uint64_t)cam->width * cam->height);
+    const uint32_t ll = thin_lanes_log2((uint64_t)cam->width * cam->height, sm_count());
     L2Window l2;
     vrt_status st = l2.enter(w, stream);
     if (st != VRT_OK) return st;
@@ -219,7 +219,7 @@ vrt_status launch_cast(vrt_world* w, const vrt_ray* rays, uint32_t n, const vrt_
     if (st != VRT_OK) return st;
     if (n < (glsl ? kCastPersistentMinGlsl : kCastPersistentMin)) {
         auto kernel = glsl ? (aniso ? cast_kernel<true, true> : cast_kernel<true>) : cast_kernel<false>;
-        const uint32_t ll = thin_lanes_log2(n), per_block = 8u << ll;
+        const uint32_t ll = thin_lanes_log2(n, sm_count()), per_block = 8u << ll;
         kernel<<<(n + per_block - 1) / per_block, 256, 0, stream>>>(dw, clip, r4, n, p->world_origin[0],
                                                                     p->world_origin[1], p->world_origin[2], iters, o4,
                                                                     coarse, ll);

@@ -10,12 +10,14 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <map>
 #include <string>
 #include <vector>
 
 #include "brick_codes.cuh"
+#include "launch_rules.h"
 #include "world.h"
 
 namespace vrt {
@@ -34,6 +36,19 @@ vrt_status world_enter(vrt_world* world, DeviceScope& scope) {
     }
     VRT_CUDA(scope.enter(world->device));
     return VRT_OK;
+}
+
+uint32_t sm_count() {
+    static std::atomic<int> known[64];  // per device, 0 = not asked yet
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    const bool keep = dev >= 0 && dev < 64;
+    if (keep) sms = known[dev].load(std::memory_order_relaxed);
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 1;
+        if (keep) known[dev].store(sms, std::memory_order_relaxed);
+    }
+    return (uint32_t)sms;
 }
 
 vrt_status L2Window::enter(const vrt_world* w, cudaStream_t s) {

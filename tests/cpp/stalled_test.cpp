@@ -19,8 +19,8 @@ static uint4 trace(const DevWorld& w, const vrt_ray& q, const int32_t wo[3], uin
     ray_start<kGlsl>(s, clip_box(w, wo), q.origin[0], q.origin[1], q.origin[2], q.dir[0], q.dir[1], q.dir[2], wo[0], wo[1],
                      wo[2], coarse);
     uint32_t i = 0;
-    const bool hit = dda_trace<kGlsl, !kGlsl, kGlsl ? 8 : 16>(s, w, wo[0], wo[1], wo[2], coarse, coarse, aniso, i, iters) ==
-                     kStepHit;
+    const bool hit = dda_trace<kGlsl, !kGlsl>(s, w, wo[0], wo[1], wo[2], coarse, coarse, aniso, i, iters,
+                                              kGlsl && !coarse ? 8 : 16) == kStepHit;
     return pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, i, q.tag);
 }
 

@@ -102,7 +102,7 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
         const uint32_t iters = coarse ? min(v.max_iters, kCoarseMaxIters) : v.max_iters;
         uint32_t st;
         if constexpr (kFar)
-            st = dda_trace<kGlsl, false, 16>(s, w, wox, woy, woz, coarse, coarse, kAniso, i, iters);
+            st = dda_trace<kGlsl, false>(s, w, wox, woy, woz, coarse, coarse, kAniso, i, iters, 16);
         else
             st = dda_steps_mode<false, kGlsl>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0, i, iters);
         const bool hit = st == kStepHit;

@@ -49,11 +49,15 @@ __global__ void __maxnreg__(48) render_view_kernel(const __grid_constant__ DevWo
     out[pix] = pack_state<false>(s, hit_material(s, w.payload, hit), hit, i, pix);
 }
 
+// A thread per ray, stalled rays looked for every `slice` steps: 16, and 8 for GLSL rays.  For
+// rayCastCoarse's, which are looked at from iteration 31 on alone, 131,072 random rays in a mixed world
+// with 8 / 16 / 32 steps 14.6 / 14.2 / 14.1 us (14.0 without the test), 120,000 with anisotropic LODs in a
+// world with 2 % of its voxels set 35.3 / 35.3 / 41.5 us (45.6 without).
 template <bool kGlsl, bool kAniso = false>
 __global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ClipBox clip,
                                                   const float4* __restrict__ rays, uint32_t n,
                                                   int32_t wox, int32_t woy, int32_t woz, uint32_t max_iters,
-                                                  uint4* __restrict__ out, bool coarse, uint32_t lanes_log2) {
+                                                  uint4* __restrict__ out, bool coarse, uint32_t lanes_log2, uint32_t slice) {
     if constexpr (kAniso) fill_forward_lut();
     const uint32_t lane = threadIdx.x & 31;
     if (lane >> lanes_log2) return;
@@ -63,7 +67,8 @@ __global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWo
     RayState s;
     ray_start<kGlsl>(s, clip, a.x, a.y, a.z, a.w, b.x, b.y, wox, woy, woz, coarse);
     uint32_t k = 0;
-    const bool hit = dda_trace<kGlsl, !kGlsl, kGlsl ? 8 : 16>(s, w, wox, woy, woz, coarse, coarse, kAniso, k, max_iters) == kStepHit;
+    const bool hit =
+        dda_trace<kGlsl, !kGlsl>(s, w, wox, woy, woz, coarse, coarse, kAniso, k, max_iters, slice) == kStepHit;
     out[i] = pack_state<kGlsl>(s, hit_material(s, w.payload, hit), hit, k, __float_as_uint(b.z));
 }
 
@@ -222,7 +227,7 @@ vrt_status launch_cast(vrt_world* w, const vrt_ray* rays, uint32_t n, const vrt_
         const uint32_t ll = thin_lanes_log2(n, sm_count()), per_block = 8u << ll;
         kernel<<<(n + per_block - 1) / per_block, 256, 0, stream>>>(dw, clip, r4, n, p->world_origin[0],
                                                                     p->world_origin[1], p->world_origin[2], iters, o4,
-                                                                    coarse, ll);
+                                                                    coarse, ll, glsl && !coarse ? 8 : 16);
     } else {
         auto kernel = glsl ? (aniso ? cast_persistent_kernel<true, true> : cast_persistent_kernel<true>)
                            : cast_persistent_kernel<false>;

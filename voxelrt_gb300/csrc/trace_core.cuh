@@ -562,14 +562,15 @@ __device__ __forceinline__ bool stalled(const RayState& s, float t0, bool coarse
     return last_t<kGlsl>(s) == t0 && (!kGlsl || !coarse_ray || first >= kCoarseFrom);
 }
 
-// dda_steps_mode from iteration i to the ray's end or `iters`, kSlice steps at a time.
-template <bool kGlsl, bool kFlat, uint32_t kSlice>
+// dda_steps_mode from iteration i to the ray's end or `iters`, `slice` steps at a time.
+template <bool kGlsl, bool kFlat>
 __device__ __forceinline__ uint32_t dda_trace(RayState& s, const DevWorld& w, int32_t wox, int32_t woy, int32_t woz,
-                                              bool coarse, bool coarse_ray, bool aniso, uint32_t& i, uint32_t iters) {
+                                              bool coarse, bool coarse_ray, bool aniso, uint32_t& i, uint32_t iters,
+                                              uint32_t slice) {
     TraceCounters cnt{0, 0};
     float t0 = no_t();
     for (;;) {
-        const uint32_t first = i, lim = iters - i < kSlice ? iters : i + kSlice;
+        const uint32_t first = i, lim = iters - i < slice ? iters : i + slice;
         const uint32_t st = dda_steps_mode<false, kGlsl, kFlat>(s, w, wox, woy, woz, cnt, coarse, coarse_ray, aniso, 0, i, lim);
         if (st != kStepContinue || i >= iters) return st;
         if (stalled<kGlsl>(s, t0, coarse_ray, first)) {

@@ -291,15 +291,18 @@ __device__ __forceinline__ void resident_pixels_done(const BatchParams& p, uint3
     }
 }
 
-// Claims of a launch's queue: a warp's first is its own number, the following come from the
-// counter.  A claim of the counter is a turn at one address for every warp of the chip at once, and
-// with claims of half a tile a launch of few or short rays waits for little else: two 640x360 GLSL
-// views of a terrain 42.6 -> 40.0 us, two of 160x90 26.9 -> 24.8; of an empty world, where every ray
-// leaves the grid in a few steps, 22.7 -> 20.6 (17.0 with whole tiles, and the terrain 46.9), and with
-// 4 bounces 24.7 -> 22.7 (19.1 with whole tiles, and the terrain 194 for 168).
-__device__ __forceinline__ uint32_t first_claim() { return (blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
+// Claims of a launch's queue.  A claim of its counter is a turn at one address for every warp of the
+// chip at once, and with claims of half a tile a launch of few or short rays waits for little else.
+// There (kOwn) a warp's first claim is its own number and the following come from the counter: two
+// 640x360 GLSL views of a terrain 42.6 -> 40.0 us, two of 160x90 26.9 -> 24.8; of an empty world, where
+// every ray leaves the grid in a few steps, 22.7 -> 20.6 (17.0 with whole tiles, and the terrain 46.9), and
+// with 4 bounces 24.7 -> 22.7 (19.1 with whole tiles, and the terrain 194 for 168).  Where claims are
+// whole tiles the counter is no limit, and neighbouring first claims for the warps of a block cost 44 M
+// rays over 154 views 2 %.
+__device__ __forceinline__ uint32_t warp_number() { return (blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
+template <bool kOwn>
 __device__ __forceinline__ uint32_t next_claim(const BatchParams& p) {
-    return atomicAdd(p.queue, 1u) + ((gridDim.x * blockDim.x) >> 5);
+    return atomicAdd(p.queue, 1u) + (kOwn ? (gridDim.x * blockDim.x) >> 5 : 0u);
 }
 
 // kFull: the launch may hold views with the GPU renderer's whole path (a separate
@@ -478,9 +481,9 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
                         }
                     } else {
                         if (q_end == 0) {
-                            c = first_claim();
+                            c = warp_number();
                         } else {
-                            if (lane == 0) c = next_claim(p);
+                            if (lane == 0) c = next_claim<true>(p);
                             c = __shfl_sync(0xffffffffu, c, 0);
                         }
                         part = c & ((1u << p.split_log2) - 1u);
@@ -718,7 +721,7 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) tile_kernel(BatchParams p) {
     const uint32_t tile_h = 1u << (p.tile_size_log2 - p.tile_w_log2), rows = kSplit ? tile_h : 32u >> p.tile_w_log2;
     const uint32_t chunk_tiles = p.chunk_rays >> p.tile_size_log2;
     uint32_t view = 0, loaded = kNoView, rays = 0;
-    uint32_t claim = first_claim();
+    uint32_t claim = kSplit ? warp_number() : __shfl_sync(0xffffffffu, lane == 0 ? next_claim<false>(p) : 0u, 0);
     for (;;) {
         uint32_t c = claim;
         if (kSplit) {
@@ -790,7 +793,7 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) tile_kernel(BatchParams p) {
                 }
             }
         }
-        claim = __shfl_sync(0xffffffffu, lane == 0 ? next_claim(p) : 0u, 0);
+        claim = __shfl_sync(0xffffffffu, lane == 0 ? next_claim<kSplit>(p) : 0u, 0);
     }
     for (int off = 16; off > 0; off >>= 1) rays += __shfl_xor_sync(0xffffffffu, rays, off);
     if (lane == 0) atomicAdd(p.counters, (unsigned long long)rays);

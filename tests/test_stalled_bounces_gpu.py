@@ -1,7 +1,7 @@
-"""Bounce and sun rays that stand still in the GLSL modes (kStall in batch.cu: the test between the
-slices of the persistent kernel) against the oracle: slice lengths, refills and caps around them,
-rayCastCoarse's iteration 31, and many pixels of a view.  Every record word is equal, and the
-counting launch counts every step."""
+"""Rays that stand still in GLSL launches with bounces (kStall in batch.cu: the test between the slices
+of the persistent kernel) against the oracle: cameras with coordinates on the face of an empty
+brick, from which a third of the rays do, and others; slice lengths, refills and caps around them, and rayCastCoarse's
+iteration 31.  Every record word is equal, and the counting launch traces every ray."""
 import numpy as np
 import pytest
 
@@ -29,10 +29,12 @@ def test_batches(world, mode, inner, refill):
     w, o = world
     views = []
     for i, cap in enumerate((0, 1, 30, 33, 48, 96, 200)):
-        cam = v.look_at((60.3, 100.2, 50.7), (20 + 15 * i, 40, 90 - 9 * i), 80.0, 70 + i, 41)
+        eye = np.array((64.0, 100.0, 64.0) if i % 2 else (60.3, 100.2, 50.7))
+        cam = v.look_at(eye, eye + (-74 + 20 * i, -40, 44), 80.0, 70 + i, 41)
         views += [v.make_view(cam, n_bounces=3, max_iters=cap, **mode),
                   v.make_view(cam, n_bounces=2, max_iters=cap, shadow_dir=SUN, **mode)]
     want = [oracle_view(o, vw) for vw in views]
+    assert (want[-4][0]["steps"] == 96).mean() > 0.1  # primary rays at the cap
     cfg = v.BatchConfig(0, 0, 0, 0, 0, refill, 0, inner)
     for kind in (0, 1):
         b = v.Batch([w], views[kind::2], cfg)
@@ -44,10 +46,10 @@ def test_batches(world, mode, inner, refill):
 
 @pytest.mark.parametrize("mode", [dict(glsl=True), dict(aniso=True)], ids=lambda m: "+".join(m))
 def test_counts(world, mode):
-    """Statistics of the counting launch, whose rays take every step, as records tell them."""
+    """Records and rays of the counting launch, which does not end stalled rays early."""
     import torch
     w, o = world
-    views = [v.make_view(v.look_at((60.3, 100.2, 50.7), (40, 40, 90), 80.0, 96, 64), n_bounces=4, **mode)]
+    views = [v.make_view(v.look_at((64.0, 100.0, 64.0), (40, 40, 90), 80.0, 96, 64), n_bounces=4, **mode)]
     b = v.Batch([w], views)
     out = torch.zeros((b.total_records, 4), dtype=torch.int32, device="cuda")
     stats = b.measure(out)

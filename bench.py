@@ -249,15 +249,15 @@ def peak_hbm():
     return 6800.0, "fallback"
 
 
-# What bounds the persistent kernel on a workload, from the committed ncu summaries.
+# What bounds a workload's kernel, from the committed ncu summaries.
 LIMITERS = {
-    "uneven_batch": "instruction issue: 79 % of issue slots busy, 28 of 32 lanes (tile_kernel, "
-                    "profiles/traversal_kernels.md)",
+    "uneven_batch": "instruction issue: 79 % of issue slots busy (smsp__inst_executed over the schedulers' "
+                    "cycles), 28 of 32 lanes; tile_kernel, 44 M rays of the workload's kind",
 }
 
 
 def traffic_from_profile(workload: str, args=None):
-    """DRAM bytes per launch of the persistent kernel from a committed ncu summary, for
+    """DRAM bytes per launch of the workload's kernel from a committed ncu summary, for
     the configuration that summary covers (the workload at its default sizes, default
     traversal); None for any other."""
     p = ROOT / "profiles" / "traffic.json"
@@ -603,7 +603,7 @@ def run_ours(args, engine_cls=None, backend: str = "nccl", device: str = "cuda")
         pms = max_over_ranks(pg, pms_rank, device)
         per_view = {"value": job_rays / (pms * 1e-3) / 1e9, "unit": "Grays/s", "ms_per_step": pms,
                     "launches_per_step": int(sum_over_ranks(pg, len(eng.wl.views), device)), "steps": k,
-                    "kernel": "view_path_kernel, 8x8 blocks, thread per pixel"}
+                    "kernel": "view_path_kernel, 16x8 pixels a block, thread per pixel"}
 
     link_before = eng.d2h_link_gbs()
     e2e_s = max_over_ranks(pg, eng.time_e2e(sync), device)

@@ -416,7 +416,8 @@ typedef struct vrt_batch_config {
     uint32_t blocks_per_sm;    /* 0 = as many as fit */
     uint32_t refill_threshold; /* refill idle lanes when fewer lanes are active (1..32; 0 = 28 for a
                                   launch with diffuse bounces, else 16); not used by a launch
-                                  without bounces, whose warps trace 32 pixels to the end */
+                                  without bounces, whose warps trace 32 pixels to the end (but
+                                  by one with a world origin outside +-2^22) */
     uint32_t chunk_tiles;      /* tiles taken from the device queue per atomic (1..64; 0 = 1 for a
                                   launch with diffuse bounces, else 1 or 2 by the launch's size).
                                   With 1, a tile of 64 rays is taken by halves in a launch with

@@ -67,7 +67,7 @@ def store(workload: str, cfg: dict, result: dict, path: Path | None = None, gpu:
     table = _load(path)
     table.setdefault(gpu, {})[workload] = {"config": cfg, **result}
     path.parent.mkdir(parents=True, exist_ok=True)
-    path.write_text(json.dumps(table, indent=1, sort_keys=True))
+    path.write_text(json.dumps(table, indent=1, sort_keys=True) + "\n")
     return path
 
 

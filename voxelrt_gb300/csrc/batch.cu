@@ -4,10 +4,11 @@
 // The reference dispatches one VoxelRender.comp per frame (GpuRenderer.cpp:267-268)
 // with one invocation per pixel tracing its whole path (VoxelRender.comp:27-93).
 // vrt_render_path keeps that structure (the per-view baseline).  vrt_batch_* puts
-// the views of many worlds behind one device queue of ray tiles: persistent warps
-// take chunks of tiles with one atomic, hand rays to idle lanes (regeneration),
-// refill when fewer than `refill_threshold` lanes are still tracing (compaction),
-// and a lane that finishes a ray continues its pixel's path in place.
+// the views of many worlds behind one device queue of ray tiles that persistent warps
+// take.  Without bounces (tile_kernel) a warp traces 32 pixels of a tile to their ends; with
+// bounces (persistent_kernel) it hands rays to idle lanes (regeneration), refills when fewer
+// than `refill_threshold` lanes are still tracing (compaction), and a lane that finishes a ray
+// continues its pixel's path in place.
 
 #include <cuda_runtime.h>
 
@@ -78,7 +79,8 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
     if (!kGlsl && !kBounces && vs.mask == kStartSolid && last == 0) {
         // the camera stands in a solid voxel: every ray hits it on iteration 0 at t = 0, face X
         const uint32_t x = vs.voxel[0] - kVoxelBias, y = vs.voxel[1] - kVoxelBias, z = vs.voxel[2] - kVoxelBias;
-        store_record<kPacked>(out, o, make_uint4(x | y << 11 | z << 21, (dx < 0.0f ? 1u : 0u) | vs.material << 8, 0u, pixel));
+        store_record<kPacked>(
+            out, o, make_uint4(x | y << 11 | z << 21, (dx < 0.0f ? 1u : 0u) | vs.material << 8, 0u, pixel));
         return 1;
     }
     const int32_t wox = v.wo[0], woy = v.wo[1], woz = v.wo[2];
@@ -145,9 +147,9 @@ __device__ __forceinline__ uint32_t trace_pixel(const ViewDev& v, const DevWorld
 // ray: 121.6 -> 118.0 us).  kFar: the world origin is not near; most rays stand still, and dda_trace
 // ends them (720p with sun rays from 2^22 voxels off, GLSL: 592 -> 148 us, CPU traversal 322 -> 113).
 template <bool kGlsl, bool kAniso, bool kBounces, bool kThin, bool kFar>
-__global__ void __launch_bounds__(kFrameThreads) view_path_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
-                                                       const __grid_constant__ ViewStart vs, uint32_t lanes_log2,
-                                                       uint4* __restrict__ out) {
+__global__ void __launch_bounds__(kFrameThreads)
+    view_path_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ViewDev v,
+                     const __grid_constant__ ViewStart vs, uint32_t lanes_log2, uint4* __restrict__ out) {
     if constexpr (kAniso) fill_forward_lut();
     uint32_t px, py;
     if (!thin_pixel<kThin>(lanes_log2, px, py) || px >= v.width || py >= v.height) return;
@@ -310,11 +312,13 @@ __device__ __forceinline__ uint32_t next_claim(const BatchParams& p) {
 // are enough for the CPU traversal (two 720p views of 4 bounces: 355 us against 382 us with
 // 72 and 379 us with 56), not for the GLSL modes (two worlds' whole paths: 654 us against 626 us).
 // kStall: rays that stand still (stalled) end early, looked at between the slices of a round.  A round
-// lasts until half of its lanes have ended, and stalled lanes hold it up to the cap: in the
-// GLSL modes many bounce rays are (a 720p view of a terrain with 2 bounces 382 -> 152 us, anisotropic
-// 358 -> 160), and of views whose world origin is not near nearly all rays (two such 720p views with
-// sun rays, CPU traversal: 599 us in tile_kernel, 193 here; GLSL 1140 and 255).  In the CPU traversal of
-// other views 1 ray in 500 is, and the test costs 6 % (spills).
+// lasts until half of its lanes have ended, and stalled lanes hold it up to the cap.  In the GLSL modes
+// 35 to 41 % of a camera's primary rays stand still when it lies in the plane of an empty brick's face
+// (a coordinate that is a multiple of 8; of others none): there a 720p view of a terrain with 2 bounces
+// 382 -> 152 us, anisotropic 358 -> 160; elsewhere the test costs up to 0.7 %.  Of views whose world
+// origin is not near nearly all rays do (two such 720p views with sun rays, CPU traversal: 599 us in
+// tile_kernel, 193 here; GLSL 1140 and 255).  In the CPU traversal of other views 1 ray in 500 does,
+// and the test costs 6 % (spills).
 template <bool kCount, bool kGlsl, bool kResident, bool kAniso, bool kFull, bool kStall>
 __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
     if constexpr (kAniso) fill_forward_lut();
@@ -522,7 +526,8 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
                         __syncwarp();
                     }
                     const ViewDev* qv = kResident ? &sview : p.views + lo;
-                    q_end = min(q_next + (kResident ? p.chunk_rays : p.chunk_rays >> p.split_log2), vget<kResident>(&qv->n_rays, true));
+                    q_end = min(q_next + (kResident ? p.chunk_rays : p.chunk_rays >> p.split_log2),
+                                vget<kResident>(&qv->n_rays, true));
                     // the view's camera origin, shared by its rays: inside the clip box?
                     // (a resident view's world index is checked before it is used)
                     const int4 qwv = vget4<kResident>(reinterpret_cast<const int4*>(qv->wo));  // origin xyz, world
@@ -681,8 +686,9 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) persistent_kernel(BatchParams p) {
 // rays are of a length (92-96 % of lanes busy in an 8x4 group on terrain), so nothing is
 // gained by refilling lanes one by one, and without it the view, its world and what its rays
 // share (ViewStart) belong to the warp: in shared memory, read at a ray's start, the step
-// loop's part in registers.  Warp instructions for 32 primary rays, against the persistent
-// kernel: 240 and 48 a step, against 335 and 52, and 170 in all for a camera in a solid voxel.
+// loop's part in registers.  Warp instructions for 32 primary rays (smsp__inst_executed at caps of
+// 1 and 5 steps): 228 and 47 to 49 a step (335 and 52 in the persistent kernel when this one was
+// built), and 175 in all for a camera in a solid voxel.
 // 44 M rays over 154 views of 16 mixed worlds: 701 us against 1109 us, 658 us with the packed adds
 // and 64 registers; six 1080p terrain views with sun rays: 754 us against 1035 us, 718 us.  64
 // registers, 32 warps a SM, in the CPU traversal (72, 28 warps: 670 and 740 us, 56: 714 and 767);
@@ -755,7 +761,8 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) tile_kernel(BatchParams p) {
             ViewStart vs = view_start(w, v);
             if (!kGlsl && vs.inside) {
                 // iteration 0 of every ray of the view: the table entry and code at the origin
-                const uint32_t x = (uint32_t)(v.wo[0] + __float2int_rd(v.ox)), y = (uint32_t)(v.wo[1] + __float2int_rd(v.oy)),
+                const uint32_t x = (uint32_t)(v.wo[0] + __float2int_rd(v.ox)),
+                               y = (uint32_t)(v.wo[1] + __float2int_rd(v.oy)),
                                z = (uint32_t)(v.wo[2] + __float2int_rd(v.oz));
                 const uint32_t e = __ldg(w.bricks + (x >> 3) + (z >> 3) * w.bsx + (y >> 3) * w.bsxz);
                 if (e < kBrickEmpty) {
@@ -781,7 +788,8 @@ __global__ void __maxnreg__(kGlsl ? 72 : 64) tile_kernel(BatchParams p) {
         uint32_t y = ty * tile_h;
         for (;;) {
             const uint32_t px = (tx << p.tile_w_log2) + kx, py = y + ky;
-            if (px < v.width && py < v.height) rays += trace_pixel<kGlsl, kAniso, false, kPacked>(v, w, sw.start, px, py, p.out);
+            if (px < v.width && py < v.height)
+                rays += trace_pixel<kGlsl, kAniso, false, kPacked>(v, w, sw.start, px, py, p.out);
             __syncwarp();
             y += rows;
             if ((y & (tile_h - 1u)) == 0) {  // the tile is done
@@ -1051,8 +1059,8 @@ PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, boo
 cudaError_t persistent_occupancy(int& occ, int threads, bool count, bool glsl, bool aniso, bool resident, bool full,
                                  bool tiles, bool far) {
     const size_t smem = full ? (size_t)threads * 6 * sizeof(float) : 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, persistent_fn(count, glsl, aniso, resident, full, tiles, far),
-                                                         threads, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &occ, persistent_fn(count, glsl, aniso, resident, full, tiles, far), threads, smem);
 }
 
 }  // namespace
@@ -1119,9 +1127,10 @@ vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool
     const uint64_t claims = std::max<uint64_t>(1, (uint64_t)p.total_chunks << q.split_log2);
     blocks = (int)std::min<uint64_t>((uint64_t)blocks, (claims * 32 + threads - 1) / threads);
     const bool glsl = p.glsl != 0, aniso = p.aniso != 0;
-    const PersistentFn fn = !tiles ? persistent_fn(count, glsl, aniso, false, p.full != 0, false, p.far != 0)
-                            : q.split_log2 ? (p.packed ? tile_fn<true, true>(glsl, aniso) : tile_fn<false, true>(glsl, aniso))
-                            : p.packed ? tile_fn<true, false>(glsl, aniso) : tile_fn<false, false>(glsl, aniso);
+    const auto tile = q.split_log2 ? (p.packed ? tile_fn<true, true> : tile_fn<false, true>)
+                                   : (p.packed ? tile_fn<true, false> : tile_fn<false, false>);
+    const PersistentFn fn = tiles ? tile(glsl, aniso)
+                                  : persistent_fn(count, glsl, aniso, false, p.full != 0, false, p.far != 0);
     fn<<<blocks, threads, pend_bytes(p, threads), stream>>>(q);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
@@ -1130,8 +1139,8 @@ vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool
 namespace {
 
 // vrt_batch_run_packed of views with bounces (tile_kernel stores this form itself): records
-// [0, n) of one part as 12-byte vrt_hit_packed, one thread per record (three 4-byte stores: a warp's stores cover 384 contiguous bytes); the 16-byte
-// records are read once, so they are loaded as streaming
+// [0, n) of one part as 12-byte vrt_hit_packed, one thread per record (three 4-byte stores: a warp's
+// stores cover 384 contiguous bytes); the 16-byte records are read once, so they are loaded as streaming
 static_assert(sizeof(vrt_hit_packed) == 12 && sizeof(vrt_hit) == 16, "record sizes");
 __global__ void __launch_bounds__(256)
     pack_records_kernel(const uint4* __restrict__ in, uint32_t* __restrict__ out, uint64_t n) {

@@ -119,9 +119,9 @@ uint64_t view_record_count(const vrt_view& v);
 vrt_status check_view(const vrt_view* v);
 // Fill defaults and validate a batch config.
 vrt_status normalize_batch_config(const vrt_batch_config* in, vrt_batch_config& out);
-// Tiles per queue chunk when a config leaves it to the library (chunk_tiles 0): about
-// eight chunks per warp of the launch, 1..16 tiles.  Fixed chunks too large for a small
-// launch leave most warps without work; the tuned table names its chunks explicitly.
+// About eight chunks of tiles per warp of the launch, 1..16 tiles each: fixed chunks too large for a
+// small launch leave most warps without work.  The chunk of a launch without bounces on the persistent
+// kernel (far_launch) whose config leaves it open; tile_kernel takes at most 2 of it.
 uint32_t auto_chunk_tiles(uint64_t tiles, uint64_t warps);
 // Whether a launch of these views runs tile_kernel: no view has bounces, and none is far.
 bool tile_launch(const vrt_view* views, uint32_t n);
@@ -130,17 +130,18 @@ bool tile_launch(const vrt_view* views, uint32_t n);
 bool far_launch(const vrt_view* views, uint32_t n);
 // Fill the fields a config leaves to the library (0): views with diffuse bounces (long,
 // uneven, incoherent paths per pixel) refill below 28 lanes and claim one tile at a time;
-// camera and sun rays refill below 16 and claim auto_chunk_tiles.
+// others refill below 16 and claim auto_chunk_tiles.
 void resolve_batch_defaults(vrt_batch_config& cfg, const vrt_view* views, uint32_t n, uint64_t warps);
-// The same for a launch of these views: with tile_kernel a chunk left open is at most 2 tiles.
+// The same for a launch of these views: with tile_kernel a chunk left open is 1 tile with sun rays
+// below 64 tiles a warp, else at most 2.
 void resolve_launch_config(vrt_batch_config& cfg, const vrt_view* views, uint32_t n, uint64_t warps);
 // Validate views against n_worlds and lay them out (tiles, queue chunks, record offsets).
 // Fields left to the library are resolved for a launch of `warps` warps
 // (resolve_launch_config), and plan.cfg holds the config used.
 vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, const vrt_batch_config& cfg,
                       LaunchPlan& plan, uint64_t warps = 0);
-// Grid of the persistent kernel: every SM, as many blocks of the launched instantiation
-// (counting, traversal mode, resident) as fit, or cfg.blocks_per_sm of them.
+// Grid of a launch: every SM, as many blocks of the kernel it runs (tile_kernel, or an instantiation
+// of the persistent kernel) as fit, or cfg.blocks_per_sm of them.
 vrt_status persistent_grid(int device, const vrt_batch_config& cfg, bool count, bool glsl, bool aniso, bool resident,
                            bool full, bool tiles, bool far, int& blocks, int& threads);
 BatchParams make_params(const LaunchPlan& plan, const DevWorld* worlds, const ViewDev* views,

@@ -815,8 +815,8 @@ vrt_status vrt_server_create(vrt_world* const* worlds, uint32_t n_worlds, const 
     sv->resident = resident;
     for (int m = 0; m < 6; m++) {
         int* g = sv->grid[m / 3][m % 3];
-        if ((st = persistent_grid(sv->device, sv->bcfg, false, m % 3 >= 1, m % 3 == 2, resident, false, m >= 3, false, g[0],
-                                  g[1])) != VRT_OK)
+        if ((st = persistent_grid(sv->device, sv->bcfg, false, m % 3 >= 1, m % 3 == 2, resident, false, m >= 3, false,
+                                  g[0], g[1])) != VRT_OK)
             return fail(st);
     }
     if (resident && (st = resident_init(sv)) != VRT_OK) return fail(st);

@@ -1,9 +1,9 @@
 // trace.cu - per-view and explicit-ray traversal kernels and their C ABI.
 //
 // vrt_render_view* is the one-launch-per-view path of GpuRenderer::RenderFrame
-// (src/VoxelRT/GpuRenderer.cpp:239-273): 8x8 thread blocks over the image, one
-// primary ray per pixel (Shaders/VoxelRender.comp:27-30), writing a headless hit
-// buffer instead of the G-buffer.  vrt_cast* traverses caller-supplied rays.
+// (src/VoxelRT/GpuRenderer.cpp:239-273): thread blocks over 16x8 pixels of the image, fewer
+// of a small one (thin_launch.cuh), one primary ray per pixel (Shaders/VoxelRender.comp:27-30),
+// writing a headless hit buffer instead of the G-buffer.  vrt_cast* traverses caller-supplied rays.
 
 #include <cuda_runtime.h>
 
@@ -44,7 +44,8 @@ __global__ void __maxnreg__(48) render_view_kernel(const __grid_constant__ DevWo
         ray_start<false>(s, clip, cam.origin[0], cam.origin[1], cam.origin[2], dx, dy, dz, wox, woy, woz);
     TraceCounters cnt;
     uint32_t i = 0;
-    const bool hit = dda_steps_mode<false, false>(s, w, wox, woy, woz, cnt, false, false, false, 0, i, max_iters) == kStepHit;
+    const bool hit =
+        dda_steps_mode<false, false>(s, w, wox, woy, woz, cnt, false, false, false, 0, i, max_iters) == kStepHit;
     const uint32_t pix = py * cam.width + px;
     out[pix] = pack_state<false>(s, hit_material(s, w.payload, hit), hit, i, pix);
 }
@@ -54,10 +55,12 @@ __global__ void __maxnreg__(48) render_view_kernel(const __grid_constant__ DevWo
 // with 8 / 16 / 32 steps 14.6 / 14.2 / 14.1 us (14.0 without the test), 120,000 with anisotropic LODs in a
 // world with 2 % of its voxels set 35.3 / 35.3 / 41.5 us (45.6 without).
 template <bool kGlsl, bool kAniso = false>
-__global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ClipBox clip,
-                                                  const float4* __restrict__ rays, uint32_t n,
-                                                  int32_t wox, int32_t woy, int32_t woz, uint32_t max_iters,
-                                                  uint4* __restrict__ out, bool coarse, uint32_t lanes_log2, uint32_t slice) {
+__global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWorld w,
+                                                  const __grid_constant__ ClipBox clip,
+                                                  const float4* __restrict__ rays, uint32_t n, int32_t wox,
+                                                  int32_t woy, int32_t woz, uint32_t max_iters,
+                                                  uint4* __restrict__ out, bool coarse, uint32_t lanes_log2,
+                                                  uint32_t slice) {
     if constexpr (kAniso) fill_forward_lut();
     const uint32_t lane = threadIdx.x & 31;
     if (lane >> lanes_log2) return;
@@ -82,7 +85,8 @@ __global__ void __launch_bounds__(256) cast_kernel(const __grid_constant__ DevWo
 // cast_kernel: a lane's steps continue from where its ray left off, and a ray's record
 // is packed from the state at its exit.
 template <bool kGlsl, bool kAniso = false>
-__global__ void __maxnreg__(56) cast_persistent_kernel(const __grid_constant__ DevWorld w, const __grid_constant__ ClipBox clip,
+__global__ void __maxnreg__(56) cast_persistent_kernel(const __grid_constant__ DevWorld w,
+                                                             const __grid_constant__ ClipBox clip,
                                                              const float4* __restrict__ rays, uint32_t n,
                                                              int32_t wox, int32_t woy, int32_t woz, uint32_t max_iters,
                                                              uint32_t inner, uint32_t refill, uint4* __restrict__ out,
@@ -150,8 +154,8 @@ __global__ void __maxnreg__(56) cast_persistent_kernel(const __grid_constant__ D
             if (active && !ended) {
                 const uint32_t first = iter, lim = max_iters - iter < inner ? max_iters : iter + inner;
                 // GLSL variants (rayCastCoarse, anisotropic LODs) are uniform over the launch
-                const uint32_t st = dda_steps_mode<false, kGlsl, true>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso, 0,
-                                                                       iter, lim);
+                const uint32_t st = dda_steps_mode<false, kGlsl, true>(s, w, wox, woy, woz, cnt, coarse, coarse, kAniso,
+                                                                       0, iter, lim);
                 if (st == kStepContinue && stalled<kGlsl>(s, t0, coarse, first)) iter = max_iters;
                 t0 = last_t<kGlsl>(s);
                 if (st != kStepContinue || iter >= max_iters) {
@@ -181,8 +185,9 @@ vrt_status launch_render(vrt_world* w, const vrt_camera* cam, uint32_t max_iters
     const DevWorld dw = w->dev();
     const float* o = cam->origin;
     const ClipBox clip = clip_box(dw, cam->world_origin);
-    render_view_kernel<<<thin_grid(ll, cam->width, cam->height), kFrameThreads, 0, stream>>>(dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]), ll,
-                                                eff_iters(max_iters), reinterpret_cast<uint4*>(hits));
+    render_view_kernel<<<thin_grid(ll, cam->width, cam->height), kFrameThreads, 0, stream>>>(
+        dw, *cam, clip, origin_inside_near(clip, o[0], o[1], o[2]), ll, eff_iters(max_iters),
+        reinterpret_cast<uint4*>(hits));
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }
@@ -237,8 +242,8 @@ vrt_status launch_cast(vrt_world* w, const vrt_ray* rays, uint32_t n, const vrt_
         VRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kCastThreads, 0));
         const uint32_t blocks = (uint32_t)(sms * std::max(occ, 1));
         kernel<<<blocks, kCastThreads, 0, stream>>>(dw, clip, r4, n, p->world_origin[0], p->world_origin[1],
-                                                    p->world_origin[2], iters, cast_slice(glsl, coarse, aniso), kCastRefill, o4,
-                                                    coarse);
+                                                    p->world_origin[2], iters, cast_slice(glsl, coarse, aniso),
+                                                    kCastRefill, o4, coarse);
     }
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;

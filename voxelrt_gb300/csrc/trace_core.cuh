@@ -44,9 +44,8 @@ __device__ __forceinline__ float add_rd(float a, float b) {
 // Two float adds in one instruction (sm_100 and later), each rounded as its scalar form: the step
 // loop is bound by instruction issue, and x and y take the same operations. 1080p frame with
 // a shadow ray 126.7 -> 121.8 us, 1080p x 8 views 754 -> 742, 64 mixed views 679 -> 671, an
-// anisotropic path batch 710 -> 694. The products stay scalar: a packed multiply that feeds a
-// packed add is contracted to a fused multiply-add also where both ask for rounding and the
-// build turns contraction off, and other results follow.
+// anisotropic path batch 710 -> 694. The products stay scalar: with a packed multiply that feeds a
+// packed add the records differ from the oracle's, as a fused multiply-add's would.
 struct F2 {
     float x, y;
 };
@@ -74,8 +73,8 @@ __device__ __forceinline__ F2 add2_rd(F2 a, F2 b) { return F2{add_rd(a.x, b.x), 
 // is exact, and add_rd(pos, K) is M + worldOrigin + floor(pos): one add on the FMA pipe takes
 // the place of a conversion (on a quarter-rate unit, the longest latency in the step's chain)
 // and of the add of worldOrigin.  A position out of the grid, an infinity or NaN among them,
-// gives bits below kVoxelBias or at least the grid's size above it (unsigned).  Back in the ray frame, the float minus K is exactly
-// voxel - worldOrigin.
+// gives bits below kVoxelBias or at least the grid's size above it (unsigned).  Back in the ray
+// frame, the float minus K is exactly voxel - worldOrigin.
 constexpr uint32_t kVoxelBias = 0x4B400000u;
 // K of an axis
 __device__ __forceinline__ float voxel_frame(int32_t wo) { return __uint_as_float(kVoxelBias + (uint32_t)wo); }
@@ -411,7 +410,7 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int
     }
     const uint32_t ux = vx - kBias, uy = vy - kBias, uz = vz - kBias;
     const bool in = ux < w.size_x && uy < w.size_y && uz < w.size_z;
-    // (the sum in 32 bits: added to the pointer term by term it takes three wide adds)
+    // (the sum in 32 bits: added to the pointer term by term 44 M camera rays took 698 us against 679)
     const uint32_t ei = (uy >> 3) * w.bsxz + ((uz >> 3) * w.bsx + (ux >> 3));
     const uint32_t vi = (ux & 7u) | (uz & 7u) << 3 | (uy & 7u) << 6;  // voxel in brick x | z<<3 | y<<6
     // The brick table holds the slot of an allocated brick, or for an empty one the
@@ -494,9 +493,9 @@ __device__ __forceinline__ uint32_t ray_step(RayState& s, const DevWorld& w, int
 
 // Steps k = k .. kmax-1 of a ray whose first step here is its iteration i0 + k, until
 // one ends it (the returned status) or kmax is reached (kStepContinue).  The general step's loop
-// follows the fast one, which it leaves in place: a choice between the two cost the fast loop
-// ten register moves a step (59 instead of 49 instructions).  A test of the distance against
-// the grid's exit in place of the three bounds compares saved nothing, and lanes past the
+// follows the fast one, which it leaves in place: with a choice between the two a step took 59 warp
+// instructions instead of 49 (smsp__inst_executed at caps of 1 and 5 steps).  A test of the distance
+// against the grid's exit in place of the three bounds compares saved nothing, and lanes past the
 // exit, stepping in the second loop, doubled the time of warps with stalled rays.
 // coarse_ray: a rayCastCoarse ray (kCoarse only).
 template <bool kCount, bool kGlsl, bool kCoarse, bool kAniso, bool kFlat>
@@ -547,10 +546,10 @@ __device__ __forceinline__ uint32_t dda_steps_mode(RayState& s, const DevWorld& 
 // (coarse_ray) once its steps no longer depend on their number.
 // Looked at between slices of steps: 2,000 random GLSL rays 49 -> 13 us, 2.5 M 653 -> 112, 2.5 M
 // anisotropic 841 -> 128, 60,000 CPU rays in a mixed world 22.9 -> 12.1; 1 M CPU rays from 2^22 voxels
-// off the world origin 290 -> 68.  The persistent kernel looks too, in the GLSL modes, whose bounce rays
-// start from hits in world coordinates (batch.cu), and views whose world origin is not near, nearly
-// all of whose rays stand still.  Other frames and batches look for none: camera rays start near the
-// world origin and do not stand still, and the slices' loop cost them 2 to 8 %.
+// off the world origin 290 -> 68.  The persistent kernel looks too (batch.cu), in the GLSL modes, where a
+// third of a camera's rays stand still when it lies in the plane of an empty brick's face, and in views
+// whose world origin is not near, nearly all of whose rays do.  Other frames and batches look for none: the
+// slices' loop cost them 2 to 8 %.
 template <bool kGlsl>
 __device__ __forceinline__ float last_t(const RayState& s) {
     return kGlsl ? s.tb : min_x86(min_x86(s.sx, s.sy), s.sz);
@@ -571,7 +570,8 @@ __device__ __forceinline__ uint32_t dda_trace(RayState& s, const DevWorld& w, in
     float t0 = no_t();
     for (;;) {
         const uint32_t first = i, lim = iters - i < slice ? iters : i + slice;
-        const uint32_t st = dda_steps_mode<false, kGlsl, kFlat>(s, w, wox, woy, woz, cnt, coarse, coarse_ray, aniso, 0, i, lim);
+        const uint32_t st =
+            dda_steps_mode<false, kGlsl, kFlat>(s, w, wox, woy, woz, cnt, coarse, coarse_ray, aniso, 0, i, lim);
         if (st != kStepContinue || i >= iters) return st;
         if (stalled<kGlsl>(s, t0, coarse_ray, first)) {
             i = iters;

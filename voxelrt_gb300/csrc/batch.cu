@@ -937,6 +937,9 @@ uint32_t auto_chunk_tiles(uint64_t tiles, uint64_t warps) {
 // the last claims, and 16 tiles (1,024 rays) of long rays run on for a third of a millisecond
 // after the queue is empty (44 M rays over 154 views: 1466 us with 16 tiles, 1041 with 4, 968
 // with 2, 950 with 1 in the kernel's first build; 658 with 2, 782 with 1 in the present one).
+// The cap holds at every size, though where the tiles are many and their rays short more are better:
+// 353 M rays of the same kind, half of whose views end at once, take 2.62 ms with 8 tiles and 2.89
+// with 2, so a large recurring batch is worth a config of its own (autotune.py).
 // Pixels with a sun ray are twice the work, so one tile up to kOneTileWarps a warp (six 1080p
 // views 718 -> 697 us).
 constexpr uint32_t kTileChunk = 2, kOneTileWarps = 64;

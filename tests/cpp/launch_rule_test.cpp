@@ -47,7 +47,7 @@ static uint32_t chunk(const std::vector<vrt_view>& views, uint64_t warps, uint32
     CHECK(plan_views(views.data(), (uint32_t)views.size(), 1, open, plan, warps) == VRT_OK);
     CHECK(plan.cfg.chunk_tiles == c.chunk_tiles);
     CHECK(plan.tiles == tile_launch(views.data(), (uint32_t)views.size()));
-    CHECK(plan.far == far_launch(views.data(), (uint32_t)views.size()));
+    CHECK(plan.stall == stall_launch(views.data(), (uint32_t)views.size()));
     return c.chunk_tiles;
 }
 
@@ -64,6 +64,20 @@ int main() {
         CHECK(!tiles({make(64, 64), make(8, 8, 0, false, wo)}));
         CHECK(far({make(64, 64), make(8, 8, 3, true, wo)}));
     }
+    // the test for rays that stand still: far views, and GLSL cameras with a whole coordinate
+    auto stall = [](float x, uint32_t flags, int32_t wo = 0) {
+        vrt_view v = make(8, 8, 2, false, wo);
+        for (float& o : v.cam.origin) o = 0.25f;
+        v.cam.origin[1] = x;
+        v.flags |= flags;
+        return stall_launch(&v, 1);
+    };
+    const uint32_t glsl = VRT_VIEW_GLSL, aniso = VRT_VIEW_GLSL | VRT_VIEW_GLSL_ANISO;
+    for (const uint32_t f : {glsl, aniso}) {
+        for (const float x : {0.0f, -0.0f, 3.0f, -16.0f, 1e9f}) CHECK(stall(x, f) && !stall(x, 0));
+        for (const float x : {0.5f, 63.999f, -1e-6f}) CHECK(!stall(x, f) && stall(x, f, near));
+    }
+    CHECK(stall(0.5f, 0, near) && !stall(0.5f, 0, near - 1));
 
     // claims of tile_kernel, left open: at most 2 tiles, 1 with sun rays below 64 tiles a warp
     const uint64_t warps = 100;

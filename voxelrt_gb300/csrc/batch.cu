@@ -15,6 +15,7 @@
 #include <cuda/atomic>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -314,8 +315,9 @@ __device__ __forceinline__ uint32_t next_claim(const BatchParams& p) {
 // kStall: rays that stand still (stalled) end early, looked at between the slices of a round.  A round
 // lasts until half of its lanes have ended, and stalled lanes hold it up to the cap.  In the GLSL modes
 // 35 to 41 % of a camera's primary rays stand still when it lies in the plane of an empty brick's face
-// (a coordinate that is a multiple of 8; of others none): there a 720p view of a terrain with 2 bounces
-// 382 -> 152 us, anisotropic 358 -> 160; elsewhere the test costs up to 0.7 %.  Of views whose world
+// (of others none): there a 720p view of a terrain with 2 bounces 382 -> 152 us, anisotropic 358 ->
+// 160; elsewhere the test costs up to 0.7 %, so stall_launch asks for it where some camera has a
+// whole coordinate (a resident launch, whose views are not known, always looks).  Of views whose world
 // origin is not near nearly all rays do (two such 720p views with sun rays, CPU traversal: 599 us in
 // tile_kernel, 193 here; GLSL 1140 and 255).  In the CPU traversal of other views 1 ray in 500 does,
 // and the test costs 6 % (spills).
@@ -953,6 +955,12 @@ bool far_launch(const vrt_view* views, uint32_t n) {
         if (!near_origin(views[i].cam.world_origin)) return true;
     return false;
 }
+bool stall_launch(const vrt_view* views, uint32_t n) {
+    for (uint32_t i = 0; i < n; i++)
+        for (int c = 0; c < 3; c++)
+            if (view_glsl(views[i]) && views[i].cam.origin[c] == std::floor(views[i].cam.origin[c])) return true;
+    return far_launch(views, n);
+}
 
 void resolve_batch_defaults(vrt_batch_config& cfg, const vrt_view* views, uint32_t n, uint64_t warps) {
     bool bounces = false;
@@ -997,7 +1005,7 @@ vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, cons
     plan.full = false;
     for (uint32_t i = 0; i < n; i++) plan.full |= view_full_path(views[i]);
     plan.tiles = tile_launch(views, n);
-    plan.far = far_launch(views, n);
+    plan.stall = stall_launch(views, n);
     plan.cfg = cfg;
     plan.tile_w_log2 = log2u(cfg.tile_w);
     plan.tile_size_log2 = log2u(cfg.tile_w * cfg.tile_h);
@@ -1034,46 +1042,49 @@ namespace {
 // The kernel a launch runs: tiles (no view has bounces), or the persistent kernel's
 // instantiation: counting, traversal mode, resident, whole-path views.
 using PersistentFn = void (*)(BatchParams);
-template <bool kCount, bool kResident, bool kFull>
-PersistentFn persistent_fn_mode(bool glsl, bool aniso, bool far) {
-    if (glsl && aniso) return persistent_kernel<kCount, true, kResident, true, kFull, !kCount>;
-    if (glsl) return persistent_kernel<kCount, true, kResident, false, kFull, !kCount>;
-    if constexpr (!kCount && !kResident)
-        if (far) return persistent_kernel<false, false, false, false, kFull, true>;
-    return persistent_kernel<kCount, false, kResident, false, kFull, false>;
+template <bool kCount, bool kResident, bool kFull, bool kGlslStall, bool kCpuStall>
+PersistentFn persistent_fn_mode(bool glsl, bool aniso) {
+    if (glsl && aniso) return persistent_kernel<kCount, true, kResident, true, kFull, kGlslStall>;
+    if (glsl) return persistent_kernel<kCount, true, kResident, false, kFull, kGlslStall>;
+    return persistent_kernel<kCount, false, kResident, false, kFull, kCpuStall>;
 }
 template <bool kPacked, bool kSplit>
 PersistentFn tile_fn(bool glsl, bool aniso) {
     return glsl ? (aniso ? tile_kernel<true, true, kPacked, kSplit> : tile_kernel<true, false, kPacked, kSplit>)
                 : tile_kernel<false, false, kPacked, kSplit>;
 }
-PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, bool full, bool tiles, bool far) {
+PersistentFn persistent_fn(bool count, bool glsl, bool aniso, bool resident, bool full, bool tiles, bool stall) {
     if (tiles && !count && !resident) return tile_fn<false, false>(glsl, aniso);
-    if (resident) return full ? persistent_fn_mode<false, true, true>(glsl, aniso, far)
-                              : persistent_fn_mode<false, true, false>(glsl, aniso, far);
-    if (count) return full ? persistent_fn_mode<true, false, true>(glsl, aniso, far)
-                           : persistent_fn_mode<true, false, false>(glsl, aniso, far);
-    return full ? persistent_fn_mode<false, false, true>(glsl, aniso, far)
-                : persistent_fn_mode<false, false, false>(glsl, aniso, far);
+    if (resident)  // (its views are not known yet)
+        return full ? persistent_fn_mode<false, true, true, true, false>(glsl, aniso)
+                    : persistent_fn_mode<false, true, false, true, false>(glsl, aniso);
+    if (count)
+        return full ? persistent_fn_mode<true, false, true, false, false>(glsl, aniso)
+                    : persistent_fn_mode<true, false, false, false, false>(glsl, aniso);
+    if (stall)
+        return full ? persistent_fn_mode<false, false, true, true, true>(glsl, aniso)
+                    : persistent_fn_mode<false, false, false, true, true>(glsl, aniso);
+    return full ? persistent_fn_mode<false, false, true, false, false>(glsl, aniso)
+                : persistent_fn_mode<false, false, false, false, false>(glsl, aniso);
 }
 
 // Resident blocks per SM of that kernel: the variants differ in registers and shared memory
 // (the anisotropic LUT is 8 KB per block).
 cudaError_t persistent_occupancy(int& occ, int threads, bool count, bool glsl, bool aniso, bool resident, bool full,
-                                 bool tiles, bool far) {
+                                 bool tiles, bool stall) {
     const size_t smem = full ? (size_t)threads * 6 * sizeof(float) : 0;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &occ, persistent_fn(count, glsl, aniso, resident, full, tiles, far), threads, smem);
+        &occ, persistent_fn(count, glsl, aniso, resident, full, tiles, stall), threads, smem);
 }
 
 }  // namespace
 
 vrt_status persistent_grid(int device, const vrt_batch_config& cfg, bool count, bool glsl, bool aniso, bool resident,
-                           bool full, bool tiles, bool far, int& blocks, int& threads) {
+                           bool full, bool tiles, bool stall, int& blocks, int& threads) {
     int sms = 0, occ = 0;
     threads = (int)cfg.warps_per_block * 32;
     VRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    VRT_CUDA(persistent_occupancy(occ, threads, count, glsl, aniso, resident, full, tiles, far));
+    VRT_CUDA(persistent_occupancy(occ, threads, count, glsl, aniso, resident, full, tiles, stall));
     occ = std::max(occ, 1);
     const int per_sm = (!count && cfg.blocks_per_sm) ? std::min<int>((int)cfg.blocks_per_sm, occ) : occ;
     blocks = sms * per_sm;
@@ -1104,7 +1115,7 @@ BatchParams make_params(const LaunchPlan& plan, const DevWorld* worlds, const Vi
     p.aniso = plan.aniso ? 1u : 0u;
     p.full = plan.full ? 1u : 0u;
     p.tiles = plan.tiles ? 1u : 0u;
-    p.far = plan.far ? 1u : 0u;
+    p.stall = plan.stall ? 1u : 0u;
     return p;
 }
 
@@ -1133,7 +1144,7 @@ vrt_status launch_persistent(const BatchParams& p, int blocks, int threads, bool
     const auto tile = q.split_log2 ? (p.packed ? tile_fn<true, true> : tile_fn<false, true>)
                                    : (p.packed ? tile_fn<true, false> : tile_fn<false, false>);
     const PersistentFn fn = tiles ? tile(glsl, aniso)
-                                  : persistent_fn(count, glsl, aniso, false, p.full != 0, false, p.far != 0);
+                                  : persistent_fn(count, glsl, aniso, false, p.full != 0, false, p.stall != 0);
     fn<<<blocks, threads, pend_bytes(p, threads), stream>>>(q);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
@@ -1276,7 +1287,7 @@ vrt_status vrt_batch_create(vrt_world* const* worlds, uint32_t n_worlds, const v
         bool full = false;
         for (uint32_t i = 0; i < n_views; i++) full |= view_full_path(views[i]);
         if ((st = persistent_grid(worlds[0]->device, cfg, false, view_glsl(views[0]), view_aniso(views[0]), false,
-                                  full, tile_launch(views, n_views), far_launch(views, n_views), grid_blocks,
+                                  full, tile_launch(views, n_views), stall_launch(views, n_views), grid_blocks,
                                   grid_threads)) != VRT_OK)
             return st;
     }
@@ -1314,7 +1325,7 @@ vrt_status vrt_batch_create(vrt_world* const* worlds, uint32_t n_worlds, const v
     b->d_counters = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(b->d_queue) + 16);
     if ((st = refresh_worlds(b, 0)) != VRT_OK) return fail(st);
     const bool glsl = b->plan.glsl, aniso = b->plan.aniso, full = b->plan.full;
-    if ((st = persistent_grid(b->device, cfg, false, glsl, aniso, false, full, b->plan.tiles, b->plan.far, b->blocks,
+    if ((st = persistent_grid(b->device, cfg, false, glsl, aniso, false, full, b->plan.tiles, b->plan.stall, b->blocks,
                               b->threads)) != VRT_OK)
         return fail(st);
     if ((st = persistent_grid(b->device, cfg, true, glsl, aniso, false, full, false, false, b->blocks_count,

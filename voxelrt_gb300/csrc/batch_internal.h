@@ -66,7 +66,7 @@ struct BatchParams {
     uint32_t aniso;  // ... with anisotropic LODs (VRT_VIEW_GLSL_ANISO)
     uint32_t tiles;  // tile_kernel traces the launch (tile_launch)
     uint32_t packed; // (tiles) records are stored in the 12-byte form
-    uint32_t far;    // some view's world origin is not near (near_origin): see far_launch
+    uint32_t stall;  // many of the launch's rays may stand still (stall_launch)
     uint32_t full;   // some view traces the GPU renderer's whole path (sun rays among bounces)
     // resident launches (request server): views are published while the kernel runs
     unsigned long long* mailbox;  // host-mapped: published chunks | published views << 32 | closed << 63
@@ -97,7 +97,7 @@ struct LaunchPlan {
     bool glsl = false;   // every view traces in the GLSL mode
     bool aniso = false;  // ... with anisotropic LODs
     bool tiles = false;  // the launch runs tile_kernel (tile_launch)
-    bool far = false;    // some view's world origin is not near (far_launch)
+    bool stall = false;  // many of its rays may stand still (stall_launch)
     bool full = false;   // some view traces the GPU renderer's whole path
 };
 
@@ -128,6 +128,9 @@ bool tile_launch(const vrt_view* views, uint32_t n);
 // Whether some view's world origin is too far for the fast step (near_origin): most of its rays
 // stand still until the cap, so the persistent kernel traces it and looks for those.
 bool far_launch(const vrt_view* views, uint32_t n);
+// Whether many rays of a launch on the persistent kernel may stand still: a far view, or in the GLSL
+// modes a camera with a whole coordinate, whose rays start on the face of an empty cell.
+bool stall_launch(const vrt_view* views, uint32_t n);
 // Fill the fields a config leaves to the library (0): views with diffuse bounces (long,
 // uneven, incoherent paths per pixel) refill below 28 lanes and claim one tile at a time;
 // others refill below 16 and claim auto_chunk_tiles.
@@ -143,7 +146,7 @@ vrt_status plan_views(const vrt_view* views, uint32_t n, uint32_t n_worlds, cons
 // Grid of a launch: every SM, as many blocks of the kernel it runs (tile_kernel, or an instantiation
 // of the persistent kernel) as fit, or cfg.blocks_per_sm of them.
 vrt_status persistent_grid(int device, const vrt_batch_config& cfg, bool count, bool glsl, bool aniso, bool resident,
-                           bool full, bool tiles, bool far, int& blocks, int& threads);
+                           bool full, bool tiles, bool stall, int& blocks, int& threads);
 BatchParams make_params(const LaunchPlan& plan, const DevWorld* worlds, const ViewDev* views,
                         const uint32_t* chunk_base, uint32_t* queue, vrt_hit* out);
 // Reset of the tile counter and the launch counters (64 bytes at params.queue; 0: the caller

@@ -117,9 +117,9 @@ extern "C" vrt_status vrt_render_views_static(vrt_world* const* worlds, uint32_t
     const bool aniso = view_aniso(views[0]);
     bool full = false;
     for (uint32_t i = 0; i < n_views; i++) full |= view_full_path(views[i]);
-    const bool tiles = tile_launch(views, n_views), far = far_launch(views, n_views);
+    const bool tiles = tile_launch(views, n_views), stall = stall_launch(views, n_views);
     int blocks = 0, threads = 0;
-    if ((st = persistent_grid(device, cfg, false, glsl, aniso, false, full, tiles, far, blocks, threads)) != VRT_OK)
+    if ((st = persistent_grid(device, cfg, false, glsl, aniso, false, full, tiles, stall, blocks, threads)) != VRT_OK)
         return st;
     resolve_launch_config(cfg, views, n_views, (uint64_t)blocks * (threads / 32));
     // lay the views out behind one tile queue (same layout as vrt_batch)
@@ -175,7 +175,7 @@ extern "C" vrt_status vrt_render_views_static(vrt_world* const* worlds, uint32_t
     p.aniso = aniso ? 1u : 0u;
     p.full = full ? 1u : 0u;
     p.tiles = tiles ? 1u : 0u;
-    p.far = far ? 1u : 0u;
+    p.stall = stall ? 1u : 0u;
     // launch_persistent zeroes the queue counter and the launch counters first
     return launch_persistent(p, blocks, threads, false, stream);
 }

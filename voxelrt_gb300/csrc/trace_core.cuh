@@ -546,9 +546,9 @@ __device__ __forceinline__ uint32_t dda_steps_mode(RayState& s, const DevWorld& 
 // (coarse_ray) once its steps no longer depend on their number.
 // Looked at between slices of steps: 2,000 random GLSL rays 49 -> 13 us, 2.5 M 653 -> 112, 2.5 M
 // anisotropic 841 -> 128, 60,000 CPU rays in a mixed world 22.9 -> 12.1; 1 M CPU rays from 2^22 voxels
-// off the world origin 290 -> 68.  The persistent kernel looks too (batch.cu), in the GLSL modes, where a
-// third of a camera's rays stand still when it lies in the plane of an empty brick's face, and in views
-// whose world origin is not near, nearly all of whose rays do.  Other frames and batches look for none: the
+// off the world origin 290 -> 68.  The persistent kernel looks too (batch.cu), in launches of the GLSL
+// modes, where a third of a camera's rays stand still when it lies in the plane of an empty brick's
+// face, and of views whose world origin is not near, nearly all of whose rays do.  Other frames and batches look for none: the
 // slices' loop cost them 2 to 8 %.
 template <bool kGlsl>
 __device__ __forceinline__ float last_t(const RayState& s) {
